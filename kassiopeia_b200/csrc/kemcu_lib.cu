@@ -1386,8 +1386,9 @@ int kemcu_field_dev(kemcu_ctx* ctx, const double* dP, size_t n, double* dout4, i
         // Morton order (meridian plane for axisymmetric models): bbox -> keys -> radix sort -> gather ->
         // evaluate -> scatter back
         const size_t cub_bytes = cub_sort_bytes(n);
+        // nine regions, each rounded up to 256 bytes by take()
         const size_t need = n * (2 * sizeof(unsigned long long) + 2 * sizeof(int) + 7 * sizeof(double)) + cub_bytes +
-                            1024 + 128 * 6 * sizeof(double);
+                            (6 + 128 * 6) * sizeof(double) + 9 * 256;
         void* base;
         if ((rc = ensure(ctx, sSort, need, &base)))
             return rc;
