@@ -93,6 +93,9 @@ __constant__ float c_qp32[kNumPairs * kQ];
 __constant__ float c_qc32[2];
 __constant__ double c_gl[10 * 2];
 __constant__ Constants c_k;
+// square roots of the integers and their reciprocals (harmonic recurrences of kemcu_fftm.cuh)
+constexpr int kNumRoots = 36;
+__constant__ double c_rt[kNumRoots], c_irt[kNumRoots];
 
 // ------------------------------------------------------------------------- helpers
 struct V3
@@ -667,6 +670,116 @@ template<int NV, bool POT, bool FIELD> __device__ __noinline__ Out4 rwg64(const 
     else
         o = rwg_at<NV, POT, FIELD>(q, P, counter, line, dmin);
     return Out4{k * o.ex, k * o.ey, k * o.ez, k * o.phi};
+}
+
+// The same integrals for a point off the element's plane and edge lines, which is nearly every
+// pair: the polygon's geometry comes from a record made once per element (rwg_build) instead of
+// being rebuilt for every pair, an edge takes one logarithm of a quotient instead of two, and the
+// solid angle one arctangent without normalising the corner vectors. With a, b, c the corners of a
+// triangle relative to P, tan(Omega / 2) = |a.(b x c)| / (|a||b||c| + (a.b)|c| + (a.c)|b| + (b.c)|a|)
+// (Van Oosterom-Strackee), and |a.(b x c)| is the distance from the plane times twice the
+// triangle's area for any triangle of it; the two halves of a rectangle add as the arguments of the
+// complex numbers D + iN (half of at most 2 pi). A point within 1e-9 of the plane or within 1e-9 of
+// an edge's line (in units of 1 + distance) takes rwg64 above, with the reference's on-line,
+// on-vertex and in-plane cases.
+enum Rwg : int
+{
+    wV = 0,    // corners (4 x 3; a triangle's fourth unused)
+    wU = 12,   // unit edge vectors: triangle 3, rectangle 2 (the other two are their negatives)
+    wM = 21,   // outward edge normals, as wU
+    wN = 30,   // unit normal
+    wCen = 33, // the point of the plane the distance is taken from
+    wArea = 36,  // twice the area of the triangle (0, 1, 2)
+    wRecSize = 38
+};
+
+template<int NV> __device__ __forceinline__ void rwg_record(const double* e, double* w)
+{
+    Polygon<NV> q;
+    make_polygon(e, q);
+    auto put = [&](int o, V3 v) { w[o] = v.x, w[o + 1] = v.y, w[o + 2] = v.z; };
+    for (int i = 0; i < NV; i++)
+        put(wV + 3 * i, q.v[i]);
+    for (int i = 0; i < (NV == 3 ? 3 : 2); i++) {
+        put(wU + 3 * i, q.u[i]);
+        put(wM + 3 * i, q.m[i]);
+    }
+    put(wN, q.n3);
+    put(wCen, q.cen);
+    w[wArea] = norm(cross(q.v[1] - q.v[0], q.v[2] - q.v[0]));
+}
+
+__global__ void rwg_build_kernel(const double* __restrict__ rec, int n, double* __restrict__ out)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n)
+        return;
+    const double* e = rec + (size_t) j * rRecSize;
+    double* w = out + (size_t) j * wRecSize;
+    for (int i = 0; i < wRecSize; i++)
+        w[i] = 0.;
+    const int type = (int) e[rType];
+    if (type == kTriangle)
+        rwg_record<3>(e, w);
+    else if (type == kRectangle)
+        rwg_record<4>(e, w);
+}
+
+template<int NV, bool POT, bool FIELD>
+__device__ __forceinline__ Out4 rwg_pair(const double* __restrict__ e, const double* __restrict__ w, V3 P)
+{
+    const V3 n = ld3(w + wN);
+    const double h = dot(n, P - ld3(w + wCen)), ah = fabs(h);
+    V3 dv[NV];
+    double r[NV], q2[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        dv[i] = ld3(w + wV + 3 * i) - P;
+        q2[i] = dot(dv[i], dv[i]);
+        r[i] = 0.5 * q2[i] * rsqrt2_acc(q2[i]);
+    }
+    // off the plane, and off every edge's line (the latter only matters near the plane, but h is
+    // part of that distance)
+    if (!(ah > 1e-9 * (1. + r[0])))
+        return rwg64<NV, POT, FIELD>(e, P);
+    double il = 0.;
+    V3 iv = v3(0., 0., 0.);
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        constexpr int half = NV == 4 ? 2 : 3;
+        const int j = (i + 1) % NV;
+        const double sg = i < half ? 1. : -1.;
+        const V3 u = ld3(w + wU + 3 * (i % half)), m = ld3(w + wM + 3 * (i % half));
+        const double sM = sg * dot(dv[i], u), sP = sg * dot(dv[j], u);
+        const bool up = r[i] + sM > r[j] - sP;
+        const double nom = up ? r[j] + sP : r[i] - sM, den = up ? r[i] + sM : r[j] - sP;
+        const double term = sg * log(nom / den);
+        if (POT)
+            il -= dot(m, dv[i]) * term;  // m.(P - point of the edge)
+        if (FIELD)
+            iv = iv + term * m;
+    }
+    const double N = ah * w[wArea];
+    const double d01 = dot(dv[0], dv[1]), d12 = dot(dv[1], dv[2]), d02 = dot(dv[0], dv[2]);
+    double re = r[0] * r[1] * r[2] + d01 * r[2] + d02 * r[1] + d12 * r[0], im = N;
+    if (NV == 4) {
+        const double d23 = dot(dv[2], dv[NV - 1]), d30 = dot(dv[NV - 1], dv[0]);
+        const double re2 = r[2] * r[NV - 1] * r[0] + d23 * r[0] + d02 * r[NV - 1] + d30 * r[2];
+        im = N * (re + re2);
+        re = re * re2 - N * N;
+    }
+    // the half angle lies in [0, pi]; rounding of im below zero there means pi
+    const double om = copysign(2. * atan2(fmax(im, 0.), re), h);
+    const double k = c_k.one_over_four_pi_eps0;
+    Out4 o{0., 0., 0., 0.};
+    if (POT)
+        o.phi = k * (-h * om - il);
+    if (FIELD) {
+        o.ex = k * (n.x * om + iv.x);
+        o.ey = k * (n.y * om + iv.y);
+        o.ez = k * (n.z * om + iv.z);
+    }
+    return o;
 }
 
 // ------------------------------------------------------------------------- line segments

@@ -412,7 +412,7 @@ __device__ __forceinline__ void fm_l2p(const double* Lh, int p, double ux, doubl
     double sr = 1., si = 0.;
     for (int m = 0; m <= p; m++) {
         if (m > 0) {
-            const double c = -sqrt((2. * m - 1.) / (2. * m));
+            const double c = -c_rt[2 * m - 1] * c_irt[2 * m];
             const double tr = c * (ux * sr - uy * si), ti = c * (ux * si + uy * sr);
             sr = tr;
             si = ti;
@@ -423,14 +423,14 @@ __device__ __forceinline__ void fm_l2p(const double* Lh, int p, double ux, doubl
             if (n > m) {
                 double nr, ni;
                 if (n == m + 1) {
-                    const double c = sqrt(2. * m + 1.) * uz;
+                    const double c = c_rt[2 * m + 1] * uz;
                     nr = c * r1r;
                     ni = c * r1i;
                 }
                 else {
-                    const double inv = 1. / sqrt((double) (n - m) * (n + m));
+                    const double inv = c_irt[n - m] * c_irt[n + m];
                     const double c1 = (2. * n - 1.) * uz * inv;
-                    const double c2 = sqrt((double) (n + m - 1) * (n - m - 1)) * r2 * inv;
+                    const double c2 = c_rt[n + m - 1] * c_rt[n - m - 1] * r2 * inv;
                     nr = c1 * r1r - c2 * r0r;
                     ni = c1 * r1i - c2 * r0i;
                 }
@@ -444,17 +444,17 @@ __device__ __forceinline__ void fm_l2p(const double* Lh, int p, double ux, doubl
             const double lr = Lh[fm_re(n, m)], li = m ? Lh[fm_im(n, m)] : 0.;
             phi += w * (lr * Rr - li * Ri);
             if (n < p) {
-                const double a = sqrt((double) (n + 1 - m) * (n + 1 + m));
+                const double a = c_rt[n + 1 - m] * c_rt[n + 1 + m];
                 const double zr = Lh[fm_re(n + 1, m)], zi = m ? Lh[fm_im(n + 1, m)] : 0.;
                 dz += w * a * (zr * Rr - zi * Ri);
                 if (m >= 1) {
-                    const double b = sqrt((double) (n + 2 - m) * (n + 1 - m));
+                    const double b = c_rt[n + 2 - m] * c_rt[n + 1 - m];
                     const double qr = Lh[fm_re(n + 1, m - 1)], qi = m - 1 ? Lh[fm_im(n + 1, m - 1)] : 0.;
                     dpr += b * (qr * Rr - qi * Ri);
                     dpi += b * (qr * Ri + qi * Rr);
                 }
                 {
-                    const double c = sqrt((double) (n + m + 2) * (n + m + 1));
+                    const double c = c_rt[n + m + 2] * c_rt[n + m + 1];
                     const double qr = Lh[fm_re(n + 1, m + 1)], qi = Lh[fm_im(n + 1, m + 1)];
                     // - conj(L) c conj(R) = -c conj(L R)
                     dpr -= c * (qr * Rr - qi * Ri);
@@ -496,7 +496,8 @@ struct FmTreeView
 constexpr int kFmEvalMinBlocks = 4, kFmMatvecMinBlocks = 5;
 
 template<bool POT, bool FIELD, bool ANALYTIC>
-__global__ void __launch_bounds__(128, kFmEvalMinBlocks) fm_eval_kernel(const double* __restrict__ rec, const double* __restrict__ src,
+__global__ void __launch_bounds__(128, kFmEvalMinBlocks) fm_eval_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
+                                                      const double* __restrict__ src,
                                                       const double* __restrict__ P, const int* __restrict__ run_key,
                                                       const int* __restrict__ run_off, const int* __restrict__ run_cnt,
                                                       int first_run, FmTreeView T, int p,
@@ -540,9 +541,10 @@ __global__ void __launch_bounds__(128, kFmEvalMinBlocks) fm_eval_kernel(const do
                             Out4 v;
                             if (ANALYTIC) {
                                 const int type = (int) r[rType];
+                                const double* w = rwg + (size_t) e * wRecSize;
                                 v = type == kLineSegment ? line_analytic<POT, FIELD>(r, x)
-                                    : type == kTriangle  ? rwg64<3, POT, FIELD>(r, x)
-                                                         : rwg64<4, POT, FIELD>(r, x);
+                                    : type == kTriangle  ? rwg_pair<3, POT, FIELD>(r, w, x)
+                                                         : rwg_pair<4, POT, FIELD>(r, w, x);
                             }
                             else
                                 v = epi<false, POT, FIELD>(r, x);

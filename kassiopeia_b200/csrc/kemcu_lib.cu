@@ -62,6 +62,7 @@ struct kemcu_ctx
     double* d_rec = nullptr;
     TargetRec* d_tgt = nullptr;
     double* d_sigma = nullptr;
+    double* d_rwg = nullptr;  // near records (rwg_build_kernel)
     bool have_sigma = false;
     // all elements axisymmetric (conic sections, rings): records in the AxRec layout
     bool axisym = false;
@@ -1210,6 +1211,13 @@ int kemcu_create(kemcu_ctx** out, const kemcu_config* cfg)
     }
     KC(cudaMemcpyToSymbol(c_gl, gl.data(), gl.size() * sizeof(double)));
     KC(cudaMemcpyToSymbol(c_k, &ctx->k, sizeof(Constants)));
+    double rt[kNumRoots], irt[kNumRoots];
+    for (int i = 0; i < kNumRoots; i++) {
+        rt[i] = std::sqrt((double) i);
+        irt[i] = i ? 1. / std::sqrt((double) i) : 0.;
+    }
+    KC(cudaMemcpyToSymbol(c_rt, rt, sizeof rt));
+    KC(cudaMemcpyToSymbol(c_irt, irt, sizeof irt));
     double rk[kStages][kStages];
     rk8_table(rk);
     KC(cudaMemcpyToSymbol(c_rk8, rk, sizeof rk));
@@ -1234,6 +1242,7 @@ int kemcu_destroy(kemcu_ctx* ctx)
         cudaFree(ctx->d_near_ptr);
         cudaFree(ctx->d_near_row);
         cudaFree(ctx->d_near_val);
+        cudaFree(ctx->d_rwg);
         cudaFree(ctx->d_counter);
         cudaFree(ctx->d_flag);
         fm_release(ctx);
@@ -1303,6 +1312,7 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     cudaFree(ctx->d_near_ptr);
     cudaFree(ctx->d_near_row);
     cudaFree(ctx->d_near_val);
+    cudaFree(ctx->d_rwg);
     ctx->d_rec = nullptr;
     ctx->d_tgt = nullptr;
     ctx->d_sigma = nullptr;
@@ -1311,6 +1321,7 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     ctx->d_near_ptr = nullptr;
     ctx->d_near_row = nullptr;
     ctx->d_near_val = nullptr;
+    ctx->d_rwg = nullptr;
     ctx->have_sigma = false;
     ctx->n = 0;
     ctx->h_rec.assign(n * rRecSize, 0.);
@@ -1332,6 +1343,11 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     KC(cudaMemcpy(ctx->d_rec, ctx->h_rec.data(), n * rRecSize * sizeof(double), cudaMemcpyHostToDevice));
     KC(cudaMemcpy(ctx->d_tgt, ctx->h_tgt.data(), n * sizeof(TargetRec), cudaMemcpyHostToDevice));
     KC(cudaMemset(ctx->d_sigma, 0, n * sizeof(double)));
+    if (!ctx->axisym) {
+        KC(cudaMalloc(&ctx->d_rwg, n * wRecSize * sizeof(double)));
+        rwg_build_kernel<<<(unsigned) ((n + 127) / 128), 128, 0, ctx->stream>>>(ctx->d_rec, (int) n, ctx->d_rwg);
+        KCHECK_LAUNCH();
+    }
     ctx->n = n;
     return KEMCU_OK;
 }
