@@ -887,18 +887,6 @@ __device__ __forceinline__ Out4 epi_far(const double* e, V3 P, V3 d, double r2, 
     return band == 2 ? cubq_pairs<6, kPair12, -1, POT, FIELD, MIXED>(e, d, r2) : cubq_pairs<3, kPair7, 0, POT, FIELD, MIXED>(e, d, r2);
 }
 
-// epi for a pair known to lie outside the analytic band (the caller has shown that its centre
-// distance exceeds the band-0 cut): the same band decision and quadrature as epi, with no call
-// to the analytic integrals in the code path
-template<bool MIXED, bool POT, bool FIELD, bool F32 = false> __device__ __forceinline__ Out4 epi_beyond_near(const double* e,
-                                                                                                           V3 P)
-{
-    V3 d;
-    double r2;
-    const int band = band_of(e, P, d, r2);
-    return epi_far<MIXED, POT, FIELD, F32>(e, P, d, r2, band);
-}
-
 template<bool MIXED, bool POT, bool FIELD, bool F32 = false> __device__ __forceinline__ Out4 epi(const double* e, V3 P)
 {
     V3 d;
@@ -909,6 +897,29 @@ template<bool MIXED, bool POT, bool FIELD, bool F32 = false> __device__ __forcei
         if (type == kLineSegment)
             return line_analytic<POT, FIELD>(e, P);
         return type == kTriangle ? rwg64<3, POT, FIELD>(e, P) : rwg64<4, POT, FIELD>(e, P);
+    }
+    return epi_far<MIXED, POT, FIELD, F32>(e, P, d, r2, band);
+}
+
+// epi with the analytic band from the element's near record w (rwg_build_kernel). Not inlined: the
+// kernels whose distant pairs take the series call it for the few that remain, and carry none of its
+// registers in their loops.
+template<int NV, bool POT, bool FIELD>
+__device__ __noinline__ Out4 rwg_call(const double* __restrict__ e, const double* __restrict__ w, V3 P)
+{
+    return rwg_pair<NV, POT, FIELD>(e, w, P);
+}
+template<bool MIXED, bool POT, bool FIELD, bool F32 = false>
+__device__ __noinline__ Out4 epi(const double* __restrict__ e, const double* __restrict__ w, V3 P)
+{
+    V3 d;
+    double r2;
+    const int band = band_of(e, P, d, r2);
+    if (band == 0) {
+        const int type = (int) e[rType];
+        if (type == kLineSegment)
+            return line_analytic<POT, FIELD>(e, P);
+        return type == kTriangle ? rwg_call<3, POT, FIELD>(e, w, P) : rwg_call<4, POT, FIELD>(e, w, P);
     }
     return epi_far<MIXED, POT, FIELD, F32>(e, P, d, r2, band);
 }

@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(128, kFmEvalMinBlocks) fm_eval_kernel(const do
                                                          : rwg_pair<4, POT, FIELD>(r, w, x);
                             }
                             else
-                                v = epi<false, POT, FIELD>(r, x);
+                                v = epi<false, POT, FIELD>(r, rwg + (size_t) e * wRecSize, x);
                             const double sg = src[e];
                             const double t4[4] = {v.ex * sg, v.ey * sg, v.ez * sg, v.phi * sg};
 #pragma unroll
@@ -579,6 +579,7 @@ __global__ void __launch_bounds__(128, kFmEvalMinBlocks) fm_eval_kernel(const do
 // (bounded for 5 resident CTAs: 7.35 ms per coax matvec against 8.9 ms unbounded, 7.6 at 4)
 template<int NR>
 __global__ void __launch_bounds__(128, kFmMatvecMinBlocks) fm_matvec_kernel(const double* __restrict__ rec,
+                                                        const double* __restrict__ rwg,
                                                         const TargetRec* __restrict__ tgt,
                                                         const int* __restrict__ tgt_order,
                                                         const int* __restrict__ run_key, const int* __restrict__ run_off,
@@ -622,7 +623,7 @@ __global__ void __launch_bounds__(128, kFmMatvecMinBlocks) fm_matvec_kernel(cons
                         const int e0 = T.own_ptr[ci], e1 = T.own_ptr[ci + 1];
                         for (int j = e0; j < e1; j++) {
                             const int e = T.own_elem[j];
-                            const double a = entry<false>(rec + (size_t) e * rRecSize, t, C);
+                            const double a = entry<false>(rec + (size_t) e * rRecSize, rwg + (size_t) e * wRecSize, t, C);
 #pragma unroll
                             for (int r = 0; r < NR; r++)
                                 if (r < nrhs) {
@@ -662,6 +663,7 @@ struct FmNear
 // the entries entry() of every run's targets with its direct elements; one CTA per run, its
 // threads over the (element, target) pairs of the run
 __global__ void __launch_bounds__(256) fm_near_fill_kernel(const double* __restrict__ rec,
+                                                           const double* __restrict__ rwg,
                                                            const TargetRec* __restrict__ tgt,
                                                            const int* __restrict__ tgt_order,
                                                            const int* __restrict__ run_off,
@@ -679,7 +681,8 @@ __global__ void __launch_bounds__(256) fm_near_fill_kernel(const double* __restr
     for (long long q = threadIdx.x; q < pairs; q += blockDim.x) {
         const int j = (int) (q / cnt), k = (int) (q % cnt);
         const TargetRec t = tgt[tgt_order[off + k]];
-        vb[q] = entry<false>(rec + (size_t) cb[j] * rRecSize, t, v3(t.cen[0], t.cen[1], t.cen[2]));
+        vb[q] = entry<false>(rec + (size_t) cb[j] * rRecSize, rwg + (size_t) cb[j] * wRecSize, t,
+                             v3(t.cen[0], t.cen[1], t.cen[2]));
     }
 }
 

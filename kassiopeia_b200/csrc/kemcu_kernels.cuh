@@ -14,11 +14,15 @@
 #pragma once
 
 #include "kemcu_device.cuh"
+#include "kemcu_series.cuh"
 
 namespace kemcu
 {
 
-constexpr int kThreads = 128;
+#ifndef KEMCU_THREADS
+#define KEMCU_THREADS 128
+#endif
+constexpr int kThreads = KEMCU_THREADS;
 // resident CTAs per SM the direct-sum kernels are compiled for (bounds their registers)
 #ifndef KEMCU_MIN_BLOCKS
 #define KEMCU_MIN_BLOCKS 5
@@ -67,7 +71,7 @@ __device__ __forceinline__ void load_tile(double* sm, const double* __restrict__
 #define KEMCU_FIELD_TILE 32
 #endif
 #ifndef KEMCU_PIPE
-#define KEMCU_PIPE 4
+#define KEMCU_PIPE 3
 #endif
 constexpr int kFieldTile = KEMCU_FIELD_TILE;
 constexpr int kPipe = KEMCU_PIPE;
@@ -269,15 +273,111 @@ template<int SIDE, int NP = kPipe, bool CYCLIC = false> struct ElementRing
     }
 };
 
-// A warp's points in a bounding sphere, and whether a tile of the element ring holds an element
-// within its analytic band of any of them: the element's centre distance from the sphere's
-// centre, less the radius and a 1e-12 rounding allowance, squared, must exceed the band-0 cut with
-// a 1e-6 margin for the tile to be far (then the fast band comparison of band_of decides band >= 1
-// for every pair, as the exact one would). Called by all 32 lanes.
-__device__ __forceinline__ void warp_sphere(bool active, V3 P, V3& wc, double& wr)
+// The same ring over the far records (kemcu_series.cuh), tile by tile of the tile table: a stage
+// holds one tile's records, its descriptor and SIDE doubles of side data per element. The CTA's
+// slice is a range of tiles, split over gridDim.y.
+template<int SIDE, int NP> struct FarRingStorage
 {
-    double lo[3] = {active ? P.x : 1e300, active ? P.y : 1e300, active ? P.z : 1e300};
-    double hi[3] = {active ? P.x : -1e300, active ? P.y : -1e300, active ? P.z : -1e300};
+    double rec[NP][kFarStage];
+    double side[NP][SIDE > 0 ? SIDE : 1][kFarSym];
+    FarTile tile[NP];
+    unsigned long long full[NP];
+    unsigned rel[NP], used[NP];
+};
+
+template<int SIDE, int NP> struct FarRing
+{
+    FarRingStorage<SIDE, NP>& S;
+    const double* far;
+    const FarTile* table;
+    int t0, t1;  // this CTA's tiles
+
+    __device__ __forceinline__ FarRing(FarRingStorage<SIDE, NP>& storage, const double* far_, const FarTile* table_,
+                                       int ntiles)
+        : S(storage), far(far_), table(table_)
+    {
+        const int per = (ntiles + (int) gridDim.y - 1) / (int) gridDim.y;
+        t0 = min(ntiles, (int) blockIdx.y * per);
+        t1 = min(ntiles, t0 + per);
+        if (threadIdx.x < NP) {
+            mbar_init(&S.full[threadIdx.x], 32);
+            S.rel[threadIdx.x] = 0u;
+            S.used[threadIdx.x] = 0u;
+            mbar_init_fence();
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ int tiles() const
+    {
+        return t1 - t0;
+    }
+    // fill stage i % NP with tile i of the slice: called by all 32 lanes of one warp
+    template<class F> __device__ __forceinline__ void fill(int i, F side_fn)
+    {
+        const int s = i % NP, lane = threadIdx.x & 31;
+        const FarTile T = table[t0 + i];
+        side_fn(S.side[s], T.first, T.count, lane);
+        if (lane == 0) {
+            S.tile[s] = T;
+            S.used[s]++;
+            fence_proxy_async();
+            const unsigned bytes = (unsigned) (T.count * (T.general ? kFarGenStride : kFarSymStride) * sizeof(double));
+            mbar_arrive_tx(&S.full[s], bytes);
+            bulk_g2s(S.rec[s], far + 2 * (size_t) T.off16, bytes, &S.full[s]);
+        }
+        else
+            mbar_arrive(&S.full[s]);
+    }
+    template<class F> __device__ __forceinline__ void prologue(F side_fn)
+    {
+        if (threadIdx.x < 32)
+            for (int i = 0; i < min(NP, tiles()); i++)
+                fill(i, side_fn);
+    }
+    __device__ __forceinline__ bool wait(int i)
+    {
+        return mbar_wait(&S.full[i % NP], (unsigned) (i / NP) & 1u);
+    }
+    // whole warp: release tile i; the warp that releases a stage last refills it
+    template<class F> __device__ __forceinline__ void release(int i, F side_fn)
+    {
+        const int s = i % NP;
+        __syncwarp();
+        unsigned last = 0u;
+        if ((threadIdx.x & 31) == 0) {
+            __threadfence_block();
+            last = atomicAdd(&S.rel[s], 1u) % (blockDim.x >> 5) == (blockDim.x >> 5) - 1u;
+        }
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (last && i + NP < tiles()) {
+            __threadfence_block();
+            fill(i + NP, side_fn);
+        }
+    }
+    // after the tile loop (all threads): report a timed-out wait in flag (|= 2) and wait,
+    // bounded, for copies still in flight
+    __device__ __forceinline__ void finish(bool ok, int* flag)
+    {
+        if (!ok && (threadIdx.x & 31) == 0)
+            atomicOr(flag, 2);
+        __syncthreads();
+        if (threadIdx.x < NP && S.used[threadIdx.x] > 0u)
+            mbar_wait(&S.full[threadIdx.x], (S.used[threadIdx.x] - 1u) & 1u);
+    }
+};
+
+// A warp's points (NP per lane) in a bounding sphere. Called by all 32 lanes.
+template<int NP> __device__ __forceinline__ void warp_sphere(const V3 (&P)[NP], V3& wc, double& wr)
+{
+    double lo[3] = {P[0].x, P[0].y, P[0].z}, hi[3] = {P[0].x, P[0].y, P[0].z};
+#pragma unroll
+    for (int p = 1; p < NP; p++) {
+        const double v[3] = {P[p].x, P[p].y, P[p].z};
+        for (int c = 0; c < 3; c++) {
+            lo[c] = fmin(lo[c], v[c]);
+            hi[c] = fmax(hi[c], v[c]);
+        }
+    }
     for (int o = 16; o > 0; o >>= 1)
         for (int c = 0; c < 3; c++) {
             lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
@@ -287,111 +387,323 @@ __device__ __forceinline__ void warp_sphere(bool active, V3 P, V3& wc, double& w
     wr = 0.5 * sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
                     (hi[2] - lo[2]) * (hi[2] - lo[2]));
 }
-template<class Ring> __device__ __forceinline__ bool tile_near(const Ring& R, int i, int cnt, V3 wc, double wr)
+
+// The context's far records as the kernels take them
+struct FarView
 {
-    bool near = false;
-    for (int j = (int) (threadIdx.x & 31); j < cnt; j += 32) {
-        const double* e = R.element(i, j);
-        const double dx = e[rCen] - wc.x, dy = e[rCen + 1] - wc.y, dz = e[rCen + 2] - wc.z;
-        const double dist = sqrt(dx * dx + dy * dy + dz * dz);
-        const double dm = dist - wr - 1e-12 * (dist + wr);
-        near = near || !(dm > 0. && dm * dm > e[rCut] * (1. + 1e-6));
+    const double* far;     // records, tile by tile
+    const FarTile* tiles;
+    int ntiles;
+    const double* pre;     // total charge per unit density over (4 pi eps0), per element
+    const double* rwg;     // near records, wRecSize doubles per element
+};
+
+// a warp's list of the elements it leaves to the cubature bands and the analytic integrals. The
+// series loops then contain no call and none of that code's registers. The list is worked off
+// between tiles whenever another tile might not fit, the element records kNearStage at a time through
+// shared memory: their loads run ahead of the pairs, which would otherwise wait for L2 once per element.
+constexpr int kNearList = 64, kNearStage = 2;
+struct NearStore
+{
+    double rec[kNearStage][rRecSize];
+    int e[kNearList];
+};
+struct NearList
+{
+    NearStore& S;
+    int n;
+    __device__ __forceinline__ bool full() const
+    {
+        return n > kNearList - kFarSym;
     }
-    return __any_sync(0xffffffffu, near);
+    // one(e, record) for every element of the list; empties it. All 32 lanes.
+    template<class F> __device__ __forceinline__ void drain(const double* __restrict__ rec, F one)
+    {
+        static_assert(rRecSize == 32, "a lane per double of a record");
+        const int lane = threadIdx.x & 31;
+        __syncwarp();
+        double v[kNearStage];
+        auto fetch = [&](int q0) {
+#pragma unroll
+            for (int k = 0; k < kNearStage; k++)
+                if (q0 + k < n)
+                    v[k] = rec[(size_t) S.e[q0 + k] * rRecSize + lane];
+        };
+        fetch(0);
+        for (int q0 = 0; q0 < n; q0 += kNearStage) {
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < kNearStage; k++)
+                if (q0 + k < n)
+                    S.rec[k][lane] = v[k];
+            __syncwarp();
+            fetch(q0 + kNearStage);
+            for (int k = 0; k < min(kNearStage, n - q0); k++)
+                one(S.e[q0 + k], S.rec[k]);
+        }
+        __syncwarp();
+        n = 0;
+    }
+};
+
+// Points per lane of the pair kernels: two share every coefficient read from shared memory (the
+// loads were a quarter of the instructions with one) and give each other's chains room
+#ifndef KEMCU_PAIR
+#define KEMCU_PAIR 1
+#endif
+constexpr int kPair = KEMCU_PAIR;
+
+template<int T> struct Tier
+{
+    static constexpr int value = T;
+};
+
+// The elements of one tile against a warp's points (NP per lane), each by the cheapest series that
+// holds for all of them, so that the choice is uniform: far(f, j, p, F, d) receives element j's sums
+// for point p (f: its record, d: the point relative to its centroid); elements without one go to the list. A lane per element finds the tier for the warp's
+// bounding sphere; an element whose tier that leaves open is tested point by point.
+template<bool FIELD, bool FAST, int NP, class Far>
+__device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, const V3 (&P)[NP], V3 wc, double wr,
+                                           NearList& L, Far far)
+{
+    const int lane = threadIdx.x & 31;
+    const int stride = T.general ? kFarGenStride : kFarSymStride;
+    const int tier = lane < T.count ? far_tier<FAST>(rec + lane * stride, wc, wr) : 0;
+    const unsigned m3 = __ballot_sync(0xffffffffu, tier == 3), m2 = __ballot_sync(0xffffffffu, tier == 2);
+    unsigned m1 = __ballot_sync(0xffffffffu, tier == 1);
+    for (unsigned m = ~(m1 | m2 | m3) & ((1u << T.count) - 1u); m; m &= m - 1u) {
+        const int j = __ffs(m) - 1;
+        const double* f = rec + j * stride;
+        bool low = true;
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+            low = low && far_point<FAST>(f, P[p]);
+        if (__all_sync(0xffffffffu, low))
+            m1 |= 1u << j;
+        else {
+            if (lane == 0)
+                L.S.e[L.n] = T.first + j;
+            L.n++;
+        }
+    }
+    // the field of general elements, whose sums take the most registers, point by point
+    constexpr int NG = FIELD ? 1 : NP;
+    auto general = [&](auto tier, unsigned m) {
+        for (; m; m &= m - 1u) {
+            const int j = __ffs(m) - 1;
+            const double* f = rec + j * kFarGenStride;
+#pragma unroll
+            for (int p0 = 0; p0 < NP; p0 += NG) {
+                V3 Q[NG], d[NG];
+                FarSum F[NG];
+#pragma unroll
+                for (int p = 0; p < NG; p++)
+                    Q[p] = P[p0 + p];
+                far_pairs<true, decltype(tier)::value, FIELD, FAST>(f, Q, d, F);
+#pragma unroll
+                for (int p = 0; p < NG; p++)
+                    far(f, j, p0 + p, F[p], d[p]);
+            }
+        }
+    };
+    auto symmetric = [&](auto tier, unsigned m) {
+        for (; m; m &= m - 1u) {
+            const int j = __ffs(m) - 1;
+            const double* f = rec + j * kFarSymStride;
+            V3 d[NP];
+            FarSum F[NP];
+            far_pairs<false, decltype(tier)::value, FIELD, FAST>(f, P, d, F);
+#pragma unroll
+            for (int p = 0; p < NP; p++)
+                far(f, j, p, F[p], d[p]);
+        }
+    };
+    if (T.general) {
+        general(Tier<3>(), m3);
+        general(Tier<2>(), m2);
+        general(Tier<1>(), m1);
+    }
+    else {
+        symmetric(Tier<3>(), m3);
+        symmetric(Tier<2>(), m2);
+        symmetric(Tier<1>(), m1);
+    }
 }
 
+// compensated sums of a CTA's threads in shared memory (touched once per tile): NS sums of kPair points
+template<int NS> struct KahanStore
+{
+    double s[NS * kPair][kThreads], c[NS * kPair][kThreads];
+    __device__ __forceinline__ void clear()
+    {
+        for (int k = 0; k < NS * kPair; k++)
+            s[k][threadIdx.x] = c[k][threadIdx.x] = 0.;
+    }
+    __device__ __forceinline__ void add(int k, double v)
+    {
+        const double s0 = s[k][threadIdx.x], y = v - c[k][threadIdx.x], t = s0 + y;
+        c[k][threadIdx.x] = (t - s0) - y;
+        s[k][threadIdx.x] = t;
+    }
+    __device__ __forceinline__ double get(int k) const
+    {
+        return s[k][threadIdx.x];
+    }
+};
+
 // K1: field and/or potential at points. out layout per point: (Ex, Ey, Ez, phi).
-// The analytic near-field pairs (band 0: RWG triangles and rectangles, analytic wires) are
-// evaluated in place through a non-inlined call: a design with a call-free quadrature kernel and
-// a second kernel for the analytic pairs was built and measured slower (the near pass ran alone,
-// latency-bound, where here its latency hides behind other warps' quadrature work).
+// Distant pairs by the far-field series, the others by the cubature bands or the analytic integrals,
+// from the element records in global memory (L1 / L2: few pairs). A warp takes kPair x 32
+// consecutive points. Sums are plain within a tile (and within a near list), compensated across.
 // nsplit == gridDim.y; partial != nullptr when nsplit > 1 (then out is untouched).
 // flag |= 2 if a pipeline wait timed out (the outputs are then incomplete).
-// MINB (resident CTAs per SM the registers are bounded for) and NP (ring stages) are the shapes
-// the autotuner chooses between (field_variants); neither changes an operation or its order, so
-// every variant gives the same result bit for bit. F32: the FP32 far-field form of the cubature
-// bands (precision KEMCU_FP32), the tile and Kahan sums staying FP64.
-template<bool MIXED, bool POT, bool FIELD, int MINB = kMinBlocks, int NP = kPipe, bool F32 = false>
-__global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __restrict__ rec, const double* __restrict__ sigma,
-                                                               int n_elem, const double* __restrict__ pts, int n_pts,
+// MINB (resident CTAs per SM the registers are bounded for) is the shape the autotuner chooses
+// (field_variants); it changes no operation and no order, so every variant gives the same result bit
+// for bit. F32: the FP32 form of the cubature bands (precision KEMCU_FP32), the series, the tile and
+// Kahan sums staying as they are.
+template<bool MIXED, bool POT, bool FIELD, int MINB = kMinBlocks, bool F32 = false>
+__global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __restrict__ rec, FarView V,
+                                                               const double* __restrict__ sigma,
+                                                               const double* __restrict__ pts, int n_pts,
                                                                double* __restrict__ out, double* __restrict__ partial,
                                                                int* __restrict__ flag)
 {
-    __shared__ __align__(128) RingStorage<1, NP> S;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = p < n_pts;
-    V3 P = v3(0., 0., 0.);
-    if (active)
-        P = v3(pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]);
-    ElementRing<1, NP> R(S, 0, n_elem);
-    auto side = [&](double (*sd)[kFieldTile], int t0, int cnt, int lane) {
+    constexpr int NS = (FIELD ? 3 : 0) + (POT ? 1 : 0), kPhi = FIELD ? 3 : 0;
+    __shared__ __align__(128) FarRingStorage<1, kPipe> S;
+    __shared__ KahanStore<NS> K;
+    __shared__ NearStore s_near[kThreads / 32];
+    const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
+    const bool busy = base - (int) (threadIdx.x & 31) < n_pts;  // the warp has points
+    V3 P[kPair];
+#pragma unroll
+    for (int p = 0; p < kPair; p++) {  // lanes past the last point repeat it
+        const size_t pi = 3 * (size_t) min(base + 32 * p, n_pts - 1);
+        P[p] = v3(pts[pi], pts[pi + 1], pts[pi + 2]);
+    }
+    FarRing<1, kPipe> R(S, V.far, V.tiles, V.ntiles);
+    auto side = [&](double (*sd)[kFarSym], int first, int cnt, int lane) {
         if (lane < cnt)
-            sd[0][lane] = sigma[t0 + lane];
+            sd[0][lane] = sigma[first + lane] * V.pre[first + lane];
     };
-    R.prologue(rec, side);
+    R.prologue(side);
     const int ntiles = R.tiles();
-    // the warp's points in a bounding sphere (no sphere without active lanes, and then every
-    // tile takes the general path)
     V3 wc;
     double wr;
-    warp_sphere(active, P, wc, wr);
-    const bool warp_active = __any_sync(0xffffffffu, active);
-    Kahan kx, ky, kz, kp;
+    warp_sphere(P, wc, wr);
+    K.clear();
+    NearList L{s_near[warp], 0};
+    double t[NS][kPair];
+    auto clear = [&]() {
+#pragma unroll
+        for (int k = 0; k < NS; k++)
+#pragma unroll
+            for (int p = 0; p < kPair; p++)
+                t[k][p] = 0.;
+    };
+    auto keep = [&]() {
+#pragma unroll
+        for (int k = 0; k < NS; k++)
+#pragma unroll
+            for (int p = 0; p < kPair; p++)
+                K.add(k * kPair + p, t[k][p]);
+    };
+    auto near = [&]() {
+        clear();
+        L.drain(rec, [&](int e, const double* r) {
+            const double sg = sigma[e];
+            for (int p = 0; p < kPair; p++) {
+                const Out4 v = epi<MIXED, POT, FIELD, F32>(r, V.rwg + (size_t) e * wRecSize, p == 0 ? P[0] : P[kPair - 1]);
+                const double w[4] = {v.ex * sg, v.ey * sg, v.ez * sg, v.phi * sg};
+#pragma unroll
+                for (int k = 0; k < NS; k++) {
+                    const double wk = k == kPhi ? w[3] : w[k];
+                    if (p == 0)
+                        t[k][0] += wk;
+                    else
+                        t[k][kPair - 1] += wk;
+                }
+            }
+        });
+        keep();
+    };
     bool ok = true;
     for (int i = 0; i < ntiles; i++) {
-        if (!R.wait(i)) {
+        if (!__all_sync(0xffffffffu, R.wait(i))) {
             ok = false;
             break;
         }
-        const int cnt = R.count(i);
-        // far tile: every element of the tile is beyond its analytic band for every point of the
-        // warp, so the pair loop needs no analytic call
-        const bool near = !warp_active || tile_near(R, i, cnt, wc, wr);
-        if (active) {
-            double tx = 0., ty = 0., tz = 0., tp = 0.;
-            if (!near) {
-                for (int j = 0; j < cnt; j++) {
-                    const Out4 r = epi_beyond_near<MIXED, POT, FIELD, F32>(R.element(i, j), P);
-                    const double sg = R.side(i, 0, j);
-                    if (FIELD) {
-                        tx = fma(r.ex, sg, tx);
-                        ty = fma(r.ey, sg, ty);
-                        tz = fma(r.ez, sg, tz);
-                    }
+        if (busy) {
+            const FarTile T = S.tile[i % kPipe];
+            const double* sp = S.side[i % kPipe][0];
+            clear();
+            tile_pairs<FIELD, MIXED || F32>(
+                S.rec[i % kPipe], T, P, wc, wr, L,
+                [&](const double* f, int j, int p, const FarSum& F, V3 d) {
+                    const double q = sp[j] * F.ir;
                     if (POT)
-                        tp = fma(r.phi, sg, tp);
-                }
-            }
-            else
-                for (int j = 0; j < cnt; j++) {
-                    const Out4 r = epi<MIXED, POT, FIELD, F32>(R.element(i, j), P);
-                    const double sg = R.side(i, 0, j);
+                        t[kPhi][p] = fma(q, F.S, t[kPhi][p]);
                     if (FIELD) {
-                        tx = fma(r.ex, sg, tx);
-                        ty = fma(r.ey, sg, ty);
-                        tz = fma(r.ez, sg, tz);
+                        const double k = q * F.ir, a = (k * F.ir) * F.cd, b = -k * F.c1, c = -k * F.c2;
+                        const V3 e1 = ld3(f + fE1), e2 = ld3(f + fE1 + 3);
+                        t[0][p] = fma(a, d.x, fma(b, e1.x, fma(c, e2.x, t[0][p])));
+                        t[1][p] = fma(a, d.y, fma(b, e1.y, fma(c, e2.y, t[1][p])));
+                        t[2][p] = fma(a, d.z, fma(b, e1.z, fma(c, e2.z, t[2][p])));
                     }
-                    if (POT)
-                        tp = fma(r.phi, sg, tp);
-                }
-            if (FIELD) {
-                kx.add(tx);
-                ky.add(ty);
-                kz.add(tz);
-            }
-            if (POT)
-                kp.add(tp);
+                });
+            keep();
+            if (L.full())
+                near();
         }
-        R.release(rec, i, side);
+        R.release(i, side);
     }
     R.finish(ok, flag);
-    if (!active)
-        return;
-    double* o = partial ? partial + ((size_t) blockIdx.y * n_pts + p) * 4 : out + (size_t) p * 4;
-    o[0] = kx.s;
-    o[1] = ky.s;
-    o[2] = kz.s;
-    o[3] = kp.s;
+    if (L.n > 0)
+        near();
+#pragma unroll
+    for (int p = 0; p < kPair; p++) {
+        const int q = base + 32 * p;
+        if (q < n_pts) {
+            double* o = partial ? partial + ((size_t) blockIdx.y * n_pts + q) * 4 : out + (size_t) q * 4;
+            o[0] = FIELD ? K.get(p) : 0.;
+            o[1] = FIELD ? K.get(kPair + p) : 0.;
+            o[2] = FIELD ? K.get(2 * kPair + p) : 0.;
+            o[3] = POT ? K.get(kPhi * kPair + p) : 0.;
+        }
+    }
+}
+
+// a few points (one probe): a thread per element and point instead of a lane per point, whose
+// other lanes would repeat it. Each CTA sums kFewElems elements for one point; the sums of the CTAs
+// are added in order by reduce_splits.
+constexpr int kFewPoints = 8, kFewElems = 128;
+template<bool MIXED, bool POT, bool FIELD, bool F32>
+__global__ void __launch_bounds__(kFewElems) field_few_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
+                                                              const double* __restrict__ sigma, int n_elem,
+                                                              const double* __restrict__ pts, int n_pts,
+                                                              double* __restrict__ partial)
+{
+    __shared__ double s_w[4][kFewElems / 32];
+    const int e = blockIdx.y * kFewElems + threadIdx.x, q = blockIdx.x;
+    const V3 P = v3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]);
+    double v[4] = {0., 0., 0., 0.};
+    if (e < n_elem) {
+        const Out4 r = epi<MIXED, POT, FIELD, F32>(rec + (size_t) e * rRecSize, rwg + (size_t) e * wRecSize, P);
+        const double sg = sigma[e];
+        v[0] = r.ex * sg, v[1] = r.ey * sg, v[2] = r.ez * sg, v[3] = r.phi * sg;
+    }
+    for (int o = 16; o > 0; o >>= 1)
+        for (int c = 0; c < 4; c++)
+            v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
+    if ((threadIdx.x & 31) == 0)
+        for (int c = 0; c < 4; c++)
+            s_w[c][threadIdx.x >> 5] = v[c];
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        Kahan k;
+        for (int w = 0; w < kFewElems / 32; w++)
+            k.add(s_w[threadIdx.x][w]);
+        partial[((size_t) blockIdx.y * n_pts + q) * 4 + threadIdx.x] = k.s;
+    }
 }
 
 // fixed-order sum of gridDim.y partial results: out[i] = sum_s partial[s][i]
@@ -416,17 +728,17 @@ struct TargetRec
     double neumann;   // 0 Dirichlet, 1 Neumann
 };
 
-// one matrix entry A(i, j) with source record e and target t (F32: the FP32 far-field form of
+// one matrix entry A(i, j) with source record e, near record w and target t (F32: the FP32 form of
 // the cubature bands)
-template<bool MIXED, bool F32 = false> __device__ __forceinline__ double entry(const double* e, const TargetRec& t, V3 C)
+template<bool MIXED, bool F32 = false>
+__device__ __forceinline__ double entry(const double* e, const double* w, const TargetRec& t, V3 C)
 {
-    if (t.neumann == 0.) {
-        return epi<MIXED, true, false, F32>(e, C).phi;
-    }
+    if (t.neumann == 0.)
+        return epi<MIXED, true, false, F32>(e, w, C).phi;
     const V3 cs = ld3(e + rCen2);
     const double dist = norm(cs - C);
     if (dist >= 1e-12) {
-        const Out4 r = epi<MIXED, false, true, F32>(e, C);
+        const Out4 r = epi<MIXED, false, true, F32>(e, w, C);
         return r.ex * t.normal[0] + r.ey * t.normal[1] + r.ez * t.normal[2];
     }
     return t.diag;
@@ -444,116 +756,200 @@ __device__ __forceinline__ double entry_far(const double* e, const TargetRec& t,
 }
 
 // one entry A(i, j) (kemcu_matrix_element), the FP64 form the matvec uses
-__global__ void entry_kernel(const double* __restrict__ rec, const TargetRec* __restrict__ tgt, int i, int j,
-                             double* __restrict__ a)
+__global__ void entry_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
+                             const TargetRec* __restrict__ tgt, int i, int j, double* __restrict__ a)
 {
     const TargetRec t = tgt[i];
-    *a = entry<false>(rec + (size_t) j * rRecSize, t, v3(t.cen[0], t.cen[1], t.cen[2]));
+    *a = entry<false>(rec + (size_t) j * rRecSize, rwg + (size_t) j * wRecSize, t, v3(t.cen[0], t.cen[1], t.cen[2]));
+}
+
+constexpr int kMaxRhs = 8;
+
+// the entries of one tile's columns in kPair rows per lane: emit(p, j, A(row p, first + j)). A warp
+// without a Neumann row sums potentials only; Neumann rows take the field along their normal.
+template<bool FAST, class Emit>
+__device__ __forceinline__ void tile_entries(const double* far, const FarTile& T, const double* pre,
+                                             const TargetRec* __restrict__ tgt, const int (&row)[kPair],
+                                             const V3 (&C)[kPair], bool any_neumann, V3 wc, double wr, NearList& L,
+                                             Emit emit)
+{
+    if (!any_neumann)
+        tile_pairs<false, FAST>(far, T, C, wc, wr, L, [&](const double*, int j, int p, const FarSum& F, V3) {
+            emit(p, j, (pre[j] * F.ir) * F.S);
+        });
+    else
+        tile_pairs<true, FAST>(far, T, C, wc, wr, L, [&](const double* f, int j, int p, const FarSum& F, V3 d) {
+            const TargetRec& t = tgt[row[p]];
+            const V3 nn = v3(t.normal[0], t.normal[1], t.normal[2]);
+            const double q = pre[j] * F.ir;
+            const double en = q * F.ir * (F.ir * F.cd * dot(nn, d) - F.c1 * dot(nn, ld3(f + fE1)) -
+                                          F.c2 * dot(nn, ld3(f + fE1 + 3)));
+            emit(p, j, t.neumann == 0. ? q * F.S : en);
+        });
 }
 
 // K2: y[r][i] = sum_j A(i, j) x[r][j] for r < nrhs (nrhs <= NR <= kMaxRhs), entries
 // recomputed on the fly (KMatrix::Multiply over KBoundaryIntegralMatrix::operator(),
-// KMatrix.hh:92-99, KBoundaryIntegralMatrix.hh:31-55). Same element ring as K1, with the
-// operand values of the tile as side data.
-constexpr int kMaxRhs = 8;
+// KMatrix.hh:92-99, KBoundaryIntegralMatrix.hh:31-55). Same pipeline as K1, with the operand values
+// of the tile as side data. rows: the matrix rows in Morton order of their collocation points, so
+// that a warp's rows are near one another and distant elements distant for all of them.
 template<bool MIXED, int NR, bool F32 = false>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) matvec_kernel(const double* __restrict__ rec, const TargetRec* __restrict__ tgt,
-                                                          int n, const double* __restrict__ x, int nrhs,
-                                                          double* __restrict__ y, double* __restrict__ partial,
-                                                          int* __restrict__ flag)
+__global__ void __launch_bounds__(kThreads, NR == 1 ? kMinBlocks : 4)
+    matvec_kernel(const double* __restrict__ rec, FarView V, const TargetRec* __restrict__ tgt,
+                  const int* __restrict__ rows, int n, const double* __restrict__ x, int nrhs, double* __restrict__ y,
+                  double* __restrict__ partial, int* __restrict__ flag)
 {
-    __shared__ __align__(128) RingStorage<NR> S;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
-    TargetRec t{};
-    V3 C = v3(0., 0., 0.);
-    if (active) {
-        t = tgt[i];
-        C = v3(t.cen[0], t.cen[1], t.cen[2]);
+    __shared__ __align__(128) FarRingStorage<NR + 1, kPipe> S;
+    __shared__ NearStore s_near[kThreads / 32];
+    const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
+    const bool busy = base - (int) (threadIdx.x & 31) < n;
+    int row[kPair];
+    V3 C[kPair];
+    bool neumann = false;
+#pragma unroll
+    for (int p = 0; p < kPair; p++) {
+        row[p] = rows[min(base + 32 * p, n - 1)];
+        const TargetRec& t = tgt[row[p]];
+        C[p] = v3(t.cen[0], t.cen[1], t.cen[2]);
+        neumann = neumann || t.neumann != 0.;
     }
-    ElementRing<NR> R(S, 0, n);
-    auto side = [&](double (*sd)[kFieldTile], int t0, int cnt, int lane) {
-        if (lane < cnt)
+    const bool any_neumann = __any_sync(0xffffffffu, neumann);
+    FarRing<NR + 1, kPipe> R(S, V.far, V.tiles, V.ntiles);
+    auto side = [&](double (*sd)[kFarSym], int first, int cnt, int lane) {
+        if (lane < cnt) {
+            sd[NR][lane] = V.pre[first + lane];
             for (int r = 0; r < nrhs; r++)
-                sd[r][lane] = x[(size_t) r * n + t0 + lane];
-    };
-    R.prologue(rec, side);
-    const int ntiles = R.tiles();
-    // (the far-tile split of K1 was built here too and measured slower: the second pair loop
-    // costs this kernel's register allocation more than the call it saves)
-    Kahan acc[NR];
-    bool ok = true;
-    for (int q = 0; q < ntiles; q++) {
-        if (!R.wait(q)) {
-            ok = false;
-            break;
+                sd[r][lane] = x[(size_t) r * n + first + lane];
         }
-        if (active) {
-            const int cnt = R.count(q);
-            for (int j = 0; j < cnt; j++) {
-                const double a = entry<MIXED, F32>(R.element(q, j), t, C);
+    };
+    R.prologue(side);
+    const int ntiles = R.tiles();
+    V3 wc;
+    double wr;
+    warp_sphere(C, wc, wr);
+    NearList L{s_near[warp], 0};
+    Kahan acc[NR][kPair];
+    auto near = [&]() {
+        L.drain(rec, [&](int e, const double* er) {
+#pragma unroll
+            for (int p = 0; p < kPair; p++) {
+                const double* w = V.rwg + (size_t) e * wRecSize;
+                const double a = any_neumann ? entry<MIXED, F32>(er, w, tgt[row[p]], C[p])
+                                             : epi<MIXED, true, false, F32>(er, w, C[p]).phi;
 #pragma unroll
                 for (int r = 0; r < NR; r++)
-                    if (r < nrhs)
-                        acc[r].add(a * R.side(q, r, j));
+                    if (NR == 1 || r < nrhs)
+                        acc[r][p].add(a * x[(size_t) r * n + e]);
             }
-        }
-        R.release(rec, q, side);
-    }
-    R.finish(ok, flag);
-    if (!active)
-        return;
-#pragma unroll
-    for (int r = 0; r < NR; r++) {
-        if (r >= nrhs)
-            break;
-        if (partial)
-            partial[((size_t) blockIdx.y * nrhs + r) * n + i] = acc[r].s;
-        else
-            y[(size_t) r * n + i] = acc[r].s;
-    }
-}
-
-// operator assembly: column-major dense A (A[j * op_ld(n) + i] = A(i, j)) for columns
-// [j0, j1), written in FP64 and, when a32 != nullptr, also rounded to FP32
-template<bool MIXED>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) assemble_kernel(const double* __restrict__ rec, const TargetRec* __restrict__ tgt,
-                                                            int n, int j0, int j1, double* __restrict__ a64,
-                                                            float* __restrict__ a32, int* __restrict__ flag)
-{
-    __shared__ __align__(128) RingStorage<0> S;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
-    TargetRec t{};
-    V3 C = v3(0., 0., 0.);
-    if (active) {
-        t = tgt[i];
-        C = v3(t.cen[0], t.cen[1], t.cen[2]);
-    }
-    ElementRing<0> R(S, j0, j1);
-    auto side = [](double (*)[kFieldTile], int, int, int) {};
-    R.prologue(rec, side);
-    const int ntiles = R.tiles();
+        });
+    };
     bool ok = true;
     for (int q = 0; q < ntiles; q++) {
-        if (!R.wait(q)) {
+        if (!__all_sync(0xffffffffu, R.wait(q))) {
             ok = false;
             break;
         }
-        if (active) {
-            const int t0 = R.first(q), cnt = R.count(q);
-            for (int j = 0; j < cnt; j++) {
-                const double a = entry<MIXED>(R.element(q, j), t, C);
-                const size_t idx = (size_t) (t0 + j - j0) * op_ld(n) + i;
-                if (a64)
-                    a64[idx] = a;
-                if (a32)
-                    a32[idx] = (float) a;
-            }
+        if (busy) {
+            const FarTile T = S.tile[q % kPipe];
+            const double(*sd)[kFarSym] = S.side[q % kPipe];
+            tile_entries<MIXED || F32>(S.rec[q % kPipe], T, sd[NR], tgt, row, C, any_neumann, wc, wr, L,
+                                       [&](int p, int j, double a) {
+#pragma unroll
+                                           for (int r = 0; r < NR; r++)
+                                               if (NR == 1 || r < nrhs)
+                                                   acc[r][p].add(a * sd[r][j]);
+                                       });
+            if (L.full())
+                near();
         }
-        R.release(rec, q, side);
+        R.release(q, side);
     }
     R.finish(ok, flag);
+    if (L.n > 0)
+        near();
+#pragma unroll
+    for (int p = 0; p < kPair; p++)
+        if (base + 32 * p < n)
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                if (NR > 1 && r >= nrhs)
+                    break;
+                if (partial)
+                    partial[((size_t) blockIdx.y * nrhs + r) * n + row[p]] = acc[r][p].s;
+                else
+                    y[(size_t) r * n + row[p]] = acc[r][p].s;
+            }
+}
+
+// operator assembly: column-major dense A (A[j * op_ld(n) + i] = A(i, j)), written in FP64 and, when
+// a32 != nullptr, also rounded to FP32
+template<bool MIXED>
+__global__ void __launch_bounds__(kThreads, kMinBlocks)
+    assemble_kernel(const double* __restrict__ rec, FarView V, const TargetRec* __restrict__ tgt,
+                    const int* __restrict__ rows, int n, double* __restrict__ a64, float* __restrict__ a32,
+                    int* __restrict__ flag)
+{
+    __shared__ __align__(128) FarRingStorage<1, kPipe> S;
+    __shared__ NearStore s_near[kThreads / 32];
+    const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
+    const bool busy = base - (int) (threadIdx.x & 31) < n;
+    int row[kPair];
+    V3 C[kPair];
+    bool neumann = false;
+#pragma unroll
+    for (int p = 0; p < kPair; p++) {
+        row[p] = rows[min(base + 32 * p, n - 1)];
+        const TargetRec& t = tgt[row[p]];
+        C[p] = v3(t.cen[0], t.cen[1], t.cen[2]);
+        neumann = neumann || t.neumann != 0.;
+    }
+    const bool any_neumann = __any_sync(0xffffffffu, neumann);
+    FarRing<1, kPipe> R(S, V.far, V.tiles, V.ntiles);
+    auto side = [&](double (*sd)[kFarSym], int first, int cnt, int lane) {
+        if (lane < cnt)
+            sd[0][lane] = V.pre[first + lane];
+    };
+    R.prologue(side);
+    const int ntiles = R.tiles();
+    V3 wc;
+    double wr;
+    warp_sphere(C, wc, wr);
+    NearList L{s_near[warp], 0};
+    auto store = [&](int p, int e, double a) {
+        if (base + 32 * p < n) {
+            const size_t idx = (size_t) e * op_ld(n) + row[p];
+            if (a64)
+                a64[idx] = a;
+            if (a32)
+                a32[idx] = (float) a;
+        }
+    };
+    auto near = [&]() {
+        L.drain(rec, [&](int e, const double* er) {
+#pragma unroll
+            for (int p = 0; p < kPair; p++)
+                store(p, e, any_neumann ? entry<MIXED>(er, V.rwg + (size_t) e * wRecSize, tgt[row[p]], C[p])
+                                        : epi<MIXED, true, false>(er, V.rwg + (size_t) e * wRecSize, C[p]).phi);
+        });
+    };
+    bool ok = true;
+    for (int q = 0; q < ntiles; q++) {
+        if (!__all_sync(0xffffffffu, R.wait(q))) {
+            ok = false;
+            break;
+        }
+        if (busy) {
+            const FarTile T = S.tile[q % kPipe];
+            tile_entries<MIXED>(S.rec[q % kPipe], T, S.side[q % kPipe][0], tgt, row, C, any_neumann, wc, wr, L,
+                                [&](int p, int j, double a) { store(p, T.first + j, a); });
+            if (L.full())
+                near();
+        }
+        R.release(q, side);
+    }
+    R.finish(ok, flag);
+    if (L.n > 0)
+        near();
 }
 
 // dense matvec on the assembled column-major operator (leading dimension ld):
@@ -859,6 +1255,23 @@ __global__ void morton_kernel(const double* __restrict__ P, int n, const double*
     for (int c = 0; c < 3; c++) {
         const double ext = box[3 + c] - box[c];
         const double t = ext > 0. ? (P[3 * i + c] - box[c]) / ext : 0.;
+        q[c] = (unsigned) fmin(fmax(t * 2097151.0, 0.), 2097151.0);
+    }
+    key[i] = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
+    idx[i] = i;
+}
+
+// the same for the matrix rows' collocation points
+__global__ void morton_rows_kernel(const TargetRec* __restrict__ tgt, int n, const double* __restrict__ box,
+                                   unsigned long long* __restrict__ key, int* __restrict__ idx)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    unsigned q[3];
+    for (int c = 0; c < 3; c++) {
+        const double ext = box[3 + c] - box[c];
+        const double t = ext > 0. ? (tgt[i].cen[c] - box[c]) / ext : 0.;
         q[c] = (unsigned) fmin(fmax(t * 2097151.0, 0.), 2097151.0);
     }
     key[i] = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);

@@ -62,7 +62,13 @@ struct kemcu_ctx
     double* d_rec = nullptr;
     TargetRec* d_tgt = nullptr;
     double* d_sigma = nullptr;
+    // far-field series of the (planar) elements: records by tile, the tile table, total charges
+    double* d_far = nullptr;
+    FarTile* d_tiles = nullptr;
+    double* d_pre = nullptr;
     double* d_rwg = nullptr;  // near records (rwg_build_kernel)
+    int ntiles = 0;
+    int* d_rows = nullptr;  // matrix rows in Morton order of their collocation points
     bool have_sigma = false;
     // all elements axisymmetric (conic sections, rings): records in the AxRec layout
     bool axisym = false;
@@ -97,6 +103,10 @@ struct kemcu_ctx
 
 void fm_release(kemcu_ctx* ctx);
 int fm_apply(kemcu_ctx* ctx, FmState* S, const double* d_x, double* d_y, int nrhs);
+namespace
+{
+FmGl fm_gauss_legendre(int q);
+}
 
 namespace
 {
@@ -314,15 +324,108 @@ int pipe_status(kemcu_ctx* ctx, const char* what)
     return KEMCU_OK;
 }
 
-int grid_split(const kemcu_ctx* ctx, size_t n_pts, size_t n_elem)
+int grid_split(const kemcu_ctx* ctx, size_t n_pts)
 {
-    // enough CTAs for four waves of the resident CTAs per SM, each split keeping >= 32 elements
-    const size_t blocks = (n_pts + kThreads - 1) / kThreads;
+    // enough CTAs for four waves of the resident CTAs per SM, each split keeping >= 2 tiles
+    const size_t blocks = (n_pts + kPair * kThreads - 1) / (kPair * kThreads);
     const size_t want = (size_t) ctx->num_sms * kMinBlocks * 4;
     size_t split = blocks >= want ? 1 : (want + blocks - 1) / blocks;
-    split = std::min(split, std::max((size_t) 1, n_elem / 32));
+    split = std::min(split, std::max((size_t) 1, (size_t) ctx->ntiles / 2));
     split = std::min(split, (size_t) 65535);
     return (int) std::max((size_t) 1, split);
+}
+
+FarView far_view(const kemcu_ctx* ctx)
+{
+    return FarView{ctx->d_far, ctx->d_tiles, ctx->ntiles, ctx->d_pre, ctx->d_rwg};
+}
+
+// The far records of the context's planar elements. Tiles in element order: a run of up to kFarSym
+// elements with two mirror axes (rectangles with orthogonal sides, wires), else up to kFarGen
+// elements of any kind in the general form.
+int build_far(kemcu_ctx* ctx)
+{
+    const size_t n = ctx->n;
+    std::vector<char> sym(n);
+    for (size_t e = 0; e < n; e++) {
+        const double* r = &ctx->h_rec[e * rRecSize];
+        // below 1e-14 the cosine of the sides' angle changes no moment's last digit
+        sym[e] = ctx->h_shape[e] == kLineSegment ||
+                 (ctx->h_shape[e] == kRectangle && std::fabs(r[rAB2]) <= 2e-14 * std::sqrt(r[rAA] * r[rBB]));
+    }
+    std::vector<FarTile> tiles;
+    size_t off = 0;
+    for (size_t e = 0; e < n;) {
+        size_t k = 0;
+        while (k < (size_t) kFarSym && e + k < n && sym[e + k])
+            k++;
+        const bool general = k < std::min((size_t) kFarGen, n - e);
+        if (general)
+            k = std::min((size_t) kFarGen, n - e);
+        tiles.push_back(FarTile{(int) e, (int) k, general ? 1 : 0, (int) (off / 2)});
+        off += k * (general ? kFarGenStride : kFarSymStride);
+        e += k;
+    }
+    if (off / 2 > (size_t) 0x7fffffff)
+        return fail(ctx, KEMCU_EINVAL, "%zu elements exceed the far-record table", n);
+    const FmGl g = fm_gauss_legendre(kFarQ);
+    FarTables gl;
+    far_tables(gl);
+    for (int i = 0; i < kFarQ; i++) {
+        gl.x[i] = g.x[i];
+        gl.w[i] = g.w[i];
+    }
+    ctx->ntiles = (int) tiles.size();
+    KC(cudaMalloc(&ctx->d_far, off * sizeof(double)));
+    KC(cudaMalloc(&ctx->d_tiles, tiles.size() * sizeof(FarTile)));
+    KC(cudaMalloc(&ctx->d_pre, n * sizeof(double)));
+    KC(cudaMemcpy(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(FarTile), cudaMemcpyHostToDevice));
+    far_build_kernel<<<(unsigned) ((tiles.size() * kFarSym + 127) / 128), 128, 0, ctx->stream>>>(
+        ctx->d_rec, ctx->d_tiles, ctx->ntiles, gl, ctx->d_far, ctx->d_pre);
+    KCHECK_LAUNCH();
+    KC(cudaMalloc(&ctx->d_rwg, n * wRecSize * sizeof(double)));
+    rwg_build_kernel<<<(unsigned) ((n + 127) / 128), 128, 0, ctx->stream>>>(ctx->d_rec, (int) n, ctx->d_rwg);
+    KCHECK_LAUNCH();
+    return KEMCU_OK;
+}
+
+size_t cub_sort_bytes(size_t n)
+{
+    size_t b = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, b, (const unsigned long long*) nullptr, (unsigned long long*) nullptr,
+                                    (const int*) nullptr, (int*) nullptr, (int) n, 0, 63);
+    return b;
+}
+
+// the matrix rows in Morton order of their collocation points
+int build_rows(kemcu_ctx* ctx)
+{
+    const size_t n = ctx->n;
+    double box[6] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
+    for (size_t i = 0; i < n; i++)
+        for (int c = 0; c < 3; c++) {
+            box[c] = std::min(box[c], ctx->h_tgt[i].cen[c]);
+            box[3 + c] = std::max(box[3 + c], ctx->h_tgt[i].cen[c]);
+        }
+    KC(cudaMalloc(&ctx->d_rows, n * sizeof(int)));
+    const size_t cub_bytes = cub_sort_bytes(n);
+    auto up = [](size_t b) { return (b + 255) & ~(size_t) 255; };
+    void* base;
+    if (int rc = ensure(ctx, sSort, 2 * up(n * 8) + up(n * 4) + 256 + up(cub_bytes), &base))
+        return rc;
+    char* q = (char*) base;
+    auto* k0 = (unsigned long long*) q;
+    auto* k1 = (unsigned long long*) (q + up(n * 8));
+    int* i0 = (int*) (q + 2 * up(n * 8));
+    double* dbox = (double*) (q + 2 * up(n * 8) + up(n * 4));
+    void* tmp = (char*) dbox + 256;
+    KC(cudaMemcpyAsync(dbox, box, sizeof box, cudaMemcpyHostToDevice, ctx->stream));
+    morton_rows_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->d_tgt, (int) n, dbox, k0, i0);
+    KCHECK_LAUNCH();
+    size_t tb = cub_bytes;
+    KC(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, i0, ctx->d_rows, (int) n, 0, 63, ctx->stream));
+    KC(cudaStreamSynchronize(ctx->stream));  // box is on this stack frame
+    return KEMCU_OK;
 }
 
 // axisymmetric elements: FP64 element integrals whatever the precision argument. The element
@@ -373,29 +476,24 @@ struct FieldVariant
 {
     int min_blocks, ring_stages;
 };
-constexpr FieldVariant kFieldVariants[] = {{kMinBlocks, kPipe}, {4, 4}, {5, 3}, {4, 3}};
+constexpr FieldVariant kFieldVariants[] = {{kMinBlocks, kPipe}, {4, kPipe}, {6, kPipe}};
 constexpr int kNumFieldVariants = (int) (sizeof(kFieldVariants) / sizeof(kFieldVariants[0]));
 
 template<bool MIXED, bool POT, bool FIELD>
-void launch_k1(int variant, dim3 grid, cudaStream_t st, const double* rec, const double* sg, int ne, const double* pts,
-               int np, double* out, double* part, int* fl)
+void launch_k1(int variant, dim3 grid, cudaStream_t st, const double* rec, const FarView& fv, const double* sg,
+               const double* pts, int np, double* out, double* part, int* fl)
 {
     if constexpr (POT && FIELD) {
-        switch (variant) {
-        case 1:
-            field_kernel<MIXED, POT, FIELD, 4, 4><<<grid, kThreads, 0, st>>>(rec, sg, ne, pts, np, out, part, fl);
+        if (variant == 1) {
+            field_kernel<MIXED, POT, FIELD, 4><<<grid, kThreads, 0, st>>>(rec, fv, sg, pts, np, out, part, fl);
             return;
-        case 2:
-            field_kernel<MIXED, POT, FIELD, 5, 3><<<grid, kThreads, 0, st>>>(rec, sg, ne, pts, np, out, part, fl);
+        }
+        if (variant == 2) {
+            field_kernel<MIXED, POT, FIELD, 6><<<grid, kThreads, 0, st>>>(rec, fv, sg, pts, np, out, part, fl);
             return;
-        case 3:
-            field_kernel<MIXED, POT, FIELD, 4, 3><<<grid, kThreads, 0, st>>>(rec, sg, ne, pts, np, out, part, fl);
-            return;
-        default:
-            break;
         }
     }
-    field_kernel<MIXED, POT, FIELD><<<grid, kThreads, 0, st>>>(rec, sg, ne, pts, np, out, part, fl);
+    field_kernel<MIXED, POT, FIELD><<<grid, kThreads, 0, st>>>(rec, fv, sg, pts, np, out, part, fl);
 }
 
 // tuning key: precision and the size class (bit length of the point count)
@@ -446,50 +544,81 @@ void finish_variant(kemcu_ctx* ctx)
     ctx->pending_key = -1;
 }
 
+template<bool MIXED, bool F32>
+void few_form(dim3 grid, cudaStream_t st, int what, const kemcu_ctx* ctx, const double* pts, int np, double* part)
+{
+    const int ne = (int) ctx->n;
+    if (what == KEMCU_POTENTIAL)
+        field_few_kernel<MIXED, true, false, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, np, part);
+    else if (what == KEMCU_FIELD)
+        field_few_kernel<MIXED, false, true, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, np, part);
+    else
+        field_few_kernel<MIXED, true, true, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, np, part);
+}
+
+void launch_few(kemcu_ctx* ctx, const double* pts, int np, int precision, int what, int split, double* part)
+{
+    const dim3 grid((unsigned) np, (unsigned) split);
+    if (precision == KEMCU_FP32)
+        few_form<false, true>(grid, ctx->stream, what, ctx, pts, np, part);
+    else if (precision == KEMCU_MIXED)
+        few_form<true, false>(grid, ctx->stream, what, ctx, pts, np, part);
+    else
+        few_form<false, false>(grid, ctx->stream, what, ctx, pts, np, part);
+}
+
 // the planar direct sum at device points (d_out n x 4): K1, split `split` ways over the element
 // list (partial sums in `partial`, then reduced in split order)
 int launch_planar_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d_out, int precision, int what,
-                        int split, double* partial)
+                        int split, double* partial, bool few = false)
 {
-    dim3 grid((unsigned) ((n + kThreads - 1) / kThreads), (unsigned) split);
+    dim3 grid((unsigned) ((n + kPair * kThreads - 1) / (kPair * kThreads)), (unsigned) split);
     if (int rc = clear_pipe_flag(ctx))
         return rc;
     const bool mixed = precision == KEMCU_MIXED;
     const double* sg = ctx->d_sigma;
-    const int ne = (int) ctx->n, np = (int) n;
+    const FarView fv = far_view(ctx);
+    const int np = (int) n;
     double* part = split > 1 ? partial : nullptr;
     int* fl = ctx->d_flag + 1;
-    const int v = choose_variant(ctx, n, precision, what);
     cudaStream_t st = ctx->stream;
+    if (few) {
+        launch_few(ctx, d_pts, np, precision, what, split, partial);
+        KCHECK_LAUNCH();
+        reduce_splits<<<1, 4 * kFewPoints, 0, st>>>(partial, split, (size_t) n * 4, d_out);
+        KCHECK_LAUNCH();
+        return KEMCU_OK;
+    }
+    const int v = choose_variant(ctx, n, precision, what);
     const bool timed = ctx->pending_key >= 0 || ctx->time_k1;
     if (timed)
         KC(cudaEventRecord(ctx->tv0, st));
     if (precision == KEMCU_FP32) {
         const double* r = ctx->d_rec;
         if (what == KEMCU_POTENTIAL)
-            field_kernel<false, true, false, kMinBlocks, kPipe, true><<<grid, kThreads, 0, st>>>(r, sg, ne, d_pts, np, d_out, part, fl);
+            field_kernel<false, true, false, kMinBlocks, true><<<grid, kThreads, 0, st>>>(r, fv, sg, d_pts, np, d_out, part, fl);
         else if (what == KEMCU_FIELD)
-            field_kernel<false, false, true, kMinBlocks, kPipe, true><<<grid, kThreads, 0, st>>>(r, sg, ne, d_pts, np, d_out, part, fl);
+            field_kernel<false, false, true, kMinBlocks, true><<<grid, kThreads, 0, st>>>(r, fv, sg, d_pts, np, d_out, part, fl);
         else
-            field_kernel<false, true, true, kMinBlocks, kPipe, true><<<grid, kThreads, 0, st>>>(r, sg, ne, d_pts, np, d_out, part, fl);
+            field_kernel<false, true, true, kMinBlocks, true><<<grid, kThreads, 0, st>>>(r, fv, sg, d_pts, np, d_out, part, fl);
     }
     else if (what == KEMCU_POTENTIAL) {
         if (mixed)
-            launch_k1<true, true, false>(v, grid, st, ctx->d_rec, sg, ne, d_pts, np, d_out, part, fl);
+            launch_k1<true, true, false>(v, grid, st, ctx->d_rec, fv, sg, d_pts, np, d_out, part, fl);
         else
-            launch_k1<false, true, false>(v, grid, st, ctx->d_rec, sg, ne, d_pts, np, d_out, part, fl);
+            launch_k1<false, true, false>(v, grid, st, ctx->d_rec, fv, sg, d_pts, np, d_out, part, fl);
     }
     else if (what == KEMCU_FIELD) {
         if (mixed)
-            launch_k1<true, false, true>(v, grid, st, ctx->d_rec, sg, ne, d_pts, np, d_out, part, fl);
+            launch_k1<true, false, true>(v, grid, st, ctx->d_rec, fv, sg, d_pts, np, d_out, part, fl);
         else
-            launch_k1<false, false, true>(v, grid, st, ctx->d_rec, sg, ne, d_pts, np, d_out, part, fl);
+            launch_k1<false, false, true>(v, grid, st, ctx->d_rec, fv, sg, d_pts, np, d_out, part, fl);
     }
     else {
         if (mixed)
-            launch_k1<true, true, true>(v, grid, st, ctx->d_rec, sg, ne, d_pts, np, d_out, part, fl);
+            launch_k1<true, true, true>(v, grid, st, ctx->d_rec, fv, sg, d_pts, np, d_out, part, fl);
         else
-            launch_k1<false, true, true>(v, grid, st, ctx->d_rec, sg, ne, d_pts, np, d_out, part, fl);
+            launch_k1<false, true, true>(v, grid, st, ctx->d_rec, fv, sg, d_pts, np, d_out, part, fl);
     }
     KCHECK_LAUNCH();
     if (timed)
@@ -507,27 +636,22 @@ int launch_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d_out, i
 {
     if (ctx->axisym)
         return launch_axisym_field(ctx, d_pts, n, d_out, what);
-    const int split = grid_split(ctx, n, ctx->n);
+    // a handful of points: a CTA per point and kFewElems elements (grids of at most 65,535 element blocks)
+    const size_t eb = (ctx->n + kFewElems - 1) / kFewElems;
+    const bool few = n <= (size_t) kFewPoints && eb <= 65535;
+    const int split = few ? (int) eb : grid_split(ctx, n);
     double* partial = nullptr;
-    if (split > 1) {
+    if (split > 1 || few) {
         void* p;
         int rc = ensure(ctx, sPartial, (size_t) split * n * 4 * sizeof(double), &p);
         if (rc)
             return rc;
         partial = (double*) p;
     }
-    return launch_planar_field(ctx, d_pts, n, d_out, precision, what, split, partial);
+    return launch_planar_field(ctx, d_pts, n, d_out, precision, what, split, partial, few);
 }
 
 constexpr size_t kSortMin = 4096;  // below this the point set is evaluated in caller order
-
-size_t cub_sort_bytes(size_t n)
-{
-    size_t b = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, b, (const unsigned long long*) nullptr, (unsigned long long*) nullptr,
-                                    (const int*) nullptr, (int*) nullptr, (int) n, 0, 63);
-    return b;
-}
 
 int check_finite(kemcu_ctx* ctx, const double* d, size_t m, const char* what)
 {
@@ -622,7 +746,7 @@ int apply_op(kemcu_ctx* ctx, int op, const double* d_x, double* d_y, int nrhs)
         return KEMCU_OK;
     }
     if (op == kFree64 || op == kFreeMixed || op == kFree32) {
-        const int split = grid_split(ctx, n, n);
+        const int split = grid_split(ctx, n);
         double* partial = nullptr;
         if (split > 1) {
             void* p;
@@ -631,29 +755,26 @@ int apply_op(kemcu_ctx* ctx, int op, const double* d_x, double* d_y, int nrhs)
                 return rc;
             partial = (double*) p;
         }
-        dim3 grid((n + kThreads - 1) / kThreads, split);
+        dim3 grid((n + kPair * kThreads - 1) / (kPair * kThreads), split);
         int* fl = ctx->d_flag + 1;
+        const FarView fv = far_view(ctx);
         if (op == kFree32) {
             if (nrhs == 1)
-                matvec_kernel<false, 1, true><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, n, d_x, nrhs, d_y,
-                                                                                partial, fl);
+                matvec_kernel<false, 1, true><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, n, d_x, nrhs, d_y, partial, fl);
             else
-                matvec_kernel<false, kMaxRhs, true><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, n, d_x, nrhs,
-                                                                                      d_y, partial, fl);
+                matvec_kernel<false, kMaxRhs, true><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, n, d_x, nrhs, d_y, partial, fl);
         }
         else if (op == kFree64) {
             if (nrhs == 1)
-                matvec_kernel<false, 1><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, n, d_x, nrhs, d_y, partial, fl);
+                matvec_kernel<false, 1><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, n, d_x, nrhs, d_y, partial, fl);
             else
-                matvec_kernel<false, kMaxRhs><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, n, d_x, nrhs, d_y,
-                                                                                  partial, fl);
+                matvec_kernel<false, kMaxRhs><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, n, d_x, nrhs, d_y, partial, fl);
         }
         else {
             if (nrhs == 1)
-                matvec_kernel<true, 1><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, n, d_x, nrhs, d_y, partial, fl);
+                matvec_kernel<true, 1><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, n, d_x, nrhs, d_y, partial, fl);
             else
-                matvec_kernel<true, kMaxRhs><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, n, d_x, nrhs, d_y,
-                                                                                 partial, fl);
+                matvec_kernel<true, kMaxRhs><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, n, d_x, nrhs, d_y, partial, fl);
         }
         KCHECK_LAUNCH();
         if (split > 1) {
@@ -742,10 +863,10 @@ int assemble(kemcu_ctx* ctx, bool want32)
         KCHECK_LAUNCH();
         return KEMCU_OK;
     }
-    const int split = grid_split(ctx, n, n);
-    dim3 grid((unsigned) ((n + kThreads - 1) / kThreads), (unsigned) split);
-    assemble_kernel<false><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, (int) n, 0, (int) n, ctx->d_a64,
-                                                              fill32 ? ctx->d_a32 : nullptr, ctx->d_flag + 1);
+    const int split = grid_split(ctx, n);
+    dim3 grid((unsigned) ((n + kPair * kThreads - 1) / (kPair * kThreads)), (unsigned) split);
+    assemble_kernel<false><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, far_view(ctx), ctx->d_tgt, ctx->d_rows, (int) n,
+                                                              ctx->d_a64, fill32 ? ctx->d_a32 : nullptr, ctx->d_flag + 1);
     KCHECK_LAUNCH();
     return KEMCU_OK;
 }
@@ -1242,7 +1363,11 @@ int kemcu_destroy(kemcu_ctx* ctx)
         cudaFree(ctx->d_near_ptr);
         cudaFree(ctx->d_near_row);
         cudaFree(ctx->d_near_val);
+        cudaFree(ctx->d_far);
+        cudaFree(ctx->d_tiles);
+        cudaFree(ctx->d_pre);
         cudaFree(ctx->d_rwg);
+        cudaFree(ctx->d_rows);
         cudaFree(ctx->d_counter);
         cudaFree(ctx->d_flag);
         fm_release(ctx);
@@ -1312,7 +1437,11 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     cudaFree(ctx->d_near_ptr);
     cudaFree(ctx->d_near_row);
     cudaFree(ctx->d_near_val);
+    cudaFree(ctx->d_far);
+    cudaFree(ctx->d_tiles);
+    cudaFree(ctx->d_pre);
     cudaFree(ctx->d_rwg);
+    cudaFree(ctx->d_rows);
     ctx->d_rec = nullptr;
     ctx->d_tgt = nullptr;
     ctx->d_sigma = nullptr;
@@ -1321,7 +1450,12 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     ctx->d_near_ptr = nullptr;
     ctx->d_near_row = nullptr;
     ctx->d_near_val = nullptr;
+    ctx->d_far = nullptr;
+    ctx->d_tiles = nullptr;
+    ctx->d_pre = nullptr;
     ctx->d_rwg = nullptr;
+    ctx->d_rows = nullptr;
+    ctx->ntiles = 0;
     ctx->have_sigma = false;
     ctx->n = 0;
     ctx->h_rec.assign(n * rRecSize, 0.);
@@ -1343,12 +1477,16 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     KC(cudaMemcpy(ctx->d_rec, ctx->h_rec.data(), n * rRecSize * sizeof(double), cudaMemcpyHostToDevice));
     KC(cudaMemcpy(ctx->d_tgt, ctx->h_tgt.data(), n * sizeof(TargetRec), cudaMemcpyHostToDevice));
     KC(cudaMemset(ctx->d_sigma, 0, n * sizeof(double)));
-    if (!ctx->axisym) {
-        KC(cudaMalloc(&ctx->d_rwg, n * wRecSize * sizeof(double)));
-        rwg_build_kernel<<<(unsigned) ((n + 127) / 128), 128, 0, ctx->stream>>>(ctx->d_rec, (int) n, ctx->d_rwg);
-        KCHECK_LAUNCH();
-    }
     ctx->n = n;
+    if (!ctx->axisym) {
+        int rc = build_far(ctx);
+        if (!rc)
+            rc = build_rows(ctx);
+        if (rc) {
+            ctx->n = 0;
+            return rc;
+        }
+    }
     return KEMCU_OK;
 }
 
@@ -1475,7 +1613,7 @@ int kemcu_field_dev_noalloc(kemcu_ctx* ctx, const double* dP, size_t n, double* 
         return check_finite(ctx, dout4, n * 4, "field result");
     }
     const size_t cap = KEMCU_NOALLOC_SCRATCH_BYTES / sizeof(double);
-    const int split = (int) std::min((size_t) grid_split(ctx, n, ctx->n), std::max((size_t) 1, cap / (4 * n)));
+    const int split = (int) std::min((size_t) grid_split(ctx, n), std::max((size_t) 1, cap / (4 * n)));
     if ((rc = launch_planar_field(ctx, dP, n, dout4, precision, what, split, ctx->noalloc_scratch)))
         return rc;
     t.stop();
@@ -1581,7 +1719,7 @@ int kemcu_matrix_element(kemcu_ctx* ctx, size_t i, size_t j, double* a)
     if (ctx->axisym)
         axisym_entry_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_rec, rRecSize, (int) i, (int) j, (double*) d);
     else
-        entry_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_rec, ctx->d_tgt, (int) i, (int) j, (double*) d);
+        entry_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_rec, ctx->d_rwg, ctx->d_tgt, (int) i, (int) j, (double*) d);
     KCHECK_LAUNCH();
     KC(cudaMemcpyAsync(a, d, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     KC(cudaStreamSynchronize(ctx->stream));

@@ -56,14 +56,15 @@ struct RhPart
 };
 
 // diagonal A(k, k) of the operator (entry<false>: the plain FP64 form, as the matvec)
-__global__ void diag_kernel(const double* __restrict__ rec, const TargetRec* __restrict__ tgt, int n,
+__global__ void diag_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
+                            const TargetRec* __restrict__ tgt, int n,
                             double* __restrict__ diag)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n)
         return;
     const TargetRec t = tgt[k];
-    diag[k] = entry<false>(rec + (size_t) k * rRecSize, t, v3(t.cen[0], t.cen[1], t.cen[2]));
+    diag[k] = entry<false>(rec + (size_t) k * rRecSize, rwg + (size_t) k * wRecSize, t, v3(t.cen[0], t.cen[1], t.cen[2]));
 }
 
 // Near-field list of the operator's columns (compressed by column): the pairs (row i, column
@@ -90,7 +91,8 @@ __global__ void near_count_kernel(const double* __restrict__ rec, const TargetRe
         count[k] = c;
 }
 
-__global__ void near_fill_kernel(const double* __restrict__ rec, const TargetRec* __restrict__ tgt, int n,
+__global__ void near_fill_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
+                                 const TargetRec* __restrict__ tgt, int n,
                                  const long long* __restrict__ ptr, int* __restrict__ rows, double* __restrict__ vals)
 {
     const int k = (int) ((blockIdx.x * (size_t) blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
@@ -112,7 +114,7 @@ __global__ void near_fill_kernel(const double* __restrict__ rec, const TargetRec
         if (near) {
             const long long q = pos + __popc(m & ((1u << lane) - 1u));
             rows[q] = i;
-            vals[q] = entry<false>(e, t, C);
+            vals[q] = entry<false>(e, rwg + (size_t) k * wRecSize, t, C);
         }
         pos += __popc(m);
     }
