@@ -195,6 +195,17 @@ __device__ __forceinline__ long long fm_cell(const FmLevel& L, int x, int y, int
     return L.base + ((long long) x * L.n + y) * L.n + z;
 }
 
+// the tree as the kernels take it
+struct FmTreeView
+{
+    FmLevel lv[12];
+    int depth;       // the leaves' level
+    int zm;
+    double wx, wy, wz;  // world cube corner (minimum)
+    const int* own_ptr;   // owned-element ranges per cell of every level (level-concatenated, +1)
+    const int* own_elem;  // elements in owner order
+};
+
 // sum_k op[k K + row] x[k]: one row of a column-major K x K operator times x, in four
 // independent chains over k mod 4 (a single accumulator is a 2K-step dependent chain, the
 // translation kernels' latency with one right-hand side)
@@ -397,6 +408,264 @@ __global__ void fm_m2l_kernel(const int* __restrict__ targets, int ntargets, FmL
                 Lx[r * lstride + (L.base + tc) * K + row] += acc[r];
 }
 
+// ------------------------------------------------------------------------- M2L on the FP64 tensor cores
+// The cells of one level that sit at the same position of their parent (one of div^3 classes) have the
+// same interaction offsets, and one offset's operator serves every one of them: a tile is up to 16
+// such targets, and for each offset L[:, targets] += op M[:, sources], an 88 x 88 x 16 product at
+// degree 8 on mma.m8n8k4 (FP64 in and out). fm_m2l_kernel above reads an operator through L1 for every
+// target (L1TEX 70 % busy at 9.5 % of the FP64 pipe); here one read serves 16 columns, and the reads are
+// whole 512-byte fragments: the operators are packed in the order the lanes hold them,
+// [operator][8 rows][8 columns][lane][2], lane (g, t) with rows g and columns t, t + 4, zero-padded.
+// With several right-hand sides the 16 columns are two targets times eight of them. One warp per 8
+// rows (two for K > 128); the moments of the next offset's sources travel to shared memory (cp.async)
+// while this one's are multiplied. The offsets, those some target of the tile has an occupied source
+// for, are split over gridDim.y; the parts are added in order by fm_m2l_sum_kernel.
+constexpr int kM2lCols = 16;
+
+struct FmTile
+{
+    int level, cls;
+    int tgt[kM2lCols];  // cell indices within the level, -1: none
+};
+struct FmOffset
+{
+    signed char x, y, z, pad;
+    int op;
+};
+// the offsets of every class of a level's cells: off[ptr[cls] .. ptr[cls + 1])
+struct FmOffsets
+{
+    const FmOffset* off;
+    const int* ptr;
+};
+
+__host__ __device__ __forceinline__ int fm_mtiles(int K)
+{
+    return (K + 7) / 8;
+}
+
+__global__ void fm_pack_kernel(const double* __restrict__ ops, int nops, int K, double* __restrict__ pk)
+{
+    const int mt = fm_mtiles(K);
+    const size_t total = (size_t) nops * mt * mt * 64;
+    for (size_t q = blockIdx.x * (size_t) blockDim.x + threadIdx.x; q < total; q += (size_t) gridDim.x * blockDim.x) {
+        const int s = (int) (q & 1), lane = (int) (q >> 1) & 31;
+        const size_t r = q >> 6;
+        const int kp = (int) (r % mt), m = (int) (r / mt % mt);
+        const size_t o = r / mt / mt;
+        const int row = m * 8 + (lane >> 2), col = kp * 8 + s * 4 + (lane & 3);
+        pk[q] = row < K && col < K ? ops[(o * K + col) * K + row] : 0.;
+    }
+}
+
+__device__ __forceinline__ void cp_async8(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// shared memory of one CTA: two buffers of kM2lCols moment vectors, then the offset list
+__host__ __device__ __forceinline__ int fm_m2l_stride(int K)
+{
+    return fm_mtiles(K) * 8 + 4;  // 4 or 12 modulo 16: the B fragments' lanes fall in different banks
+}
+__host__ __device__ __forceinline__ size_t fm_m2l_smem(int K, int max_off)
+{
+    return 2 * sizeof(double) * kM2lCols * fm_m2l_stride(K) + (size_t) max_off * (sizeof(int) + sizeof(unsigned));
+}
+
+template<int MT, int RW>
+__global__ void __launch_bounds__(MT == 1 ? 512 : 1024)
+    fm_m2l_mma_kernel(const FmTile* __restrict__ tiles, int ntiles, FmTreeView T, FmOffsets first, FmOffsets rest,
+                      const unsigned char* __restrict__ occ, const double* __restrict__ pk, int K,
+                      const double* __restrict__ M, size_t mstride, double* __restrict__ Lx, size_t lstride, int nrhs,
+                      double* __restrict__ partial)
+{
+    extern __shared__ __align__(16) double fm_x[];
+    __shared__ int s_xyz[kM2lCols][3], s_cell[kM2lCols];
+    __shared__ int s_n;
+    constexpr int TW = kM2lCols / RW;  // targets of this CTA: the part blockIdx.z of the tile's 16
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const int mt = fm_mtiles(K), stride = fm_m2l_stride(K);
+    double* buf[2] = {fm_x, fm_x + kM2lCols * stride};
+    const FmTile& tile = tiles[blockIdx.x];
+    const FmLevel L = T.lv[tile.level];
+    const FmOffsets list = tile.level == 1 ? first : rest;
+    const int o0 = list.ptr[tile.cls], no = list.ptr[tile.cls + 1] - o0;
+    int* s_off = reinterpret_cast<int*>(fm_x + 2 * kM2lCols * stride);
+    unsigned* s_mask = reinterpret_cast<unsigned*>(s_off + no);
+    if (tid < TW) {
+        const int c = tile.tgt[blockIdx.z * TW + tid];
+        s_cell[tid] = c;
+        s_xyz[tid][0] = c < 0 ? -1000000 : c / (L.n * L.n);
+        s_xyz[tid][1] = c < 0 ? 0 : c / L.n % L.n;
+        s_xyz[tid][2] = c < 0 ? 0 : c % L.n;
+    }
+    for (int q = tid; q < 2 * kM2lCols * stride; q += blockDim.x)
+        fm_x[q] = 0.;  // the padding columns stay zero
+    __syncthreads();
+    // which targets have an occupied source at each offset
+    for (int q = tid; q < no; q += blockDim.x) {
+        const FmOffset o = list.off[o0 + q];
+        unsigned m = 0u;
+        for (int t = 0; t < TW; t++) {
+            const int x = s_xyz[t][0] + o.x, y = s_xyz[t][1] + o.y, z = s_xyz[t][2] + o.z;
+            if (x >= 0 && y >= 0 && z >= 0 && x < L.n && y < L.n && z < L.n && occ[fm_cell(L, x, y, z)])
+                m |= 1u << t;
+        }
+        s_mask[q] = m;
+    }
+    __syncthreads();
+    // the offsets with any, in order (one warp)
+    if (warp == 0) {
+        int n = 0;
+        for (int q0 = 0; q0 < no; q0 += 32) {
+            const bool on = q0 + lane < no && s_mask[q0 + lane] != 0u;
+            const unsigned b = __ballot_sync(0xffffffffu, on);
+            if (on)
+                s_off[n + __popc(b & ((1u << lane) - 1u))] = q0 + lane;
+            n += __popc(b);
+        }
+        if (lane == 0)
+            s_n = n;
+    }
+    __syncthreads();
+    const int per = (s_n + (int) gridDim.y - 1) / (int) gridDim.y;
+    const int q0 = min(s_n, (int) blockIdx.y * per), q1 = min(s_n, q0 + per);
+    // the sources' moments of active offset q into buffer b: a warp per column
+    auto stage = [&](int q, int b) {
+        const int oq = s_off[q];
+        const FmOffset o = list.off[o0 + oq];
+        const unsigned m = s_mask[oq];
+        for (int c = warp; c < kM2lCols; c += nw) {
+            const int t = c / RW, r = c % RW;
+            double* dst = buf[b] + c * stride;
+            if ((m >> t & 1u) && r < nrhs) {
+                const long long si = fm_cell(L, s_xyz[t][0] + o.x, s_xyz[t][1] + o.y, s_xyz[t][2] + o.z);
+                const double* src = M + r * mstride + (size_t) si * K;
+                for (int k = lane; k < K; k += 32)
+                    cp_async8(dst + k, src + k);
+            }
+            else
+                for (int k = lane; k < K; k += 32)
+                    dst[k] = 0.;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[MT][2][2];
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+        acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.;
+    if (q0 < q1)
+        stage(q0, 0);
+    for (int q = q0; q < q1; q++) {
+        const int b = (q - q0) & 1;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // this offset's moments are there, the other buffer is free
+        if (q + 1 < q1)
+            stage(q + 1, b ^ 1);
+        const int oq = s_off[q];
+        const unsigned m = s_mask[oq];
+        const bool lo = (m & ((1u << (8 / RW)) - 1u)) != 0u, hi = (m >> (8 / RW)) != 0u;
+        const int op = list.off[o0 + oq].op;
+        const double* B = buf[b] + (lane >> 2) * stride + (lane & 3);
+#pragma unroll
+        for (int i = 0; i < MT; i++) {
+            const int row = warp + i * nw;
+            if (row >= mt)
+                break;
+            const double2* A = reinterpret_cast<const double2*>(pk) + (((size_t) op * mt + row) * mt) * 32 + lane;
+#pragma unroll 4
+            for (int kp = 0; kp < mt; kp++) {
+                const double2 a = __ldg(A + (size_t) kp * 32);
+                const double* p = B + kp * 8;
+                if (lo) {
+                    mma_884(acc[i][0][0], acc[i][0][1], a.x, p[0]);
+                    mma_884(acc[i][0][0], acc[i][0][1], a.y, p[4]);
+                }
+                if (hi) {
+                    mma_884(acc[i][1][0], acc[i][1][1], a.x, p[8 * stride]);
+                    mma_884(acc[i][1][0], acc[i][1][1], a.y, p[8 * stride + 4]);
+                }
+            }
+        }
+    }
+    // lane (g, t) holds row g of its tile for columns 2t, 2t + 1
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+        const int row = (warp + i * nw) * 8 + (lane >> 2);
+        if (row >= K || warp + i * nw >= mt)
+            continue;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int c = h * 8 + (lane & 3) * 2 + j, t = c / RW, r = c % RW;
+                if (s_cell[t] < 0 || r >= nrhs)
+                    continue;
+                if (gridDim.y == 1)
+                    Lx[r * lstride + (size_t) (L.base + s_cell[t]) * K + row] = acc[i][h][j];
+                else
+                    partial[((((size_t) blockIdx.y * ntiles + blockIdx.x) * gridDim.z + blockIdx.z) * kM2lCols + c) * K + row] =
+                        acc[i][h][j];
+            }
+    }
+}
+
+// the parts of fm_m2l_mma_kernel added in order: one CTA per tile and part of it
+template<int RW>
+__global__ void fm_m2l_sum_kernel(const FmTile* __restrict__ tiles, int ntiles, int nsplit, FmTreeView T, int K,
+                                  const double* __restrict__ partial, double* __restrict__ Lx, size_t lstride, int nrhs)
+{
+    constexpr int TW = kM2lCols / RW;
+    const FmTile& tile = tiles[blockIdx.x];
+    const long long base = T.lv[tile.level].base;
+    for (int q = threadIdx.x; q < kM2lCols * K; q += blockDim.x) {
+        const int c = q / K, row = q % K, t = c / RW, r = c % RW;
+        const int cell = tile.tgt[blockIdx.z * TW + t];
+        if (cell < 0 || r >= nrhs)
+            continue;
+        double v = 0.;
+        for (int s = 0; s < nsplit; s++)
+            v += partial[((((size_t) s * ntiles + blockIdx.x) * gridDim.z + blockIdx.z) * kM2lCols + c) * K + row];
+        Lx[r * lstride + (size_t) (base + cell) * K + row] = v;
+    }
+}
+
+// tiles of the flagged cells of one level (field evaluation): the cells of one class under a block of
+// 4 x 2 x 2 parents; a thread per block and class
+__global__ void fm_tile_kernel(const unsigned char* __restrict__ flag, FmLevel L, int level, FmTile* __restrict__ tiles,
+                               unsigned* __restrict__ count)
+{
+    const int d = L.div, np = L.n / d;
+    const int bx = (np + 3) / 4, by = (np + 1) / 2, bz = by, ncls = d * d * d;
+    const long long total = (long long) bx * by * bz * ncls;
+    for (long long q = blockIdx.x * (long long) blockDim.x + threadIdx.x; q < total;
+         q += (long long) gridDim.x * blockDim.x) {
+        const int cls = (int) (q % ncls);
+        const long long b = q / ncls;
+        const int z0 = (int) (b % bz) * 2, y0 = (int) (b / bz % by) * 2, x0 = (int) (b / bz / by) * 4;
+        const int cx = cls / (d * d), cy = cls / d % d, cz = cls % d;
+        FmTile t;
+        t.level = level;
+        t.cls = cls;
+        bool any = false;
+#pragma unroll
+        for (int k = 0; k < kM2lCols; k++) {
+            const int px = x0 + (k >> 2), py = y0 + (k >> 1 & 1), pz = z0 + (k & 1);
+            t.tgt[k] = -1;
+            if (px < np && py < np && pz < np) {
+                const long long c = ((long long) (px * d + cx) * L.n + (py * d + cy)) * L.n + (pz * d + cz);
+                if (flag[L.base + c]) {
+                    t.tgt[k] = (int) c;
+                    any = true;
+                }
+            }
+        }
+        if (any)
+            tiles[atomicAdd(count, 1u)] = t;
+    }
+}
+
 // ------------------------------------------------------------------------- L2P
 // potential and field of the local expansion Lh (scaled, K reals) at u = (x - c) / side: the
 // regular harmonics by the same recurrences as P2M, streamed (no table), and the gradient by
@@ -478,15 +747,6 @@ __device__ __forceinline__ void fm_l2p(const double* Lh, int p, double ux, doubl
 // KFMElectrostaticFastMultipoleFieldSolver.cc:107-133), compensated (Kahan) like the direct
 // sum. ANALYTIC evaluates every direct pair with the analytic integrals (as the reference's
 // FFTM field solver does, KEBIFactory::MakeAnalytic()), else with the numeric policy.
-struct FmTreeView
-{
-    FmLevel lv[12];
-    int depth;       // the leaves' level
-    int zm;
-    double wx, wy, wz;  // world cube corner (minimum)
-    const int* own_ptr;   // owned-element ranges per cell of every level (level-concatenated, +1)
-    const int* own_elem;  // elements in owner order
-};
 
 //
 // Register budget: the analytic integrals (rwg64) take up to 255 registers unbounded, which left
