@@ -87,23 +87,25 @@ __device__ __noinline__ void rwg_vertex_grad(const double* e, V3 P, const double
     }
 }
 
-// Node-gradient moments of one (element, point) pair for a rule of N nodes from node OFF.
-// With d = P - centroid, node offsets o_k = s'_k (A N1) + t'_k (B N2), r_k = |d - o_k| and
+// Node moments of one (element, point) pair for a rule of N nodes from node OFF. With d = P - centroid,
+// node offsets o_k = s'_k (A N1) + t'_k (B N2), r_k = |d - o_k| and
 //   c1_k = w_k (wphi / r^3 + 3 (wE . (d - o_k)) / r^5),  c2_k = w_k / r^3,
 // the gradient of w . F with respect to node k is pf (c1_k (d - o_k) - c2_k wE), and a vertex
 // gradient is its barycentric weight times that, summed over nodes. Both sums are linear in
 // the node moments m = (sum c1, sum s'c1, sum t'c1, sum s'^2 c1, sum s't' c1, sum t'^2 c1,
-// sum c2, sum s'c2, sum t'c2), accumulated here (9 FMAs per node, no per-node vectors).
+// sum c2, sum s'c2, sum t'c2), and w . F itself is pf (wE . (d m6 - (A N1) m7 - (B N2) m8) + wphi m9)
+// with m9 = sum w_k / r_k: one pass over the nodes gives the density gradient and the vertex gradients.
+// (The reciprocal square root comes doubled, z = 2 / r; the powers of 2 are taken out at the end.)
 constexpr int kQA = 6;
 __constant__ double c_qa[kNumNodes * kQA];  // per node: w, w s', w t', w s'^2, w s't', w t'^2
 template<int N, int OFF, bool FAST>
-__device__ __forceinline__ void node_moments(const double* e, V3 d, V3 wE, double wphi, double m[9])
+__device__ __forceinline__ void node_moments(const double* e, V3 d, double R2, V3 wE, double wphi, double m[10])
 {
     const V3 a = ld3(e + rEa), b = ld3(e + rEb);
-    const double R2 = dot(d, d), Da = dot(d, a), Db = dot(d, b);
+    const double Da = dot(d, a), Db = dot(d, b);
     const double aa = e[rAA], ab2 = e[rAB2], bb = e[rBB];
-    // 3 wE.(d - o_k) = 3 wE.d + (-2 s') (1.5 wE.a) + (-2 t') (1.5 wE.b)
-    const double w3d = 3. * dot(wE, d), w3a = 1.5 * dot(wE, a), w3b = 1.5 * dot(wE, b);
+    // 3/4 wE.(d - o_k) = 3/4 wE.d + (-2 s') (3/8 wE.a) + (-2 t') (3/8 wE.b); 1 / r^2 = z^2 / 4
+    const double w3d = 0.75 * dot(wE, d), w3a = 0.375 * dot(wE, a), w3b = 0.375 * dot(wE, b);
     constexpr int G = N % KEMCU_GROUP == 0 ? KEMCU_GROUP : N;
 #pragma unroll 1
     for (int g = 0; g < N / G; g++) {
@@ -118,21 +120,30 @@ __device__ __forceinline__ void node_moments(const double* e, V3 d, V3 wE, doubl
             q2 = fma(c[2], aa, q2);
             q2 = fma(c[3], ab2, q2);
             q2 = fma(c[4], bb, q2);
-            const double ir = 0.5 * irsq<FAST>(q2), ir2 = ir * ir, ir3 = ir2 * ir;
+            const double z = irsq<FAST>(q2), z2 = z * z, z3 = z2 * z;
             const double wd3 = fma(c[1], w3b, fma(c[0], w3a, w3d));
-            const double c1 = ir3 * fma(wd3, ir2, wphi);
+            const double c1 = z3 * fma(wd3, z2, wphi);
 #pragma unroll
             for (int q = 0; q < 6; q++)
                 m[q] = fma(w[q], c1, m[q]);
 #pragma unroll
             for (int q = 0; q < 3; q++)
-                m[6 + q] = fma(w[q], ir3, m[6 + q]);
+                m[6 + q] = fma(w[q], z3, m[6 + q]);
+            m[9] = fma(w[0], z, m[9]);
         }
     }
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+        m[q] *= 0.125;
+    m[9] *= 0.5;
 }
 
+// Bound by the FP64 pipe: ~28 operations a node (43 when the field and the moments were two passes).
+// Four resident CTAs: the analytic integrals of the near pairs would take 255 registers, which left 8
+// warps per SM.
+constexpr int kAdjMinBlocks = 4;
 template<bool MIXED>
-__global__ void __launch_bounds__(kAdjThreads) vjp_kernel(const double* __restrict__ rec, int n_elem,
+__global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks) vjp_kernel(const double* __restrict__ rec, int n_elem,
                                                           const double* __restrict__ pts, const double* __restrict__ wts,
                                                           int n_pts, double* __restrict__ part_s,
                                                           double* __restrict__ part_g)
@@ -188,35 +199,40 @@ __global__ void __launch_bounds__(kAdjThreads) vjp_kernel(const double* __restri
         for (int q = 0; q < cnt; q++) {
             const V3 P = v3(s_p[q][0], s_p[q][1], s_p[q][2]);
             const double* w = s_w[q];
-            const Out4 F = epi<MIXED, true, true>(e, P);
-            S.add(w[0] * F.ex + w[1] * F.ey + w[2] * F.ez + w[3] * F.phi);
-            if (type == kLineSegment)
-                continue;
-            const int band = band_of(e, P);
-            if (band == 0) {
-                rwg_vertex_grad(e, P, w, g);
+            V3 dc;
+            double r2;
+            const int band = band_of(e, P, dc, r2);
+            if (type == kLineSegment || band == 0) {
+                const Out4 F = epi<MIXED, true, true>(e, P);
+                const double wf = w[0] * F.ex + w[1] * F.ey + w[2] * F.ez + w[3] * F.phi;
+                S.add(wf);
+                if (type != kLineSegment) {
+                    rwg_vertex_grad(e, P, w, g);
+                }
                 continue;
             }
-            // node gradients from the rule's node moments (node_moments), mapped to the vertices
-            const V3 dc = P - ld3(e + rCen), a = ld3(e + rEa), b = ld3(e + rEb);
+            // field and node gradients from the rule's node moments, mapped to the vertices
+            const V3 a = ld3(e + rEa), b = ld3(e + rEb);
             const V3 wE = v3(w[0], w[1], w[2]);
-            double m[9] = {0., 0., 0., 0., 0., 0., 0., 0., 0.};
+            double m[10] = {0., 0., 0., 0., 0., 0., 0., 0., 0., 0.};
             if (type == kTriangle) {
                 if (band == 1)
-                    node_moments<33, kTri33, MIXED>(e, dc, wE, w[3], m);
+                    node_moments<33, kTri33, MIXED>(e, dc, r2, wE, w[3], m);
                 else if (band == 2)
-                    node_moments<12, kTri12, MIXED>(e, dc, wE, w[3], m);
+                    node_moments<12, kTri12, MIXED>(e, dc, r2, wE, w[3], m);
                 else
-                    node_moments<7, kTri7, MIXED>(e, dc, wE, w[3], m);
+                    node_moments<7, kTri7, MIXED>(e, dc, r2, wE, w[3], m);
             }
             else {
                 if (band == 1)
-                    node_moments<33, kRect33, MIXED>(e, dc, wE, w[3], m);
+                    node_moments<33, kRect33, MIXED>(e, dc, r2, wE, w[3], m);
                 else if (band == 2)
-                    node_moments<12, kRect12, MIXED>(e, dc, wE, w[3], m);
+                    node_moments<12, kRect12, MIXED>(e, dc, r2, wE, w[3], m);
                 else
-                    node_moments<7, kRect7, MIXED>(e, dc, wE, w[3], m);
+                    node_moments<7, kRect7, MIXED>(e, dc, r2, wE, w[3], m);
             }
+            const double wf = e[rPrefac] * (w[3] * m[9] + (dot(wE, dc) * m[6] - dot(wE, a) * m[7] - dot(wE, b) * m[8]));
+            S.add(wf);
             {
                 // barycentric weights of the nodes: P1 weight s = s' + sc, P2 weight t = t' + sc
                 const double sc = type == kTriangle ? 1. / 3. : 0.5;
@@ -244,7 +260,6 @@ __global__ void __launch_bounds__(kAdjThreads) vjp_kernel(const double* __restri
                 g[8] += G[2].z;
             }
             // area term for this point: (w . F) dA / A, added per point so the frozen band holds
-            const double wf = w[0] * F.ex + w[1] * F.ey + w[2] * F.ez + w[3] * F.phi;
             g[0] -= wf * (dA1.x + dA2.x);
             g[1] -= wf * (dA1.y + dA2.y);
             g[2] -= wf * (dA1.z + dA2.z);
