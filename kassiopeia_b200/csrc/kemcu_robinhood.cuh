@@ -387,4 +387,123 @@ __global__ void __launch_bounds__(kRhThreads) robin_hood_kernel(const double* __
     }
 }
 
+// The assembled operator's corrections on one CTA, for systems whose rows its registers hold (RPT rows
+// a thread, up to kRhSmallRows). A correction is a chain: column k from L2, the rows' residuals,
+// their argmax, the next k. The argmax takes warp reductions of the residual's bit pattern
+// (non-negative doubles order as their bits: the high words, the low words of those that tie, then
+// the smallest row) and one CTA barrier: every warp reduces the warps' winners itself, from one of two
+// buffers. Seven 32-bit shuffles a step and three barriers took 2.6 us a correction.
+constexpr int kRhSmallThreads = 1024, kRhSmallRows = 4 * kRhSmallThreads;
+
+// the largest (hi, lo) of the warp, its smallest row on ties; rows at or above 2^31 - 1 take no part
+__device__ __forceinline__ int rh_warp_argmax(unsigned& hi, unsigned& lo, int row)
+{
+    const unsigned h = __reduce_max_sync(0xffffffffu, hi);
+    bool in = hi == h && row != 0x7fffffff;
+    const unsigned l = __reduce_max_sync(0xffffffffu, in ? lo : 0u);
+    in = in && lo == l;
+    const int best = (int) __reduce_min_sync(0xffffffffu, in ? (unsigned) row : 0x7fffffffu);
+    hi = h;
+    lo = l;
+    return best;
+}
+
+template<int RPT>
+__global__ void __launch_bounds__(kRhSmallThreads)
+    robin_hood_small_kernel(int n, const double* __restrict__ A, size_t ld, const double* __restrict__ diag,
+                            const double* __restrict__ b, double* __restrict__ bit, double* __restrict__ x, double binf,
+                            double tol, int interval, long long budget, RhState* __restrict__ st)
+{
+    struct Win
+    {
+        double r, d;
+        unsigned hi, lo;
+        int row, pad;
+    };
+    __shared__ Win s_win[2][32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = (int) blockDim.x, nw = T >> 5;
+    double vb[RPT], vbit[RPT], vd[RPT];
+#pragma unroll
+    for (int i = 0; i < RPT; i++) {
+        const int row = tid + i * T;
+        vb[i] = row < n ? b[row] : 0.;
+        vbit[i] = row < n ? bit[row] : 0.;
+        vd[i] = row < n ? diag[row] : 1.;
+    }
+    RhState S = *st;
+    int parity = 0;
+    // the row of the largest |b - b_it| (the first on ties; NaN takes no part), its residual and diagonal
+    auto pick = [&]() {
+        unsigned hi = 0u, lo = 0u;
+        int row = 0x7fffffff;
+        double br = 0., bd = 1., bv = -1.;
+#pragma unroll
+        for (int i = 0; i < RPT; i++) {
+            const double r = vb[i] - vbit[i], v = fabs(r);
+            if (tid + i * T < n && v > bv) {  // rows increase with i
+                bv = v;
+                br = r;
+                bd = vd[i];
+                row = tid + i * T;
+            }
+        }
+        if (row != 0x7fffffff) {
+            hi = (unsigned) __double2hiint(bv);
+            lo = (unsigned) __double2loint(bv);
+        }
+        const int best = rh_warp_argmax(hi, lo, row);
+        if (best == 0x7fffffff ? lane == 0 : row == best)
+            s_win[parity][warp] = Win{br, bd, hi, lo, best, 0};
+        __syncthreads();
+        unsigned h2 = 0u, l2 = 0u;
+        int r2 = 0x7fffffff;
+        if (lane < nw) {
+            h2 = s_win[parity][lane].hi;
+            l2 = s_win[parity][lane].lo;
+            r2 = s_win[parity][lane].row;
+        }
+        const int mine = r2;
+        const int k = rh_warp_argmax(h2, l2, r2);
+        const unsigned who = __ballot_sync(0xffffffffu, mine == k && lane < nw);
+        const Win& w = s_win[parity][__ffs(who) - 1];
+        S.k = k;
+        S.rk = w.r;
+        S.dk = w.d;
+        S.rmax = k == 0x7fffffff ? -1. : fabs(w.r);
+        parity ^= 1;
+    };
+    if (S.k < 0)
+        pick();
+    long long done = 0;
+    while (S.norm > tol && done < budget && S.k != 0x7fffffff) {
+        if (++S.sub % interval == 0) {
+            S.sub = 0;
+            S.norm = S.rmax / binf;
+            S.iterations++;
+        }
+        const int k = S.k;
+        const double* col = A + (size_t) k * ld;
+        double a[RPT];
+#pragma unroll
+        for (int i = 0; i < RPT; i++)
+            a[i] = tid + i * T < n ? __ldg(col + tid + i * T) : 0.;
+        const double c = S.rk / S.dk;
+        if (tid == 0)
+            atomicAdd(x + k, c);  // one thread, in order: no wait for the old value
+#pragma unroll
+        for (int i = 0; i < RPT; i++)
+            vbit[i] = __dadd_rn(vbit[i], __dmul_rn(a[i], c));  // reference rounding, no FMA
+        pick();
+        done++;
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; i++)
+        if (tid + i * T < n)
+            bit[tid + i * T] = vbit[i];
+    if (tid == 0) {
+        S.subiterations += done;
+        *st = S;
+    }
+}
+
 }  // namespace kemcu
