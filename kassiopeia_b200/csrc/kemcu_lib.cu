@@ -25,6 +25,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 using namespace kemcu;
@@ -66,6 +67,7 @@ struct kemcu_ctx
     double* d_far = nullptr;
     FarTile* d_tiles = nullptr;
     double* d_pre = nullptr;
+    int2* d_where = nullptr;  // per element: its far record (16-byte units) and whether it is general
     double* d_rwg = nullptr;  // near records (rwg_build_kernel)
     int ntiles = 0;
     int* d_rows = nullptr;  // matrix rows in Morton order of their collocation points
@@ -379,9 +381,10 @@ int build_far(kemcu_ctx* ctx)
     KC(cudaMalloc(&ctx->d_far, off * sizeof(double)));
     KC(cudaMalloc(&ctx->d_tiles, tiles.size() * sizeof(FarTile)));
     KC(cudaMalloc(&ctx->d_pre, n * sizeof(double)));
+    KC(cudaMalloc(&ctx->d_where, n * sizeof(int2)));
     KC(cudaMemcpy(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(FarTile), cudaMemcpyHostToDevice));
     far_build_kernel<<<(unsigned) ((tiles.size() * kFarSym + 127) / 128), 128, 0, ctx->stream>>>(
-        ctx->d_rec, ctx->d_tiles, ctx->ntiles, gl, ctx->d_far, ctx->d_pre);
+        ctx->d_rec, ctx->d_tiles, ctx->ntiles, gl, ctx->d_far, ctx->d_pre, ctx->d_where);
     KCHECK_LAUNCH();
     KC(cudaMalloc(&ctx->d_rwg, n * wRecSize * sizeof(double)));
     rwg_build_kernel<<<(unsigned) ((n + 127) / 128), 128, 0, ctx->stream>>>(ctx->d_rec, (int) n, ctx->d_rwg);
@@ -1366,6 +1369,7 @@ int kemcu_destroy(kemcu_ctx* ctx)
         cudaFree(ctx->d_far);
         cudaFree(ctx->d_tiles);
         cudaFree(ctx->d_pre);
+        cudaFree(ctx->d_where);
         cudaFree(ctx->d_rwg);
         cudaFree(ctx->d_rows);
         cudaFree(ctx->d_counter);
@@ -1440,6 +1444,7 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     cudaFree(ctx->d_far);
     cudaFree(ctx->d_tiles);
     cudaFree(ctx->d_pre);
+    cudaFree(ctx->d_where);
     cudaFree(ctx->d_rwg);
     cudaFree(ctx->d_rows);
     ctx->d_rec = nullptr;
@@ -1453,6 +1458,7 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     ctx->d_far = nullptr;
     ctx->d_tiles = nullptr;
     ctx->d_pre = nullptr;
+    ctx->d_where = nullptr;
     ctx->d_rwg = nullptr;
     ctx->d_rows = nullptr;
     ctx->ntiles = 0;

@@ -173,7 +173,7 @@ template<class T> __device__ __noinline__ int far_class(const FarTables& t, cons
 // Far record of every element from its element record, one thread per element; the moments of
 // rectangles and wires are closed forms, a triangle's an exact cubature.
 __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* __restrict__ tiles, int ntiles,
-                                 const __grid_constant__ FarTables gl, double* __restrict__ far, double* __restrict__ pre)
+                                 const __grid_constant__ FarTables gl, double* __restrict__ far, double* __restrict__ pre, int2* __restrict__ where)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int ti = q / kFarSym, k = q % kFarSym;
@@ -324,6 +324,7 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
     if (!(s > 0.) || !isfinite(chk))
         for (int i = 0; i < 6; i++)
             f[fCut + i] = CUDART_INF;
+    where[T.first + k] = make_int2(T.off16 + k * stride / 2, T.general);
     pre[T.first + k] = type == kLineSegment ? e[rPrefac] * e[rA] : e[rPrefac];
 }
 

@@ -8,13 +8,17 @@
 //   d/dt (t, s, x, p) = (1, |v|, v, q E(x)),  v = p / (m gamma),  gamma = sqrt(1 + p^2 / (m c)^2)
 // with E(x) the Kahan-summed direct sum of KIntegratingFieldSolver::ElectricField.
 //
-// Layout: a CTA owns kTrackSlots slots (one per thread). Every RK stage of all slots of a CTA
-// is one pass over the element records, streamed through a cyclic shared-memory ring
-// (ElementRing, bulk copies; no CTA barrier per tile, so warps drift up to a tile apart); the
-// 13 stage derivatives of each slot live in shared memory. A slot whose track ends (electrode
-// hit, leaving the volume, step limit, non-finite state) or has taken `budget` steps in this
-// launch writes it back and takes the next track index from a global work counter, so tracks
-// of very different lengths keep every slot busy and one launch advances every listed track
+// Layout: a CTA owns 32 slots, one per lane, and W warps that share the elements: warp w sums
+// elements w, w + W, ... for all 32 slots, and warp 0 adds the warps' sums in order and advances the
+// slots. The element records come a warp at a time through its own piece of shared memory, the next
+// one's loads in flight during the pairs of this one, so a stage has no CTA barrier but the two around
+// it. (One thread per track left 4 warps on an SM at 16,384 tracks, waiting for FP64 latencies.) Slots
+// take tracks in Morton order of their positions, so that a warp's lanes agree on an element's form;
+// each lane takes the form its own distance asks for, whoever its neighbours are, so a track does not
+// depend on the others. The 13 stage derivatives of each slot live in shared memory. A slot whose
+// track ends (electrode hit, leaving the volume, step limit, non-finite state) or has taken `budget`
+// steps in this launch writes it back and takes the next track of the list from a global work counter,
+// so tracks of very different lengths keep every slot busy and one launch advances every listed track
 // by at most `budget` steps; unfinished tracks stay active for the next launch.
 #pragma once
 
@@ -23,9 +27,8 @@
 namespace kemcu
 {
 
-constexpr int kTrackSlots = 128;
+constexpr int kTrackSlots = 32;  // per CTA: a lane each
 constexpr int kStages = 13;
-constexpr int kTrackPipe = 3;  // ring stages (the stage derivatives take most shared memory)
 constexpr int kTrackK = 6;     // stored per stage and slot: v (3), q E (3)
 
 // Butcher coefficients a[s][k] (row s gives stage value s from derivatives 0..s; row 12 is
@@ -82,34 +85,58 @@ inline unsigned rk8_live_stages(const double a[kStages][kStages])
     return live;
 }
 
+// the field of one element at X per unit charge density, by the form the lane's distance asks for: the
+// series wherever one holds, in its nearest tier (the farther ones are cheaper, but the lanes of a warp
+// lie on both sides of their cuts and would run both), else the cubature bands or the analytic integrals. f: far record, e: element record, w: near record.
+template<bool MIXED> __device__ __forceinline__ V3 track_pair(const double* f, bool general, const double* e,
+                                                              const double* __restrict__ w, double pre, V3 X)
+{
+    const double* c = f + (MIXED ? fCutM : fCut);
+    const V3 d0 = v3(X.x - f[fCen], X.y - f[fCen + 1], X.z - f[fCen + 2]);
+    const double d2 = dot(d0, d0) * (1. - 1e-9);
+    if (d2 > c[2] * c[2]) {
+        const V3 P[1] = {X};
+        V3 d[1];
+        FarSum F[1];
+        if (general)
+            far_pairs<true, 1, true, MIXED>(f, P, d, F);
+        else
+            far_pairs<false, 1, true, MIXED>(f, P, d, F);
+        const double k = pre * F[0].ir * F[0].ir, a = (k * F[0].ir) * F[0].cd, b = -k * F[0].c1, q = -k * F[0].c2;
+        const V3 e1 = ld3(f + fE1), e2 = ld3(f + fE1 + 3);
+        return v3(fma(a, d[0].x, fma(b, e1.x, q * e2.x)), fma(a, d[0].y, fma(b, e1.y, q * e2.y)),
+                  fma(a, d[0].z, fma(b, e1.z, q * e2.z)));
+    }
+    const Out4 r = epi<MIXED, false, true>(e, w, X);
+    return v3(r.ex, r.ey, r.ez);
+}
+
+// far record of element j: its tile holds kFarSym symmetric or kFarGen general elements in order
+struct TrackElems
+{
+    FarView V;
+    const double* rec;
+    const int2* where;  // per element: offset of its far record in 16-byte units, general
+    const double* sigma;
+    int n;
+};
+
 // state: n x 8; steps, status: n; list: n_list track indices to work on; next: work counter;
 // done_steps: total steps taken (for statistics); dpsum (n, may be null): per track the sum over
-// its steps of |p_after - p_before|, accumulated; flag |= 2 if a ring wait timed out.
-// Dynamic shared memory: kStages * kTrackK * kTrackSlots doubles.
-template<bool MIXED>
-__global__ void __launch_bounds__(kTrackSlots) rk8_tracker_kernel(const double* __restrict__ rec, const double* __restrict__ sigma,
-                                                                  int n_elem, double* __restrict__ state,
-                                                                  int* __restrict__ steps, int* __restrict__ status,
-                                                                  const int* __restrict__ list, unsigned* __restrict__ next,
-                                                                  unsigned long long* __restrict__ done_steps,
-                                                                  double* __restrict__ dpsum, TrackParams prm,
-                                                                  int* __restrict__ flag)
+// its steps of |p_after - p_before|, accumulated.
+template<bool MIXED, int W>
+__global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems el, double* __restrict__ state,
+                                                                     int* __restrict__ steps, int* __restrict__ status,
+                                                                     const int* __restrict__ list,
+                                                                     unsigned* __restrict__ next,
+                                                                     unsigned long long* __restrict__ done_steps,
+                                                                     double* __restrict__ dpsum, TrackParams prm)
 {
-    extern __shared__ __align__(16) double s_k[];  // [kStages][kTrackK][kTrackSlots]
-    __shared__ __align__(128) RingStorage<1, kTrackPipe> S;
-    __shared__ int s_abort;
-    const int tid = threadIdx.x;
-    auto K = [&](int st, int c) -> double& { return s_k[(st * kTrackK + c) * kTrackSlots + tid]; };
-    if (tid == 0)
-        s_abort = 0;
-    ElementRing<1, kTrackPipe, true> R(S, 0, n_elem);  // synchronises the CTA
-    auto side = [&](double (*sd)[kFieldTile], int t0, int cnt, int lane) {
-        if (lane < cnt)
-            sd[0][lane] = sigma[t0 + lane];
-    };
-    R.prologue(rec, side);
-    const int ntiles = R.tiles();
-
+    __shared__ double s_k[kStages][kTrackK][kTrackSlots];
+    __shared__ double s_x[3][kTrackSlots];
+    __shared__ __align__(16) double s_far[W][kFarGenStride], s_rec[W][rRecSize];
+    __shared__ int s_any;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int track = -1, tsteps = 0;
     double y[8];
     double dps = 0.;
@@ -126,75 +153,126 @@ __global__ void __launch_bounds__(kTrackSlots) rk8_tracker_kernel(const double* 
             dps = dpsum ? dpsum[track] : 0.;
         }
     };
-    pull();
+    // this warp's share of the field at the 32 slot positions
+    auto field = [&]() {
+        const V3 X = v3(s_x[0][lane], s_x[1][lane], s_x[2][lane]);
+        Kahan ex, ey, ez;
+        constexpr int NV = (kFarGenStride + 31) / 32;
+        double v[NV], r = 0., pre_next = 0., sg_next = 0.;
+        int2 at = make_int2(0, 0);
+        auto fetch = [&](int j) {
+            at = el.where[j];
+            const double* f = el.V.far + 2 * (size_t) at.x;
+            const int len = at.y ? kFarGenStride : kFarSymStride;
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                if (lane + 32 * k < len)
+                    v[k] = __ldg(f + lane + 32 * k);
+            r = __ldg(el.rec + (size_t) j * rRecSize + lane);
+            pre_next = __ldg(el.V.pre + j);
+            sg_next = __ldg(el.sigma + j);
+        };
+        if (warp < el.n)
+            fetch(warp);
+        for (int j = warp; j < el.n; j += W) {
+            __syncwarp();
+            const bool general = at.y != 0;
+            const int len = general ? kFarGenStride : kFarSymStride;
+#pragma unroll
+            for (int k = 0; k < NV; k++)
+                if (lane + 32 * k < len)
+                    s_far[warp][lane + 32 * k] = v[k];
+            s_rec[warp][lane] = r;
+            __syncwarp();
+            const double pre = pre_next, sg = sg_next;
+            if (j + W < el.n)
+                fetch(j + W);
+            const V3 E = track_pair<MIXED>(s_far[warp], general, s_rec[warp], el.V.rwg + (size_t) j * wRecSize, pre, X);
+            ex.add(E.x * sg);
+            ey.add(E.y * sg);
+            ez.add(E.z * sg);
+        }
+        __syncwarp();  // the record's piece now takes the warp's sums
+        s_far[warp][lane] = ex.s;
+        s_far[warp][32 + lane] = ey.s;
+        s_far[warp][64 + lane] = ez.s;
+    };
+    if (warp == 0)
+        pull();
     unsigned long long my_steps = 0;
-    int gi = 0;  // position in the ring's tile sequence
-    bool ok = true;
-    // every iteration is one RK8 step of all busy slots; ends when the list is exhausted (or a
-    // ring wait of some warp timed out)
+    // every iteration is one RK8 step of all busy slots; ends when the list is exhausted
     while (true) {
-        const int any = __syncthreads_or(track >= 0);
-        if (!any || s_abort)
+        if (warp == 0) {
+            const bool any = __any_sync(0xffffffffu, track >= 0);
+            // slots without a track sit where some busy slot is: they take its elements' forms
+            const unsigned busy = __ballot_sync(0xffffffffu, track >= 0);
+            if (any) {
+                const int src = track >= 0 ? lane : __ffs(busy) - 1;
+                for (int c = 0; c < 8; c++) {
+                    const double q = __shfl_sync(0xffffffffu, y[c], src);
+                    if (track < 0)
+                        y[c] = q;
+                }
+            }
+            if (lane == 0)
+                s_any = any;
+        }
+        __syncthreads();
+        if (!s_any)
             break;
         double ds = 0.;  // sum over stages of a[12][k] |v_k|
         for (int st = 0; st < kStages; st++) {
             if (!((prm.live >> st) & 1u))
                 continue;  // unused derivative (its column of the table is zero): not evaluated
-            // stage position and momentum: value_{st-1} = y0 + dt sum_k a[st-1][k] k_k
-            V3 X = v3(y[2], y[3], y[4]), Pm = v3(y[5], y[6], y[7]);
-            if (track >= 0 && st > 0) {
-                double sx = 0., sy = 0., sz = 0., px = 0., py = 0., pz = 0.;
-                for (int k = 0; k < st; k++) {
-                    if (!((prm.live >> k) & 1u))
-                        continue;
-                    const double a = c_rk8[st - 1][k];
-                    sx += a * K(k, 0);
-                    sy += a * K(k, 1);
-                    sz += a * K(k, 2);
-                    px += a * K(k, 3);
-                    py += a * K(k, 4);
-                    pz += a * K(k, 5);
-                }
-                X = v3(y[2] + prm.dt * sx, y[3] + prm.dt * sy, y[4] + prm.dt * sz);
-                Pm = v3(y[5] + prm.dt * px, y[6] + prm.dt * py, y[7] + prm.dt * pz);
-            }
-            // E(X): one pass of all elements through the ring
-            Kahan ex, ey, ez;
-            if (ok) {
-                for (int i = 0; i < ntiles; i++, gi++) {
-                    if (!__all_sync(0xffffffffu, R.wait(gi))) {
-                        ok = false;
-                        s_abort = 1;
-                        break;
+            V3 Pm = v3(0., 0., 0.);
+            if (warp == 0) {
+                // stage position and momentum: value_{st-1} = y0 + dt sum_k a[st-1][k] k_k
+                V3 X = v3(y[2], y[3], y[4]);
+                Pm = v3(y[5], y[6], y[7]);
+                if (st > 0) {
+                    double sx = 0., sy = 0., sz = 0., px = 0., py = 0., pz = 0.;
+                    for (int k = 0; k < st; k++) {
+                        if (!((prm.live >> k) & 1u))
+                            continue;
+                        const double a = c_rk8[st - 1][k];
+                        sx += a * s_k[k][0][lane];
+                        sy += a * s_k[k][1][lane];
+                        sz += a * s_k[k][2][lane];
+                        px += a * s_k[k][3][lane];
+                        py += a * s_k[k][4][lane];
+                        pz += a * s_k[k][5][lane];
                     }
-                    if (track >= 0) {
-                        const int cnt = R.count(gi);
-                        for (int j = 0; j < cnt; j++) {
-                            const Out4 r = epi<MIXED, false, true>(R.element(gi, j), X);
-                            const double sg = R.side(gi, 0, j);
-                            ex.add(r.ex * sg);
-                            ey.add(r.ey * sg);
-                            ez.add(r.ez * sg);
-                        }
-                    }
-                    R.release(rec, gi, side);
+                    X = v3(y[2] + prm.dt * sx, y[3] + prm.dt * sy, y[4] + prm.dt * sz);
+                    Pm = v3(y[5] + prm.dt * px, y[6] + prm.dt * py, y[7] + prm.dt * pz);
                 }
+                s_x[0][lane] = X.x;
+                s_x[1][lane] = X.y;
+                s_x[2][lane] = X.z;
             }
-            if (track >= 0) {
+            __syncthreads();
+            field();
+            __syncthreads();
+            if (warp == 0) {
+                Kahan ex, ey, ez;
+                for (int w = 0; w < W; w++) {
+                    ex.add(s_far[w][lane]);
+                    ey.add(s_far[w][32 + lane]);
+                    ez.add(s_far[w][64 + lane]);
+                }
                 const double p2 = dot(Pm, Pm);
                 const double gam = sqrt(1. + p2 / (prm.mass * prm.mass * prm.c2));
                 const double inv = 1. / (prm.mass * gam);
                 const double vx = inv * Pm.x, vy = inv * Pm.y, vz = inv * Pm.z;
-                K(st, 0) = vx;
-                K(st, 1) = vy;
-                K(st, 2) = vz;
-                K(st, 3) = prm.charge * ex.s;
-                K(st, 4) = prm.charge * ey.s;
-                K(st, 5) = prm.charge * ez.s;
+                s_k[st][0][lane] = vx;
+                s_k[st][1][lane] = vy;
+                s_k[st][2][lane] = vz;
+                s_k[st][3][lane] = prm.charge * ex.s;
+                s_k[st][4][lane] = prm.charge * ey.s;
+                s_k[st][5][lane] = prm.charge * ez.s;
                 ds += c_rk8[kStages - 1][st] * sqrt(vx * vx + vy * vy + vz * vz);
             }
         }
-        if (track >= 0 && ok) {
+        if (warp == 0 && track >= 0) {
             // final combination (row 12) for t (derivative 1), s (|v|), x and p
             double dtt = 0., d[6] = {0., 0., 0., 0., 0., 0.};
             for (int k = 0; k < kStages; k++) {
@@ -203,7 +281,7 @@ __global__ void __launch_bounds__(kTrackSlots) rk8_tracker_kernel(const double* 
                 if (!((prm.live >> k) & 1u))
                     continue;
                 for (int c = 0; c < 6; c++)
-                    d[c] += a * K(k, c);
+                    d[c] += a * s_k[k][c][lane];
             }
             y[0] += prm.dt * dtt;
             y[1] += prm.dt * ds;
@@ -242,9 +320,27 @@ __global__ void __launch_bounds__(kTrackSlots) rk8_tracker_kernel(const double* 
                 pull();
             }
         }
+        __syncthreads();  // s_any is read before warp 0 writes it again
     }
-    R.finish(ok, flag);
-    atomicAdd(done_steps, my_steps);
+    if (warp == 0)
+        atomicAdd(done_steps, my_steps);
+}
+
+// positions of the listed tracks (for their Morton order), and the list in that order
+__global__ void track_points_kernel(const double* __restrict__ state, const int* __restrict__ list, int n,
+                                    double* __restrict__ P)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        for (int c = 0; c < 3; c++)
+            P[3 * i + c] = state[(size_t) list[i] * 8 + 2 + c];
+}
+__global__ void track_permute_kernel(const int* __restrict__ list, const int* __restrict__ perm, int n,
+                                     int* __restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        out[i] = list[perm[i]];
 }
 
 // list of ACTIVE tracks: list[atomicAdd(count)] = i for status[i] == 0

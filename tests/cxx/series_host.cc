@@ -26,6 +26,8 @@ inline V3 ld3(const double* p) { return v3(p[0], p[1], p[2]); }
 template<bool FAST> double irsq(double x) { return 2. / std::sqrt(x); }
 struct float4 { float x, y, z, w; };
 struct double2 { double x, y; };
+struct int2 { int x, y; };
+inline int2 make_int2(int x, int y) { return int2{x, y}; }
 struct Dim { int x; };
 static Dim blockIdx, blockDim{1}, threadIdx;
 }  // namespace kemcu
@@ -66,7 +68,8 @@ extern "C" void series_host(const double* rec, int general, int mixed, int tier,
     far_tables(gl);
     for (int i = 0; i < kFarQ; i++)
         gl.x[i] = gx[i], gl.w[i] = gw[i];
-    far_build_kernel(rec, &T, 1, gl, far, &pre);
+    int2 where;
+    far_build_kernel(rec, &T, 1, gl, far, &pre, &where);
     for (int k = 0; k < 3; k++)
         cuts[k] = far[(mixed ? fCutM : fCut) + k];
     for (int i = 0; i < n; i += 2) {  // pairs of points, n even
