@@ -95,7 +95,7 @@ __device__ __noinline__ void rwg_vertex_grad(const double* e, V3 P, const double
 // the node moments m = (sum c1, sum s'c1, sum t'c1, sum s'^2 c1, sum s't' c1, sum t'^2 c1,
 // sum c2, sum s'c2, sum t'c2), and w . F itself is pf (wE . (d m6 - (A N1) m7 - (B N2) m8) + wphi m9)
 // with m9 = sum w_k / r_k: one pass over the nodes gives the density gradient and the vertex gradients.
-// (The reciprocal square root comes doubled, z = 2 / r; the powers of 2 are taken out at the end.)
+// (MIXED's reciprocal square root comes doubled, z = 2 / r; the powers of 2 are taken out at the end.)
 constexpr int kQA = 6;
 __constant__ double c_qa[kNumNodes * kQA];  // per node: w, w s', w t', w s'^2, w s't', w t'^2
 template<int N, int OFF, bool FAST>
@@ -104,8 +104,9 @@ __device__ __forceinline__ void node_moments(const double* e, V3 d, double R2, V
     const V3 a = ld3(e + rEa), b = ld3(e + rEb);
     const double Da = dot(d, a), Db = dot(d, b);
     const double aa = e[rAA], ab2 = e[rAB2], bb = e[rBB];
-    // 3/4 wE.(d - o_k) = 3/4 wE.d + (-2 s') (3/8 wE.a) + (-2 t') (3/8 wE.b); 1 / r^2 = z^2 / 4
-    const double w3d = 0.75 * dot(wE, d), w3a = 0.375 * dot(wE, a), w3b = 0.375 * dot(wE, b);
+    // with z = kIrsq / r: 3 wE.(d - o_k) / r^2 = z^2 q (wE.d + (-2 s') wE.a / 2 + (-2 t') wE.b / 2)
+    constexpr double u = kPotScale<FAST>, q3 = 3. * u * u;
+    const double w3d = q3 * dot(wE, d), w3a = (0.5 * q3) * dot(wE, a), w3b = (0.5 * q3) * dot(wE, b);
     constexpr int G = N % KEMCU_GROUP == 0 ? KEMCU_GROUP : N;
 #pragma unroll 1
     for (int g = 0; g < N / G; g++) {
@@ -134,8 +135,8 @@ __device__ __forceinline__ void node_moments(const double* e, V3 d, double R2, V
     }
 #pragma unroll
     for (int q = 0; q < 9; q++)
-        m[q] *= 0.125;
-    m[9] *= 0.5;
+        m[q] *= kFieldScale<FAST>;
+    m[9] *= u;
 }
 
 // Bound by the FP64 pipe: ~28 operations a node (43 when the field and the moments were two passes).

@@ -20,7 +20,7 @@
 // forming the node and the difference vector, and the field sum collapses to
 // d S0 - (A N1) Ss - (B N2) St with three scalar node sums. Two reciprocal square roots, both
 // from the FP32-class hardware estimate (rsqrt.approx.f64, ~2^-23 relative):
-//   * FP64  -- refined by two FP64 Newton steps (within one unit in the last place);
+//   * FP64  -- refined by one FP64 step of third order (within one unit in the last place);
 //   * MIXED -- refined by one FP64 Newton step (~1e-13 relative).
 // RWG near-field integrals and the analytic line segment are FP64 in both forms.
 #pragma once
@@ -28,6 +28,8 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 namespace kemcu
 {
@@ -217,38 +219,61 @@ __device__ __forceinline__ double rsqrt2_acc(double x)
     const double e4 = fma(-(x * z), z, 4.);
     return fma(0.125 * z, e4, z);
 }
-// the reciprocal square root of a form, returned doubled (folded back by kPotScale/kFieldScale)
+// The FP64 reciprocal square root to within about one unit in the last place in one step of third
+// order from the hardware estimate y0 (relative error below 2^-22): with e = 1 - x y0^2,
+// 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3 e^2/8 + O(e^3)), and 5 e^3/16 < 1e-19. Five FP64
+// operations after the estimate (the two Newton steps of rsqrt2_acc take seven).
+__device__ __forceinline__ double rsqrt_cubic(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.);
+    return fma(fma(e, 0.375, 0.5), e * y, y);
+}
+// kIrsq times the reciprocal square root of a form: MIXED returns it doubled (rsqrt2_fast), callers
+// fold the powers of kIrsq into their element sums
 template<bool FAST> __device__ __forceinline__ double irsq(double x)
 {
-    return FAST ? rsqrt2_fast(x) : rsqrt2_acc(x);
+    return FAST ? rsqrt2_fast(x) : rsqrt_cubic(x);
 }
-template<bool FAST> constexpr double kPotScale = 0.5;
-template<bool FAST> constexpr double kFieldScale = 0.125;
+template<bool FAST> constexpr double kIrsq = FAST ? 2. : 1.;
+template<bool FAST> constexpr double kPotScale = 1. / kIrsq<FAST>;
+template<bool FAST> constexpr double kFieldScale = kPotScale<FAST> * kPotScale<FAST> * kPotScale<FAST>;
 
-// Nodes per unrolled group of the node loop (rules whose size it divides are run as a loop
-// over groups, the others fully unrolled). The reciprocal square root of the MIXED form is
-// straight-line code, so a fully unrolled 33-point rule lets the compiler interleave all 33
-// nodes and spill; a loop over groups bounds that window.
+// Nodes per group of a rule (a rule whose size it does not divide is one group). A group is unrolled
+// with its constants at fixed offsets of the constant bank, so that they are operands of the
+// arithmetic; the groups follow one another in the code, held apart by an empty asm through which C1
+// and C2 pass, because the compiler would interleave 33 unrolled nodes and spill. (As a loop over the
+// groups the same code takes a constant load per constant wherever the compiler cannot prove the
+// group index uniform over the warp, such as in a function that is not inlined: a fifth of the
+// instructions of the matrix-free product.)
 #ifndef KEMCU_GROUP
 #define KEMCU_GROUP 11
 #endif
+template<int I, int N, class F> __device__ __forceinline__ void node_groups(double& C1, double& C2, F one)
+{
+    if constexpr (I < N) {
+        constexpr int G = N % KEMCU_GROUP == 0 ? KEMCU_GROUP : N;
+        one(std::integral_constant<int, I>(), std::integral_constant<int, G>());
+        if constexpr (I + G < N) {
+            asm volatile("" : "+d"(C1), "+d"(C2));
+            node_groups<I + G, N>(C1, C2, one);
+        }
+    }
+}
 
-// N nodes of the rule starting at node OFF (both compile-time, so the rule constants are
-// constant-bank operands with fixed offsets within a group)
+// N nodes of the rule starting at node OFF
 template<int N, int OFF, bool POT, bool FIELD, bool FAST>
 __device__ __forceinline__ Out4 cubq(const double* e, V3 d, double R2)
 {
     const V3 a = ld3(e + rEa), b = ld3(e + rEb);
-    const double C1 = dot(d, a), C2 = dot(d, b);  // the rule tables carry the factor -2
+    double C1 = dot(d, a), C2 = dot(d, b);  // the rule tables carry the factor -2
     const double aa = e[rAA], ab2 = e[rAB2], bb = e[rBB];
     double sp = 0., s0 = 0., ss = 0., st = 0.;
-    constexpr int G = N % KEMCU_GROUP == 0 ? KEMCU_GROUP : N;
-#pragma unroll 1
-    for (int g = 0; g < N / G; g++) {
-        const double* cg = c_q + kQ * (OFF + g * G);
+    node_groups<0, N>(C1, C2, [&](auto first, auto count) {
 #pragma unroll
-        for (int k = 0; k < G; k++) {
-            const double* c = cg + kQ * k;
+        for (int k = 0; k < decltype(count)::value; k++) {
+            const double* c = c_q + kQ * (OFF + decltype(first)::value + k);
             double q2 = fma(c[0], C1, R2);
             q2 = fma(c[1], C2, q2);
             q2 = fma(c[2], aa, q2);
@@ -264,7 +289,7 @@ __device__ __forceinline__ Out4 cubq(const double* e, V3 d, double R2)
                 st = fma(c[7], ir3, st);
             }
         }
-    }
+    });
     const double pf = e[rPrefac];
     Out4 o{0., 0., 0., 0.};
     if (POT)
@@ -395,13 +420,11 @@ __device__ __forceinline__ Out4 cubq32(const double* e, V3 d, double R2)
     const V3 a = ld3(e + rEa), b = ld3(e + rEb);
     const Far32 f = far32_setup(e, d, R2, a, b);
     float sp = 0.f, s0 = 0.f, ss = 0.f, st = 0.f;
-    constexpr int G = N % KEMCU_GROUP == 0 ? KEMCU_GROUP : N;
-#pragma unroll 1
-    for (int g = 0; g < N / G; g++) {
-        const float* cg = c_q32 + kQ * (OFF + g * G);
+    double C1 = 0., C2 = 0.;  // (the groups' fence)
+    node_groups<0, N>(C1, C2, [&](auto first, auto count) {
 #pragma unroll
-        for (int k = 0; k < G; k++) {
-            const float* c = cg + kQ * k;
+        for (int k = 0; k < decltype(count)::value; k++) {
+            const float* c = c_q32 + kQ * (OFF + decltype(first)::value + k);
             float x = c[4] * f.bb;
             x = fmaf(c[3], f.ab, x);
             x = fmaf(c[2], f.aa, x);
@@ -417,7 +440,7 @@ __device__ __forceinline__ Out4 cubq32(const double* e, V3 d, double R2)
                 st = fmaf(c[7], r3, st);
             }
         }
-    }
+    });
     return far32_finish<POT, FIELD>(e, d, a, b, f, sp, s0, ss, st);
 }
 

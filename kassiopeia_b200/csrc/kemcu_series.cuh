@@ -465,25 +465,31 @@ __device__ __forceinline__ void far_sym(const double* f, const double (&X)[NP], 
 }
 
 // other elements. n = 2, 3, 4 in FP64, in the FP64 form also n = 5 unless TIER == 3; the rest to
-// n = 6, 8, 10 (TIER 3, 2, 1) in FP32
+// n = 6, 8, 10 (TIER 3, 2, 1) in FP32. The FP32 tail is put together in FP32 (X Po + Y Qo + t (Pe + XY Qe))
+// and joins as four numbers: sixteen conversions of its classes' accumulators cost more than that.
 template<int TIER, bool FIELD, bool FAST, int NP>
 __device__ __forceinline__ void far_gen(const double* f, const double (&X)[NP], const double (&Y)[NP], double s,
                                         FarSum (&F)[NP])
 {
+    constexpr bool d5 = TIER != 3 && !FAST;  // n = 5 in FP64
     const float* g = reinterpret_cast<const float*>(f + fGenF);
-    double x2[NP], y2[NP], h[NP];
+    double x2[NP], y2[NP], h[NP], t[NP];
     float xf[NP], yf[NP], hf[NP];
+    // the tail over t^5, and its gradient's three sums
+    float Sf[NP], Wf[NP], Gx[NP], Gy[NP];
 #pragma unroll
     for (int p = 0; p < NP; p++) {
-        const double t = s * F[p].ir;
-        x2[p] = X[p] * X[p], y2[p] = Y[p] * Y[p], h[p] = t * t;
-        xf[p] = (float) x2[p], yf[p] = (float) y2[p], hf[p] = (float) h[p];
+        t[p] = s * F[p].ir;
+        x2[p] = X[p] * X[p], y2[p] = Y[p] * Y[p], h[p] = t[p] * t[p];
     }
-    // the odd orders, X Po + Y Qo, then the even ones, Pe + XY Qe
-    FarAcc<double> A[NP], C[NP];
-    double So[NP], Wo[NP], ox[NP], oy[NP];
     {
-        FarAcc<float> po[NP], qo[NP];
+        float Xs[NP], Ys[NP], ts[NP];
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            Xs[p] = (float) X[p], Ys[p] = (float) Y[p], ts[p] = (float) t[p];
+            xf[p] = Xs[p] * Xs[p], yf[p] = Ys[p] * Ys[p], hf[p] = ts[p] * ts[p];
+        }
+        FarAcc<float> po[NP], qo[NP], pe[NP], qe[NP];
         if (TIER == 1) {
             far_step<4, FIELD, true>(po, g + kG9p, xf, yf, hf, 10.f);
             far_step<4, FIELD, true>(qo, g + kG9q, xf, yf, hf, 10.f);
@@ -492,16 +498,51 @@ __device__ __forceinline__ void far_gen(const double* f, const double (&X)[NP], 
             far_step<3, FIELD, TIER == 2>(po, g + kG7p, xf, yf, hf, 8.f);
             far_step<3, FIELD, TIER == 2>(qo, g + kG7q, xf, yf, hf, 8.f);
         }
-        if (TIER == 3 || FAST) {
+        if (!d5) {
             far_step<2, FIELD, TIER == 3>(po, g + kG5p, xf, yf, hf, 6.f);
             far_step<2, FIELD, TIER == 3>(qo, g + kG5q, xf, yf, hf, 6.f);
         }
-        far_up<FIELD>(po, A);
-        far_up<FIELD>(qo, C);
-        if (TIER <= 2 && !FAST) {
-            far_step<2, FIELD, false>(A, f + fGenD5, x2, y2, h, 6.);
-            far_step<2, FIELD, false>(C, f + fGenD5 + 6, x2, y2, h, 6.);
+        // odd part: n = 5 first (n = 7 first where 5 is in FP64: one more h)
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            const float u = d5 ? hf[p] : 1.f;
+            Sf[p] = u * fmaf(Xs[p], po[p].v, Ys[p] * qo[p].v);
+            if (FIELD) {
+                const float xy2 = 2.f * Xs[p] * Ys[p];
+                Wf[p] = u * fmaf(Xs[p], po[p].w, Ys[p] * qo[p].w);
+                Gx[p] = u * fmaf(xy2, qo[p].x, fmaf(2.f * xf[p], po[p].x, po[p].v));
+                Gy[p] = u * fmaf(xy2, po[p].y, fmaf(2.f * yf[p], qo[p].y, qo[p].v));
+            }
         }
+        if (TIER == 1) {
+            far_step<5, FIELD, true>(pe, g + kG10p, xf, yf, hf, 11.f);
+            far_step<4, FIELD, true>(qe, g + kG10q, xf, yf, hf, 11.f);
+        }
+        if (TIER <= 2) {
+            far_step<4, FIELD, TIER == 2>(pe, g + kG8p, xf, yf, hf, 9.f);
+            far_step<3, FIELD, TIER == 2>(qe, g + kG8q, xf, yf, hf, 9.f);
+        }
+        far_step<3, FIELD, TIER == 3>(pe, g + kG6p, xf, yf, hf, 7.f);
+        far_step<2, FIELD, TIER == 3>(qe, g + kG6q, xf, yf, hf, 7.f);
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            const float xy = Xs[p] * Ys[p];
+            Sf[p] = fmaf(ts[p], fmaf(xy, qe[p].v, pe[p].v), Sf[p]);
+            if (FIELD) {
+                Wf[p] = fmaf(ts[p], fmaf(xy, qe[p].w, pe[p].w), Wf[p]);
+                Gx[p] = fmaf(ts[p], fmaf(2.f * Xs[p], pe[p].x, Ys[p] * fmaf(2.f * xf[p], qe[p].x, qe[p].v)), Gx[p]);
+                Gy[p] = fmaf(ts[p], fmaf(2.f * Ys[p], pe[p].y, Xs[p] * fmaf(2.f * yf[p], qe[p].y, qe[p].v)), Gy[p]);
+            }
+        }
+    }
+    // FP64: X Po + Y Qo of n = 3 (and 5), Pe + XY Qe of n = 2, 4
+    FarAcc<double> A[NP], C[NP];
+    if (d5) {
+        far_step<2, FIELD, true>(A, f + fGenD5, x2, y2, h, 6.);
+        far_step<2, FIELD, true>(C, f + fGenD5 + 6, x2, y2, h, 6.);
+    }
+    double So[NP], Wo[NP], ox[NP], oy[NP];
+    {
         double k3[6];
         far_load(f + fGenD3, k3);
 #pragma unroll
@@ -509,12 +550,16 @@ __device__ __forceinline__ void far_gen(const double* f, const double (&X)[NP], 
             double v, vx, vy;
             auto add = [&](FarAcc<double>& Q, const double* c) {
                 far_poly<1, FIELD>(c, x2[p], y2[p], v, vx, vy);
-                Q.v = fma(Q.v, h[p], v);
-                if (FIELD) {
-                    Q.w = fma(Q.w, h[p], 4. * v);
-                    Q.x = fma(Q.x, h[p], vx);
-                    Q.y = fma(Q.y, h[p], vy);
+                if (d5) {
+                    Q.v = fma(Q.v, h[p], v);
+                    if (FIELD) {
+                        Q.w = fma(Q.w, h[p], 4. * v);
+                        Q.x = fma(Q.x, h[p], vx);
+                        Q.y = fma(Q.y, h[p], vy);
+                    }
                 }
+                else
+                    Q = FarAcc<double>{v, 4. * v, vx, vy};
             };
             add(A[p], k3);
             add(C[p], k3 + 3);
@@ -527,42 +572,29 @@ __device__ __forceinline__ void far_gen(const double* f, const double (&X)[NP], 
             }
         }
     }
-    {
-        FarAcc<float> pe[NP], qe[NP];
-        if (TIER == 1) {
-            far_step<5, FIELD, true>(pe, g + kG10p, xf, yf, hf, 11.f);
-            far_step<4, FIELD, true>(qe, g + kG10q, xf, yf, hf, 11.f);
-        }
-        if (TIER <= 2) {
-            far_step<4, FIELD, TIER == 2>(pe, g + kG8p, xf, yf, hf, 9.f);
-            far_step<3, FIELD, TIER == 2>(qe, g + kG8q, xf, yf, hf, 9.f);
-        }
-        far_step<3, FIELD, TIER == 3>(pe, g + kG6p, xf, yf, hf, 7.f);
-        far_step<2, FIELD, TIER == 3>(qe, g + kG6q, xf, yf, hf, 7.f);
-        far_up<FIELD>(pe, A);
-        far_up<FIELD>(qe, C);
-        far_step<2, FIELD, false>(A, f + fD4, x2, y2, h, 5.);
-        far_step<1, FIELD, false>(C, f + fGenQ4, x2, y2, h, 5.);
-        double k2[4];
-        far_load(f + fD2, k2);
+    far_step<2, FIELD, true>(A, f + fD4, x2, y2, h, 5.);
+    far_step<1, FIELD, true>(C, f + fGenQ4, x2, y2, h, 5.);
+    double k2[4];
+    far_load(f + fD2, k2);
 #pragma unroll
-        for (int p = 0; p < NP; p++) {
-            double v, vx, vy;
-            far_poly<1, FIELD>(k2, x2[p], y2[p], v, vx, vy);
-            const double q = fma(C[p].v, h[p], k2[3]);  // Qe of n = 2: a constant
-            const double XY = X[p] * Y[p], t = s * F[p].ir;
-            F[p].S = fma(fma(t, So[p], fma(XY, q, fma(A[p].v, h[p], v))), h[p], 1.);
-            if (FIELD) {
-                const double qw = fma(C[p].w, h[p], 3. * k2[3]), qx = C[p].x * h[p], qy = C[p].y * h[p];
-                const double pw = fma(A[p].w, h[p], 3. * v), px = fma(A[p].x, h[p], vx), py = fma(A[p].y, h[p], vy);
-                const double W = fma(t, Wo[p], fma(XY, qw, pw));
-                // d/dX: 2X Pe_x + Y (Qe + 2 x2 Qe_x) + t (Po + 2 x2 Po_x + 2 XY Qo_x), d/dY alike
-                const double ex = fma(2. * X[p], px, Y[p] * fma(2. * x2[p], qx, q));
-                const double ey = fma(2. * Y[p], py, X[p] * fma(2. * y2[p], qy, q));
-                F[p].c1 = h[p] * fma(t, ox[p], ex);
-                F[p].c2 = h[p] * fma(t, oy[p], ey);
-                F[p].cd = fma(X[p], F[p].c1, fma(Y[p], F[p].c2, fma(W, h[p], 1.)));
-            }
+    for (int p = 0; p < NP; p++) {
+        double v, vx, vy;
+        far_poly<1, FIELD>(k2, x2[p], y2[p], v, vx, vy);
+        const double q = fma(C[p].v, h[p], k2[3]);  // Qe of n = 2: a constant
+        // t^2 (even + t (odd + t^2 tail)): the tail starts at t^5
+        const double XY = X[p] * Y[p], th = t[p] * h[p];
+        const double h1 = h[p];
+        F[p].S = fma(fma(t[p], fma(h1, (double) Sf[p], So[p]), fma(XY, q, fma(A[p].v, h1, v))), h1, 1.);
+        if (FIELD) {
+            const double qw = fma(C[p].w, h1, 3. * k2[3]), qx = C[p].x * h1, qy = C[p].y * h1;
+            const double pw = fma(A[p].w, h1, 3. * v), px = fma(A[p].x, h1, vx), py = fma(A[p].y, h1, vy);
+            const double W = fma(t[p], fma(h1, (double) Wf[p], Wo[p]), fma(XY, qw, pw));
+            // d/dX: 2X Pe_x + Y (Qe + 2 x2 Qe_x) + t (Po + 2 x2 Po_x + 2 XY Qo_x), d/dY alike
+            const double ex = fma(2. * X[p], px, Y[p] * fma(2. * x2[p], qx, q));
+            const double ey = fma(2. * Y[p], py, X[p] * fma(2. * y2[p], qy, q));
+            F[p].c1 = fma(th, fma(h1, (double) Gx[p], ox[p]), h1 * ex);
+            F[p].c2 = fma(th, fma(h1, (double) Gy[p], oy[p]), h1 * ey);
+            F[p].cd = fma(X[p], F[p].c1, fma(Y[p], F[p].c2, fma(W, h1, 1.)));
         }
     }
 }
@@ -579,7 +611,7 @@ __device__ __forceinline__ void far_pairs(const double* f, const V3 (&P)[NP], V3
 #pragma unroll
     for (int p = 0; p < NP; p++) {
         d[p] = v3(P[p].x - hd[fCen], P[p].y - hd[fCen + 1], P[p].z - hd[fCen + 2]);
-        F[p].ir = 0.5 * irsq<FAST>(dot(d[p], d[p]));
+        F[p].ir = kPotScale<FAST> * irsq<FAST>(dot(d[p], d[p]));
         X[p] = F[p].ir * dot(d[p], e1);
         Y[p] = F[p].ir * dot(d[p], e2);
     }

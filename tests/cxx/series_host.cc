@@ -24,6 +24,7 @@ inline double dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 inline double norm(V3 a) { return std::sqrt(dot(a, a)); }
 inline V3 ld3(const double* p) { return v3(p[0], p[1], p[2]); }
 template<bool FAST> double irsq(double x) { return 2. / std::sqrt(x); }
+template<bool FAST> constexpr double kPotScale = 0.5;
 struct float4 { float x, y, z, w; };
 struct double2 { double x, y; };
 struct int2 { int x, y; };
@@ -32,6 +33,7 @@ struct Dim { int x; };
 static Dim blockIdx, blockDim{1}, threadIdx;
 }  // namespace kemcu
 using std::fma;
+using std::fmaf;
 using std::pow;
 using std::sqrt;
 using std::cos;
