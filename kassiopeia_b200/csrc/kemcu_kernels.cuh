@@ -706,6 +706,26 @@ __global__ void __launch_bounds__(kFewElems) field_few_kernel(const double* __re
     }
 }
 
+// the element blocks' sums of a few points added in order, and whether all are finite: one launch
+// instead of reduce_splits, a clear and finite_kernel; flag[0] = 1 for a result that is not finite
+__global__ void field_few_sum_kernel(const double* __restrict__ partial, int nsplit, int m, double* __restrict__ out,
+                                     int* __restrict__ flag)
+{
+    const int i = threadIdx.x;  // one warp: m <= 4 kFewPoints
+    static_assert(4 * kFewPoints <= 32, "one warp holds the values of a few points");
+    Kahan k;
+    if (i < m) {
+        for (int s = 0; s < nsplit; s++)
+            k.add(partial[(size_t) s * m + i]);
+        out[i] = k.s;
+    }
+    const bool bad = __any_sync(0xffffffffu, i < m && !isfinite(k.s));
+    if (i == 0) {
+        flag[0] = bad;
+        flag[1] = 0;
+    }
+}
+
 // fixed-order sum of gridDim.y partial results: out[i] = sum_s partial[s][i]
 __global__ void reduce_splits(const double* __restrict__ partial, int nsplit, size_t n, double* __restrict__ out)
 {

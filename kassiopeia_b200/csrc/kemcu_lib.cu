@@ -83,6 +83,7 @@ struct kemcu_ctx
     double* d_near_val = nullptr;
     // grow-only scratch
     DevBuf scratch[16];
+    void* h_stage = nullptr;  // pinned host memory for the copies of small calls (kStageBytes)
     unsigned* d_counter = nullptr;
     int* d_flag = nullptr;
     double* noalloc_scratch = nullptr;  // device address of g_noalloc_scratch on this context's device
@@ -559,21 +560,10 @@ void few_form(dim3 grid, cudaStream_t st, int what, const kemcu_ctx* ctx, const 
         field_few_kernel<MIXED, true, true, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, np, part);
 }
 
-void launch_few(kemcu_ctx* ctx, const double* pts, int np, int precision, int what, int split, double* part)
-{
-    const dim3 grid((unsigned) np, (unsigned) split);
-    if (precision == KEMCU_FP32)
-        few_form<false, true>(grid, ctx->stream, what, ctx, pts, np, part);
-    else if (precision == KEMCU_MIXED)
-        few_form<true, false>(grid, ctx->stream, what, ctx, pts, np, part);
-    else
-        few_form<false, false>(grid, ctx->stream, what, ctx, pts, np, part);
-}
-
 // the planar direct sum at device points (d_out n x 4): K1, split `split` ways over the element
 // list (partial sums in `partial`, then reduced in split order)
 int launch_planar_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d_out, int precision, int what,
-                        int split, double* partial, bool few = false)
+                        int split, double* partial)
 {
     dim3 grid((unsigned) ((n + kPair * kThreads - 1) / (kPair * kThreads)), (unsigned) split);
     if (int rc = clear_pipe_flag(ctx))
@@ -585,13 +575,6 @@ int launch_planar_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d
     double* part = split > 1 ? partial : nullptr;
     int* fl = ctx->d_flag + 1;
     cudaStream_t st = ctx->stream;
-    if (few) {
-        launch_few(ctx, d_pts, np, precision, what, split, partial);
-        KCHECK_LAUNCH();
-        reduce_splits<<<1, 4 * kFewPoints, 0, st>>>(partial, split, (size_t) n * 4, d_out);
-        KCHECK_LAUNCH();
-        return KEMCU_OK;
-    }
     const int v = choose_variant(ctx, n, precision, what);
     const bool timed = ctx->pending_key >= 0 || ctx->time_k1;
     if (timed)
@@ -639,21 +622,20 @@ int launch_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d_out, i
 {
     if (ctx->axisym)
         return launch_axisym_field(ctx, d_pts, n, d_out, what);
-    // a handful of points: a CTA per point and kFewElems elements (grids of at most 65,535 element blocks)
-    const size_t eb = (ctx->n + kFewElems - 1) / kFewElems;
-    const bool few = n <= (size_t) kFewPoints && eb <= 65535;
-    const int split = few ? (int) eb : grid_split(ctx, n);
+    const int split = grid_split(ctx, n);
     double* partial = nullptr;
-    if (split > 1 || few) {
+    if (split > 1) {
         void* p;
         int rc = ensure(ctx, sPartial, (size_t) split * n * 4 * sizeof(double), &p);
         if (rc)
             return rc;
         partial = (double*) p;
     }
-    return launch_planar_field(ctx, d_pts, n, d_out, precision, what, split, partial, few);
+    return launch_planar_field(ctx, d_pts, n, d_out, precision, what, split, partial);
 }
 
+// bytes of the context's pinned staging memory: the points, results and flags of a few points
+constexpr size_t kStageBytes = 4096;
 constexpr size_t kSortMin = 4096;  // below this the point set is evaluated in caller order
 
 int check_finite(kemcu_ctx* ctx, const double* d, size_t m, const char* what)
@@ -668,6 +650,67 @@ int check_finite(kemcu_ctx* ctx, const double* d, size_t m, const char* what)
         return fail(ctx, KEMCU_ETIMEOUT, "element pipeline wait timed out while computing the %s", what);
     if (flag[0])
         return fail(ctx, KEMCU_ENONFINITE, "%s contains NaN or Inf", what);
+    return KEMCU_OK;
+}
+
+// A handful of points (field_few_kernel), planar elements. The points come from device memory dP or
+// host memory P, the results go to dout or, from host memory, to out. One wait for the GPU, on copies
+// through pinned memory: a probe's time is launches, copies and waits (99.6 us for one point of a
+// 1,280-triangle sphere with K1, two memsets, four kernels and three waits).
+bool few_points(const kemcu_ctx* ctx, size_t n)
+{
+    // (the tuner's forced shapes are K1's)
+    return !ctx->axisym && n <= (size_t) kFewPoints && ctx->force_variant < 0 &&
+           (ctx->n + kFewElems - 1) / kFewElems <= 65535;
+}
+
+int field_few(kemcu_ctx* ctx, const double* P, const double* dP, size_t n, double* out, double* dout, int precision,
+              int what)
+{
+    const int split = (int) ((ctx->n + kFewElems - 1) / kFewElems), m = 4 * (int) n;
+    void* base;
+    const size_t bytes = (4 + 3) * kFewPoints * sizeof(double) + 2 * sizeof(int);
+    static_assert((4 + 3) * kFewPoints * sizeof(double) + 2 * sizeof(int) <= kStageBytes, "staging of a few points");
+    if (int rc = ensure(ctx, sPartial, bytes + 64 + (size_t) split * m * sizeof(double), &base))
+        return rc;
+    // results | flags | points | partial sums
+    double* d_res = (double*) base;
+    int* d_fl = (int*) (d_res + 4 * kFewPoints);
+    double* d_pts = d_res + 4 * kFewPoints + 1;
+    double* d_part = (double*) ((char*) base + ((bytes + 63) & ~(size_t) 63));
+    double* h = (double*) ctx->h_stage;
+    cudaStream_t st = ctx->stream;
+    if (P) {
+        std::memcpy(h, P, n * 3 * sizeof(double));
+        KC(cudaMemcpyAsync(d_pts, h, n * 3 * sizeof(double), cudaMemcpyHostToDevice, st));
+    }
+    KC(cudaEventRecord(ctx->ev0, st));
+    const dim3 grid((unsigned) n, (unsigned) split);
+    const double* pts = P ? d_pts : dP;
+    if (precision == KEMCU_FP32)
+        few_form<false, true>(grid, st, what, ctx, pts, (int) n, d_part);
+    else if (precision == KEMCU_MIXED)
+        few_form<true, false>(grid, st, what, ctx, pts, (int) n, d_part);
+    else
+        few_form<false, false>(grid, st, what, ctx, pts, (int) n, d_part);
+    KCHECK_LAUNCH();
+    field_few_sum_kernel<<<1, 32, 0, st>>>(d_part, split, m, out ? d_res : dout, d_fl);
+    KCHECK_LAUNCH();
+    KC(cudaEventRecord(ctx->ev1, st));
+    // results and flags lie together
+    const int* hf = (const int*) (h + 4 * kFewPoints);
+    if (out)
+        KC(cudaMemcpyAsync(h, d_res, 4 * kFewPoints * sizeof(double) + 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    else
+        KC(cudaMemcpyAsync((void*) hf, d_fl, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    KC(cudaStreamSynchronize(st));
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+    ctx->last_ms = ms;
+    if (hf[0])
+        return fail(ctx, KEMCU_ENONFINITE, "field result contains NaN or Inf");
+    if (out)
+        std::memcpy(out, h, m * sizeof(double));
     return KEMCU_OK;
 }
 
@@ -1261,6 +1304,7 @@ int kemcu_create(kemcu_ctx** out, const kemcu_config* cfg)
     KC(cudaEventCreate(&ctx->tv0));
     KC(cudaEventCreate(&ctx->tv1));
     ctx->autotune = cfg->autotune != 0;
+    KC(cudaMallocHost(&ctx->h_stage, kStageBytes));
     KC(cudaMalloc(&ctx->d_counter, 64 * sizeof(unsigned)));
     KC(cudaMemset(ctx->d_counter, 0, 64 * sizeof(unsigned)));
     // [0]: non-finite values seen; [1]: a direct-sum pipeline wait timed out
@@ -1372,6 +1416,7 @@ int kemcu_destroy(kemcu_ctx* ctx)
         cudaFree(ctx->d_where);
         cudaFree(ctx->d_rwg);
         cudaFree(ctx->d_rows);
+        cudaFreeHost(ctx->h_stage);
         cudaFree(ctx->d_counter);
         cudaFree(ctx->d_flag);
         fm_release(ctx);
@@ -1537,6 +1582,8 @@ int kemcu_field_dev(kemcu_ctx* ctx, const double* dP, size_t n, double* dout4, i
         what > 2)
         return fail(ctx, KEMCU_EINVAL, "invalid field arguments");
     KC(cudaSetDevice(ctx->device));
+    if (few_points(ctx, n))
+        return field_few(ctx, nullptr, dP, n, nullptr, dout4, precision, what);
     Timer t(ctx);
     if (n < kSortMin) {
         if ((rc = launch_field(ctx, dP, n, dout4, precision, what)))
@@ -1640,6 +1687,11 @@ int kemcu_field(kemcu_ctx* ctx, const double* P, size_t n, double* out4, int pre
     if (!P || !out4)
         return fail(ctx, KEMCU_EINVAL, "null point or output buffer");
     KC(cudaSetDevice(ctx->device));
+    if (few_points(ctx, n)) {
+        if (precision < KEMCU_FP64 || precision > KEMCU_FP32 || what < 0 || what > 2)
+            return fail(ctx, KEMCU_EINVAL, "invalid field arguments");
+        return field_few(ctx, P, nullptr, n, out4, nullptr, precision, what);
+    }
     void *dp, *dout;
     if ((rc = ensure(ctx, sPts, n * 3 * sizeof(double), &dp)) || (rc = ensure(ctx, sOut, n * 4 * sizeof(double), &dout)))
         return rc;
