@@ -40,7 +40,8 @@ def test_port_moments_equal_reference_fixture():
 
 def test_port_local_field_equals_reference_fixture():
     fx = golden.load("fftm")
-    k = 8.9875517873681764e9 if not ref.available() else ref.constant("one_over_four_pi_eps0")
+    # the fixture's constant (CODATA 2018, KConst epoch 2021), also where the reference library is not at hand
+    k = K.ONE_OVER_FOUR_PI_EPS0 if not ref.available() else ref.constant("one_over_four_pi_eps0")
     got = fm_port.local_field(int(fx["l2p_degree"]), fx["l2p_origin"], fx["l2p_coeff"], fx["l2p_points"][:20], k)
     want = fx["l2p"][:20]
     scale = np.abs(want).max(axis=0)
