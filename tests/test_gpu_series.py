@@ -75,16 +75,20 @@ def test_operator_edges(n_elem):
     A, _ = port.PortProblem(m).matrix()
     rng = np.random.default_rng(3)
     finite = np.isfinite(A).all(1) & (np.arange(m.n) >= 0)
+    # a wire's potential on its own axis has logarithms of R - s with R^2 - s^2 = (diameter / 2)^2: eps
+    # (length / diameter)^2 of rounding in each of two, in this code and in the restatement alike
+    wire = m.shape == G.LINE_SEGMENT
+    own = np.where(wire, 2 * 2.2e-16 * (.3 / 1e-4) ** 2, 0.) * np.abs(np.diag(A))
     with K.CUDAElectrostaticContext(0) as ctx:
         ctx.SetGeometry(m)
         for nr in (1, 2, 8):
             x = rng.normal(size=(nr, m.n))
-            want, size = x @ A.T, np.abs(x) @ np.abs(A).T
+            want, size, extra = x @ A.T, np.abs(x) @ np.abs(A).T, np.abs(x) * own
             for prec, tol in TOL.items():
                 y = ctx.Multiply(x if nr > 1 else x[0], precision=prec).reshape(nr, -1)
-                assert np.all(np.abs(y - want)[:, finite] <= tol * size[:, finite]), (nr, prec)
+                assert np.all(np.abs(y - want)[:, finite] <= (tol * size + extra)[:, finite]), (nr, prec)
             y = ctx.Multiply(x if nr > 1 else x[0], assembled=True).reshape(nr, -1)
-            assert np.all(np.abs(y - want)[:, finite] <= TOL[K.FP64] * size[:, finite]), nr
+            assert np.all(np.abs(y - want)[:, finite] <= (TOL[K.FP64] * size + extra)[:, finite]), nr
 
 
 def test_degenerate_elements_keep_the_cubature():
