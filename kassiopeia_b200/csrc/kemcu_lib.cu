@@ -383,7 +383,8 @@ int build_far(kemcu_ctx* ctx)
     KC(cudaMalloc(&ctx->d_tiles, tiles.size() * sizeof(FarTile)));
     KC(cudaMalloc(&ctx->d_pre, n * sizeof(double)));
     KC(cudaMalloc(&ctx->d_where, n * sizeof(int2)));
-    KC(cudaMemcpy(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(FarTile), cudaMemcpyHostToDevice));
+    KC(cudaMemcpyAsync(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(FarTile),
+                       cudaMemcpyHostToDevice, ctx->stream));
     far_build_kernel<<<(unsigned) ((tiles.size() * kFarSym + 127) / 128), 128, 0, ctx->stream>>>(
         ctx->d_rec, ctx->d_tiles, ctx->ntiles, gl, ctx->d_far, ctx->d_pre, ctx->d_where);
     KCHECK_LAUNCH();
@@ -1525,9 +1526,10 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     KC(cudaMalloc(&ctx->d_rec, n * rRecSize * sizeof(double)));
     KC(cudaMalloc(&ctx->d_tgt, n * sizeof(TargetRec)));
     KC(cudaMalloc(&ctx->d_sigma, n * sizeof(double)));
-    KC(cudaMemcpy(ctx->d_rec, ctx->h_rec.data(), n * rRecSize * sizeof(double), cudaMemcpyHostToDevice));
-    KC(cudaMemcpy(ctx->d_tgt, ctx->h_tgt.data(), n * sizeof(TargetRec), cudaMemcpyHostToDevice));
-    KC(cudaMemset(ctx->d_sigma, 0, n * sizeof(double)));
+    KC(cudaMemcpyAsync(ctx->d_rec, ctx->h_rec.data(), n * rRecSize * sizeof(double),
+                       cudaMemcpyHostToDevice, ctx->stream));
+    KC(cudaMemcpyAsync(ctx->d_tgt, ctx->h_tgt.data(), n * sizeof(TargetRec), cudaMemcpyHostToDevice, ctx->stream));
+    KC(cudaMemsetAsync(ctx->d_sigma, 0, n * sizeof(double), ctx->stream));
     ctx->n = n;
     if (!ctx->axisym) {
         int rc = build_far(ctx);
@@ -1538,6 +1540,9 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
             return rc;
         }
     }
+    // the records are in place for whichever stream the next call runs on; the copies above are ordered on
+    // this stream because a copy from pageable memory may return before it has arrived
+    KC(cudaStreamSynchronize(ctx->stream));
     return KEMCU_OK;
 }
 
