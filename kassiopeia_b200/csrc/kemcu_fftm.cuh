@@ -89,7 +89,7 @@ __global__ void fm_p2m_kernel(const double* __restrict__ rec, const double* __re
             // sectoral R_m^m = prod_k (-sqrt((2k-1)/(2k))) (x + i y)
             double sr = 1., si = 0.;
             for (int q = 1; q <= m; q++) {
-                const double c = -sqrt((2. * q - 1.) / (2. * q));
+                const double c = -c_rt[2 * q - 1] * c_irt[2 * q];
                 const double tr = c * (ux * sr - uy * si), ti = c * (ux * si + uy * sr);
                 sr = tr;
                 si = ti;
@@ -101,14 +101,14 @@ __global__ void fm_p2m_kernel(const double* __restrict__ rec, const double* __re
             for (int nn = m + 1; nn <= p; nn++) {
                 double nr, ni;
                 if (nn == m + 1) {
-                    const double c = sqrt(2. * m + 1.) * uz;
+                    const double c = c_rt[2 * m + 1] * uz;
                     nr = c * r1r;
                     ni = c * r1i;
                 }
                 else {
-                    const double inv = 1. / sqrt((double) (nn - m) * (nn + m));
+                    const double inv = c_irt[nn - m] * c_irt[nn + m];
                     const double c1 = (2. * nn - 1.) * uz * inv;
-                    const double c2 = sqrt((double) (nn + m - 1) * (nn - m - 1)) * r2 * inv;
+                    const double c2 = c_rt[nn + m - 1] * c_rt[nn - m - 1] * r2 * inv;
                     nr = c1 * r1r - c2 * r0r;
                     ni = c1 * r1i - c2 * r0i;
                 }
@@ -747,13 +747,12 @@ __device__ __forceinline__ void fm_l2p(const double* Lh, int p, double ux, doubl
 // KFMElectrostaticFastMultipoleFieldSolver.cc:107-133), compensated (Kahan) like the direct
 // sum. ANALYTIC evaluates every direct pair with the analytic integrals (as the reference's
 // FFTM field solver does, KEBIFactory::MakeAnalytic()), else with the numeric policy.
-
 //
-// Register budget: the analytic integrals (rwg64) take up to 255 registers unbounded, which left
-// two CTAs per SM; bounded for 4 resident CTAs they spill a little and the kernel runs 18 %
-// faster (coax, 10^6 points, degree 8: 24.8 ms at depth 5, 17.6 ms at depth 6, against 30.2 and
-// 22.3; 3 and 5 CTAs measured 25.5 / 18.8 and 25.8 / 17.2 ms; results bit-identical).
-constexpr int kFmEvalMinBlocks = 4, kFmMatvecMinBlocks = 5;
+// Resident CTAs the registers are bounded for: the chains of the analytic integrals leave the FP64 pipe
+// idle, and more warps fill it better than the spills cost. Coax, 80,000 elements, 10^6 points, degree 8,
+// depth 6, ms per field and potential: 3 CTAs 9.28, 4 8.26, 5 7.80, 6 7.43, 7 7.29; the matrix product (kFmMatvecMinBlocks)
+// 5 CTAs 1.05, 6 1.06, 8 1.10 ms.
+constexpr int kFmEvalMinBlocks = 7, kFmMatvecMinBlocks = 5;
 
 template<bool POT, bool FIELD, bool ANALYTIC>
 __global__ void __launch_bounds__(128, kFmEvalMinBlocks) fm_eval_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
