@@ -360,6 +360,71 @@ __device__ __forceinline__ Out4 cubq_pairs(const double* e, V3 d, double R2)
     return o;
 }
 
+// cubq_pairs for the rectangles' 33-node rule from a table in shared memory (PairTable), two pairs
+// unrolled: the same sums in the same order. Unrolled, the rule is ~400 instructions that a warp runs through
+// once per element, and a kernel whose warps are at different elements of a mixed mesh then waits for
+// instructions (5 of 16 warps at any time on a product over 12,896 elements). The reads of the table, the
+// same for all lanes, take four shared-memory loads a pair of nodes. With it, and with the near list worked off
+// in one place of each kernel, that product (coaxial rectangles and triangles) went from 5.14 to 4.37 ms, and the one
+// over 28,800 triangles stayed at 21.4 ms. A triangle's nodes come singly and would
+// take as many loads for half the arithmetic: from the table, the product over 28,800 triangles took 26.6
+// instead of 21.3 ms, so their rule stays unrolled.
+struct PairTable
+{
+    double c[16 * kQ];
+};
+__device__ __forceinline__ void load_rules(PairTable& t)  // the whole CTA; a barrier before the first use
+{
+    for (int i = threadIdx.x; i < 16 * kQ; i += blockDim.x)
+        t.c[i] = c_qp[kQ * kPair33 + i];
+}
+template<bool POT, bool FIELD, bool FAST>
+__device__ __forceinline__ Out4 cubq_pairs_table(const PairTable& T, const double* e, V3 d, double R2)
+{
+    const V3 a = ld3(e + rEa), b = ld3(e + rEb);
+    const double C1 = dot(d, a), C2 = dot(d, b);
+    const double aa = e[rAA], ab2 = e[rAB2], bb = e[rBB];
+    const double ir = irsq<FAST>(R2);
+    double sp = c_qc[1] * ir, s0 = c_qc[1] * (ir * ir * ir), ss = 0., st = 0.;
+#pragma unroll 1
+    for (int g = 0; g < 16; g += 2) {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            double c[kQ];
+#pragma unroll
+            for (int i = 0; i < kQ; i += 2) {
+                const double2 v = *reinterpret_cast<const double2*>(T.c + (g + k) * kQ + i);
+                c[i] = v.x, c[i + 1] = v.y;
+            }
+            const double L = fma(c[1], C2, c[0] * C1);
+            double Q = fma(c[2], aa, R2);
+            Q = fma(c[3], ab2, Q);
+            Q = fma(c[4], bb, Q);
+            const double irp = irsq<FAST>(Q + L), irm = irsq<FAST>(Q - L);
+            if (POT)
+                sp = fma(c[5], irp + irm, sp);
+            if (FIELD) {
+                const double i3p = irp * irp * irp, i3m = irm * irm * irm;
+                s0 = fma(c[5], i3p + i3m, s0);
+                const double dd = i3p - i3m;
+                ss = fma(c[6], dd, ss);
+                st = fma(c[7], dd, st);
+            }
+        }
+    }
+    const double pf = e[rPrefac];
+    Out4 o{0., 0., 0., 0.};
+    if (POT)
+        o.phi = (kPotScale<FAST> * pf) * sp;
+    if (FIELD) {
+        const double pff = kFieldScale<FAST> * pf;
+        o.ex = pff * (d.x * s0 - a.x * ss - b.x * st);
+        o.ey = pff * (d.y * s0 - a.y * ss - b.y * st);
+        o.ez = pff * (d.z * s0 - a.z * ss - b.z * st);
+    }
+    return o;
+}
+
 // ------------------------------------------------------------------------- FP32 far field
 // The FP32 form of the cubature bands (precision KEMCU_FP32): the per-element set-up stays FP64
 // (d = P - centroid, R^2 from the band test, R^-1 to an ulp), and every node works on the
@@ -944,6 +1009,22 @@ __device__ __noinline__ Out4 epi(const double* __restrict__ e, const double* __r
             return line_analytic<POT, FIELD>(e, P);
         return type == kTriangle ? rwg_call<3, POT, FIELD>(e, w, P) : rwg_call<4, POT, FIELD>(e, w, P);
     }
+    return epi_far<MIXED, POT, FIELD, F32>(e, P, d, r2, band);
+}
+// the same with the rectangles' largest rule from a table in shared memory
+template<bool MIXED, bool POT, bool FIELD, bool F32 = false>
+__device__ __noinline__ Out4 epi(const PairTable& T, const double* __restrict__ e, const double* __restrict__ w, V3 P)
+{
+    V3 d;
+    double r2;
+    const int band = band_of(e, P, d, r2), type = (int) e[rType];
+    if (band == 0) {
+        if (type == kLineSegment)
+            return line_analytic<POT, FIELD>(e, P);
+        return type == kTriangle ? rwg_call<3, POT, FIELD>(e, w, P) : rwg_call<4, POT, FIELD>(e, w, P);
+    }
+    if (!F32 && band == 1 && type == kRectangle)
+        return cubq_pairs_table<POT, FIELD, MIXED>(T, e, d, r2);
     return epi_far<MIXED, POT, FIELD, F32>(e, P, d, r2, band);
 }
 

@@ -2,15 +2,15 @@
 // boundary-integral matvec (K2), operator assembly and the dense (assembled) matvec.
 //
 // Layout: one thread owns one evaluation point (a field point, or a target centroid for the
-// matvec); a CTA of kThreads points streams its slice of the element records (256 B each)
-// through a ring of shared-memory stages filled by bulk copies (ElementRing), and every
-// thread sums the contributions with Kahan compensation, as the reference's
-// KIntegratingFieldSolver does (KElectrostaticIntegratingFieldSolver.hh:261-339); the direct
-// sum adds the 32 contributions of a tile in plain FP64 first and compensates across tiles
-// (16 fewer FP64 operations per element, differences at the 1e-15 level). When there
-// are too few points to fill the GPU the element list is split over gridDim.y; each split
-// writes a partial sum to scratch and reduce_splits adds the splits in a fixed order, so the
-// result does not depend on scheduling.
+// matvec); a CTA of kThreads points streams its slice of the elements' far records (kemcu_series.cuh)
+// through a ring of shared-memory stages filled by bulk copies (FarRing). Distant pairs take the
+// far-field series there; the elements near some point of a warp go to the warp's list (NearList), which is
+// worked off with the cubature rules and the analytic integrals. Every thread sums its contributions with
+// Kahan compensation, as the reference's KIntegratingFieldSolver does
+// (KElectrostaticIntegratingFieldSolver.hh:261-339); the direct sum adds the contributions of a tile of up
+// to 16 elements in plain FP64 first and compensates across tiles. When there are too few points to fill the
+// GPU the element list is split over gridDim.y; each split writes a partial sum to scratch and reduce_splits
+// adds the splits in a fixed order, so the result does not depend on scheduling.
 #pragma once
 
 #include "kemcu_device.cuh"
@@ -48,34 +48,18 @@ struct Kahan
     }
 };
 
-// cooperative copy of `count` element records (256 B each) into shared memory (tracker)
-__device__ __forceinline__ void load_tile(double* sm, const double* __restrict__ rec, int first, int count)
-{
-    const double2* src = reinterpret_cast<const double2*>(rec + (size_t) first * rRecSize);
-    double2* dst = reinterpret_cast<double2*>(sm);
-    const int n2 = count * (rRecSize / 2);
-    for (int i = threadIdx.x; i < n2; i += blockDim.x)
-        dst[i] = __ldg(src + i);
-}
-
 // ------------------------------------------------------------------------- element pipeline
-// K1 streams element records through a ring of kPipe shared-memory stages of kFieldTile
-// records each. A stage is filled by one bulk copy (cp.async.bulk, completion counted on the
-// stage's mbarrier together with the 32 arrivals of the filling warp, whose lanes also store
-// the tile's charge densities). Warps consume stages at their own pace; each warp counts its
-// release of a stage in a shared counter, and the warp that releases it last refills it with
-// the tile kPipe ahead. A warp therefore waits only for data, never for the other warps
-// (which a __syncthreads per tile would impose), so warps that meet near-field elements and
-// warps that meet far-field ones drift apart by up to kPipe - 1 tiles.
-#ifndef KEMCU_FIELD_TILE
-#define KEMCU_FIELD_TILE 32
-#endif
+// The far records come through a ring of kPipe shared-memory stages of one tile each. A stage is filled by
+// one bulk copy (cp.async.bulk, completion counted on the stage's mbarrier together with the 32 arrivals of the
+// filling warp, whose lanes also store the tile's charge densities). Warps consume stages at their own pace;
+// each warp counts its release of a stage in a shared counter, and the warp that releases it last refills it
+// with the tile kPipe ahead. A warp therefore waits only for data, never for the other warps (which a
+// __syncthreads per tile would impose), so warps that work off a near list and warps that do not drift apart by
+// up to kPipe - 1 tiles.
 #ifndef KEMCU_PIPE
 #define KEMCU_PIPE 3
 #endif
-constexpr int kFieldTile = KEMCU_FIELD_TILE;
 constexpr int kPipe = KEMCU_PIPE;
-static_assert(kFieldTile <= 32 && kFieldTile % 2 == 0, "one lane of the filling warp per element");
 
 __device__ __forceinline__ unsigned smem_u32(const void* p)
 {
@@ -132,7 +116,7 @@ __device__ __forceinline__ bool mbar_wait_limit(unsigned long long* bar, unsigne
 
 // Self-test of the timeout path: one warp waits on an mbarrier phase that completes only when
 // `complete` is set (one arrival of the expected one); otherwise the wait gives up after
-// `limit` cycles and the kernel reports it in flag (|= 2), as the element ring does.
+// `limit` cycles and the kernel reports it in flag (|= 2), as the ring does.
 __global__ void wait_timeout_selftest_kernel(int* __restrict__ flag, long long limit, int complete)
 {
     __shared__ __align__(8) unsigned long long bar;
@@ -160,122 +144,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
                  : "memory");
 }
 
-// element slice [e0, e1) of [first, last) for split blockIdx.y, in whole tiles
-__device__ __forceinline__ void split_range(int first, int last, int& e0, int& e1)
-{
-    const int span = last - first;
-    const int per = ((span + (int) gridDim.y - 1) / (int) gridDim.y + kFieldTile - 1) / kFieldTile * kFieldTile;
-    e0 = min(last, first + (int) blockIdx.y * per);
-    e1 = min(last, e0 + per);
-}
-
-// The ring: NP stages (kPipe by default) of kFieldTile element records plus SIDE doubles of
-// per-element side data (charge densities, matvec operands) per element, stored by the filling
-// warp's lanes. RingStorage lives in shared memory; ElementRing (registers) holds the CTA's
-// element slice and a reference to it. A CYCLIC ring passes over the slice again and again
-// (the tracker's stage evaluations) and keeps prefetching until finish().
-template<int SIDE, int NP = kPipe> struct RingStorage
-{
-    double rec[NP][kFieldTile * rRecSize];
-    double side[NP][SIDE > 0 ? SIDE : 1][kFieldTile];
-    unsigned long long full[NP];
-    unsigned rel[NP], used[NP];
-};
-
-template<int SIDE, int NP = kPipe, bool CYCLIC = false> struct ElementRing
-{
-    RingStorage<SIDE, NP>& S;
-    int e0, e1;  // this CTA's element slice
-
-    __device__ __forceinline__ ElementRing(RingStorage<SIDE, NP>& storage, int first, int last) : S(storage)
-    {
-        split_range(first, last, e0, e1);
-        if (threadIdx.x < NP) {
-            mbar_init(&S.full[threadIdx.x], 32);
-            S.rel[threadIdx.x] = 0u;
-            S.used[threadIdx.x] = 0u;
-            mbar_init_fence();
-        }
-        __syncthreads();
-    }
-    __device__ __forceinline__ int tiles() const
-    {
-        return (e1 - e0 + kFieldTile - 1) / kFieldTile;
-    }
-    // first element of tile i of the sequence (CYCLIC: the slice is passed over repeatedly)
-    __device__ __forceinline__ int first(int i) const
-    {
-        return e0 + (CYCLIC ? i % tiles() : i) * kFieldTile;
-    }
-    __device__ __forceinline__ int count(int i) const
-    {
-        return min(kFieldTile, e1 - first(i));
-    }
-    __device__ __forceinline__ const double* element(int i, int j) const
-    {
-        return S.rec[i % NP] + j * rRecSize;
-    }
-    __device__ __forceinline__ double side(int i, int k, int j) const
-    {
-        return S.side[i % NP][k][j];
-    }
-    // fill stage i % NP with tile i: called by all 32 lanes of one warp;
-    // side_fn(double (*side)[kFieldTile], int t0, int cnt, int lane) stores the side data
-    template<class F> __device__ __forceinline__ void fill(const double* __restrict__ src, int i, F side_fn)
-    {
-        const int s = i % NP, t0 = first(i), cnt = count(i), lane = threadIdx.x & 31;
-        side_fn(S.side[s], t0, cnt, lane);
-        if (lane == 0) {
-            S.used[s]++;
-            fence_proxy_async();
-            const unsigned bytes = (unsigned) (cnt * rRecSize * sizeof(double));
-            mbar_arrive_tx(&S.full[s], bytes);
-            bulk_g2s(S.rec[s], src + (size_t) t0 * rRecSize, bytes, &S.full[s]);
-        }
-        else
-            mbar_arrive(&S.full[s]);
-    }
-    template<class F> __device__ __forceinline__ void prologue(const double* __restrict__ src, F side_fn)
-    {
-        if (threadIdx.x < 32)
-            for (int i = 0; i < (CYCLIC ? NP : min(NP, tiles())); i++)
-                fill(src, i, side_fn);
-    }
-    __device__ __forceinline__ bool wait(int i)
-    {
-        return mbar_wait(&S.full[i % NP], (unsigned) (i / NP) & 1u);
-    }
-    // whole warp: release tile i; the warp that releases a stage last refills it
-    template<class F> __device__ __forceinline__ void release(const double* __restrict__ src, int i, F side_fn)
-    {
-        const int s = i % NP;
-        __syncwarp();
-        unsigned last = 0u;
-        if ((threadIdx.x & 31) == 0) {
-            __threadfence_block();
-            last = atomicAdd(&S.rel[s], 1u) % (blockDim.x >> 5) == (blockDim.x >> 5) - 1u;
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (last && (CYCLIC || i + NP < tiles())) {
-            __threadfence_block();
-            fill(src, i + NP, side_fn);
-        }
-    }
-    // after the tile loop (all threads): report a timed-out wait in flag (|= 2) and wait,
-    // bounded, for copies still in flight
-    __device__ __forceinline__ void finish(bool ok, int* flag)
-    {
-        if (!ok && (threadIdx.x & 31) == 0)
-            atomicOr(flag, 2);
-        __syncthreads();
-        if (threadIdx.x < NP && S.used[threadIdx.x] > 0u)
-            mbar_wait(&S.full[threadIdx.x], (S.used[threadIdx.x] - 1u) & 1u);
-    }
-};
-
-// The same ring over the far records (kemcu_series.cuh), tile by tile of the tile table: a stage
-// holds one tile's records, its descriptor and SIDE doubles of side data per element. The CTA's
-// slice is a range of tiles, split over gridDim.y.
+// The ring: NP stages of one tile of the tile table, its records, its descriptor and SIDE doubles of side
+// data per element (charge densities, matvec operands). FarRingStorage lives in shared memory; FarRing
+// (registers) holds the CTA's slice, a range of tiles split over gridDim.y.
 template<int SIDE, int NP> struct FarRingStorage
 {
     double rec[NP][kFarStage];
@@ -446,8 +317,9 @@ struct NearList
     }
 };
 
-// Points per lane of the pair kernels: two share every coefficient read from shared memory (the
-// loads were a quarter of the instructions with one) and give each other's chains room
+// Points per lane of the pair kernels. Two share every coefficient read from shared memory, but the field
+// kernels then spill (193 against 147 ms for 400,000 points of a coaxial pair), and so does the product (26.4
+// against 21.7 ms over 28,800 triangles).
 #ifndef KEMCU_PAIR
 #define KEMCU_PAIR 1
 #endif
@@ -764,6 +636,19 @@ __device__ __forceinline__ double entry(const double* e, const double* w, const 
     return t.diag;
 }
 
+// the same with the rectangles' largest rule from a table in shared memory
+template<bool MIXED, bool F32 = false>
+__device__ __forceinline__ double entry(const PairTable& T, const double* e, const double* w, const TargetRec& t, V3 C)
+{
+    if (t.neumann == 0.)
+        return epi<MIXED, true, false, F32>(T, e, w, C).phi;
+    if (norm(ld3(e + rCen2) - C) >= 1e-12) {
+        const Out4 r = epi<MIXED, false, true, F32>(T, e, w, C);
+        return r.ex * t.normal[0] + r.ey * t.normal[1] + r.ez * t.normal[2];
+    }
+    return t.diag;
+}
+
 // an entry whose pair is in a quadrature band (band_of returned band >= 1 with d, r2): the same
 // value as entry<MIXED>, without the analytic near-field code (a Neumann self term is band 0)
 template<bool MIXED>
@@ -821,6 +706,8 @@ __global__ void __launch_bounds__(kThreads, NR == 1 ? kMinBlocks : 4)
 {
     __shared__ __align__(128) FarRingStorage<NR + 1, kPipe> S;
     __shared__ NearStore s_near[kThreads / 32];
+    __shared__ __align__(16) PairTable s_rules;
+    load_rules(s_rules);  // the ring's constructor has the barrier
     const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
     const bool busy = base - (int) (threadIdx.x & 31) < n;
     int row[kPair];
@@ -854,8 +741,8 @@ __global__ void __launch_bounds__(kThreads, NR == 1 ? kMinBlocks : 4)
 #pragma unroll
             for (int p = 0; p < kPair; p++) {
                 const double* w = V.rwg + (size_t) e * wRecSize;
-                const double a = any_neumann ? entry<MIXED, F32>(er, w, tgt[row[p]], C[p])
-                                             : epi<MIXED, true, false, F32>(er, w, C[p]).phi;
+                const double a = any_neumann ? entry<MIXED, F32>(s_rules, er, w, tgt[row[p]], C[p])
+                                             : epi<MIXED, true, false, F32>(s_rules, er, w, C[p]).phi;
 #pragma unroll
                 for (int r = 0; r < NR; r++)
                     if (NR == 1 || r < nrhs)
@@ -879,14 +766,12 @@ __global__ void __launch_bounds__(kThreads, NR == 1 ? kMinBlocks : 4)
                                                if (NR == 1 || r < nrhs)
                                                    acc[r][p].add(a * sd[r][j]);
                                        });
-            if (L.full())
+            if (L.full() || (q == ntiles - 1 && L.n > 0))  // one place: its code is large
                 near();
         }
         R.release(q, side);
     }
     R.finish(ok, flag);
-    if (L.n > 0)
-        near();
 #pragma unroll
     for (int p = 0; p < kPair; p++)
         if (base + 32 * p < n)
@@ -911,6 +796,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 {
     __shared__ __align__(128) FarRingStorage<1, kPipe> S;
     __shared__ NearStore s_near[kThreads / 32];
+    __shared__ __align__(16) PairTable s_rules;
+    load_rules(s_rules);  // the ring's constructor has the barrier
     const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
     const bool busy = base - (int) (threadIdx.x & 31) < n;
     int row[kPair];
@@ -948,8 +835,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         L.drain(rec, [&](int e, const double* er) {
 #pragma unroll
             for (int p = 0; p < kPair; p++)
-                store(p, e, any_neumann ? entry<MIXED>(er, V.rwg + (size_t) e * wRecSize, tgt[row[p]], C[p])
-                                        : epi<MIXED, true, false>(er, V.rwg + (size_t) e * wRecSize, C[p]).phi);
+                store(p, e, any_neumann ? entry<MIXED>(s_rules, er, V.rwg + (size_t) e * wRecSize, tgt[row[p]], C[p])
+                                        : epi<MIXED, true, false>(s_rules, er, V.rwg + (size_t) e * wRecSize, C[p]).phi);
         });
     };
     bool ok = true;
@@ -962,14 +849,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
             const FarTile T = S.tile[q % kPipe];
             tile_entries<MIXED>(S.rec[q % kPipe], T, S.side[q % kPipe][0], tgt, row, C, any_neumann, wc, wr, L,
                                 [&](int p, int j, double a) { store(p, T.first + j, a); });
-            if (L.full())
+            if (L.full() || (q == ntiles - 1 && L.n > 0))  // one place: its code is large
                 near();
         }
         R.release(q, side);
     }
     R.finish(ok, flag);
-    if (L.n > 0)
-        near();
 }
 
 // dense matvec on the assembled column-major operator (leading dimension ld):

@@ -18,7 +18,8 @@
 // an FP32 one for one, so the cost of a pair is 2 x FP64 + the rest in issue cycles (measured within
 // 20 %: 250 cycles per 32 pairs for 67 FP64 and 81 other instructions). A 33-node pair of the rules
 // takes ~440 FP64 operations, a 12-node one ~190; the series of a symmetric element 54 to 88 and 45 to
-// 75 others. Two points per lane share the coefficient loads.
+// 75 others. (Two points per lane would share the coefficient loads, but take 131 to 168 registers and spill:
+// 193 instead of 147 ms for 400,000 points of a coaxial electrode pair.)
 //
 // Precision. FP64 form: n <= 4 in FP64, nearer elements also n = 5 (general) or 6 (symmetric); the
 // tail of higher orders is at most ~2e-9 of the term where it is used, so its FP32 rounding is 1e-16
