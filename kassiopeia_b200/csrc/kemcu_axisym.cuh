@@ -172,7 +172,7 @@ __device__ __forceinline__ RingGeom ring_at(double p, const AxPar& q)
 // c_n = (a_{n-1} - b_{n-1}) / 2 and c_1^2 / k^2 = k^2 / (16 a_1^2). Square roots and reciprocals are the
 // hardware estimates with one step of third order. It agrees with Cody's series to 1e-15 and takes
 // ~110 FP64 operations a node where the series, logarithm, square roots and divisions took ~260. The
-// field kernel is bound by them (FP64 pipe 61 %): 20,000 points and 4,416 elements 17.4 -> 8.2 ms.
+// field kernel is bound by them (FP64 pipe 61 %): 20,015 points and 1,776 elements 17.4 -> 8.2 ms.
 constexpr double kAxFast = 0.01;
 
 __device__ __forceinline__ double rcp_cubic(double x)
