@@ -56,12 +56,14 @@ enum kemcu_shape {
 enum kemcu_boundary { KEMCU_DIRICHLET = 0, KEMCU_NEUMANN = 1 };
 /* arithmetic form of the element integrals */
 enum kemcu_precision {
-    KEMCU_FP64 = 0,  /* every node in FP64: the plain form */
+    KEMCU_FP64 = 0,  /* every node in FP64: the plain form. Distant pairs are the rules' far-field
+                        series, whose FP32 tail and left-out orders are below 5e-16 of the pair */
     KEMCU_MIXED = 1, /* cubature nodes with the FP32-class hardware reciprocal square root
                         refined by one FP64 Newton step (~1e-13 relative); RWG / analytic
                         near field and the compensated accumulation as in FP64 */
-    KEMCU_FP32 = 2   /* far field in FP32: the cubature nodes of triangles and rectangles on
-                        FP32 FMAs and the FP32 hardware reciprocal square root, relative to the
+    KEMCU_FP32 = 2   /* far field in FP32: the cubature nodes of triangles and rectangles nearer
+                        than the far-field series (which is that of KEMCU_MIXED) on FP32 FMAs
+                        and the FP32 hardware reciprocal square root, relative to the
                         element's FP64 centre distance (~1e-7 relative per element); the RWG /
                         analytic near field, wires, the per-element set-up and the compensated
                         element sums in FP64. Field evaluation and matrix-free matvec only (the
@@ -177,7 +179,7 @@ int kemcu_field_dev_noalloc(kemcu_ctx* ctx, const double* dP, size_t n, double* 
 /* ---- autotuner of the direct sum's launch shape (no counterpart in the reference: the OpenCL
         plugin fixes its work-group size at build time, KOpenCLElectrostaticIntegratingFieldSolver.hh)
    The direct-sum kernel exists in kemcu_field_variant_count() launch shapes (resident CTAs per SM
-   its registers are bounded for, element-ring stages: kemcu_field_variant_info); all compute the
+   its registers are bounded for, ring stages: kemcu_field_variant_info); all compute the
    same operations in the same order, so every shape returns the same bits. Per context, precision
    and size class (the bit length of the point count) the library keeps the fastest shape: with
    kemcu_config.autotune set, the first field-and-potential calls of a class each run one shape
@@ -217,7 +219,8 @@ void kemcu_set_iteration_callback(kemcu_ctx* ctx, kemcu_iteration_callback cb, v
    b: n values or NULL for the boundary values; x: n values, in: initial guess (as the
    reference, A x is applied when |x|_inf > 1e-16), out: solution, also stored as the
    context's sigma. assembled != 0 reads the columns from the assembled FP64 operator (built
-   on first use), else computes them on the fly. Returns KEMCU_ENOTCONVERGED after
+   on first use), else computes them on the fly (a system of up to 4,096 rows keeps the computed
+   columns, at most 128 MB, for the length of the solve). Returns KEMCU_ENOTCONVERGED after
    max_subiterations (0 = unlimited) or when the iteration callback asks to stop (it is
    called after every residual check with the check count and the relative residual). */
 typedef struct {
