@@ -96,7 +96,7 @@ __constant__ float c_qc32[2];
 __constant__ double c_gl[10 * 2];
 __constant__ Constants c_k;
 // square roots of the integers and their reciprocals (harmonic recurrences of kemcu_fftm.cuh)
-constexpr int kNumRoots = 36;
+constexpr int kNumRoots = 61;
 __constant__ double c_rt[kNumRoots], c_irt[kNumRoots];
 
 // ------------------------------------------------------------------------- helpers

@@ -22,6 +22,10 @@
 namespace kemcu
 {
 constexpr int kFmMaxDegree = 15;  // P2M runs one lane per order m on half a warp
+// local expansions given by the caller (kemcu_fm_local_field); the recurrences of a degree p take the
+// roots of the integers up to 2p
+constexpr int kFmMaxLocalDegree = 30;
+static_assert(kNumRoots > 2 * kFmMaxLocalDegree && kNumRoots > 2 * kFmMaxDegree, "table of roots");
 constexpr int kFmMaxQ = 9;        // Gauss-Legendre points per direction: exact to degree 17
 
 __host__ __device__ __forceinline__ int fm_re(int n, int m)

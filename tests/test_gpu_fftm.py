@@ -10,7 +10,7 @@ import pytest
 
 import kassiopeia_b200 as K
 from kassiopeia_b200 import geometry as G
-from oracle import golden, ref_fm
+from oracle import fm_port, golden, ref_fm
 from oracle.golden import mesh_from
 
 pytestmark = pytest.mark.gpu
@@ -65,6 +65,27 @@ def test_local_field_equals_reference_fixture():
     got = ctx.LocalExpansionField(int(fx["l2p_degree"]), fx["l2p_origin"], fx["l2p_coeff"], fx["l2p_points"])
     want = fx["l2p"]
     assert np.all(np.abs(got - want).max(axis=0) <= 1e-13 * np.abs(want).max(axis=0))
+
+
+@pytest.mark.parametrize("degree", [0, 1, 15, 16, 17, 18, 25, 30])
+def test_local_field_at_every_accepted_degree(degree):
+    # beyond the trees' degrees, to the last one that is accepted
+    rng = np.random.default_rng(degree)
+    nm = [(n, m) for n in range(degree + 1) for m in range(n + 1)]
+    c = rng.normal(size=len(nm)) + 1j * rng.normal(size=len(nm)) * np.array([m > 0 for _, m in nm])
+    o, P, h = np.array([.1, -.2, .3]), rng.uniform(-.6, .6, (12, 3)), 1e-5
+    k = K.ONE_OVER_FOUR_PI_EPS0
+    want = fm_port.local_field(degree, o, c, P, k, h)
+    with K.CUDAElectrostaticContext(0) as ctx:
+        ctx.SetGeometry(G.icosphere(1))
+        got = ctx.LocalExpansionField(degree, o, c, P)
+    # |R_n^m| <= r^n, and a derivative takes another factor n / r; both sides' recurrences round by some n eps a
+    # term, the differences by eps S / h and h^2 / 6 of the third derivative
+    r, n = np.linalg.norm(P - o, axis=1)[:, None], np.array([n for n, _ in nm])
+    size = np.array([1. if m == 0 else 2. for _, m in nm]) * np.abs(c)
+    S, S1, S3 = (size * r ** n).sum(1), (size * n * r ** (n - 1.)).sum(1), (size * n ** 3. * r ** (n - 3.)).sum(1)
+    assert np.all(np.abs(got[:, 3] - want[:, 3]) <= 1e-12 * k * S)
+    assert np.all(np.abs(got[:, :3] - want[:, :3]).max(1) <= k * (1e-12 * S1 + 1e-13 * S / h + h * h / 6. * S3))
 
 
 @pytest.mark.parametrize("depth", [3, 4])
