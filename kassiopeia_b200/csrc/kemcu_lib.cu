@@ -1307,14 +1307,18 @@ int kemcu_create(kemcu_ctx** out, const kemcu_config* cfg)
     ctx->autotune = cfg->autotune != 0;
     KC(cudaMallocHost(&ctx->h_stage, kStageBytes));
     KC(cudaMalloc(&ctx->d_counter, 64 * sizeof(unsigned)));
-    KC(cudaMemset(ctx->d_counter, 0, 64 * sizeof(unsigned)));
+    KC(cudaMemsetAsync(ctx->d_counter, 0, 64 * sizeof(unsigned), ctx->stream));
     // [0]: non-finite values seen; [1]: a direct-sum pipeline wait timed out
     KC(cudaMalloc(&ctx->d_flag, 2 * sizeof(int)));
-    KC(cudaMemset(ctx->d_flag, 0, 2 * sizeof(int)));
+    KC(cudaMemsetAsync(ctx->d_flag, 0, 2 * sizeof(int), ctx->stream));
     // set-up of kemcu_field_dev_noalloc: the static scratch array's device address on this
     // device (host code may not use the symbol itself as a device pointer)
     KC(cudaGetSymbolAddress((void**) &ctx->noalloc_scratch, g_noalloc_scratch));
-    // rule tables
+    // rule tables. Copies go through the context's stream: from pageable memory a copy may return before it
+    // has arrived, and the kernels' stream does not wait for the default one
+    auto constant = [&](const auto& symbol, const void* src, size_t bytes) {
+        return cudaMemcpyToSymbolAsync(symbol, src, bytes, 0, cudaMemcpyHostToDevice, ctx->stream);
+    };
     std::vector<double> rules(kNumNodes * 3), gl(20), q(kNumNodes * kQ);
     tables::build(rules.data(), gl.data());
     for (int k = 0; k < kNumNodes; k++) {
@@ -1324,7 +1328,7 @@ int kemcu_create(kemcu_ctx** out, const kemcu_config* cfg)
         for (int c = 0; c < kQ; c++)
             q[kQ * k + c] = v[c];
     }
-    KC(cudaMemcpyToSymbol(c_q, q.data(), q.size() * sizeof(double)));
+    KC(constant(c_q, q.data(), q.size() * sizeof(double)));
     std::vector<double> qa(kNumNodes * kQA);
     for (int k = 0; k < kNumNodes; k++) {
         const double sc = k < kRect7 ? 1. / 3. : 0.5;
@@ -1333,7 +1337,7 @@ int kemcu_create(kemcu_ctx** out, const kemcu_config* cfg)
         for (int c = 0; c < kQA; c++)
             qa[kQA * k + c] = v[c];
     }
-    KC(cudaMemcpyToSymbol(c_qa, qa.data(), qa.size() * sizeof(double)));
+    KC(constant(c_qa, qa.data(), qa.size() * sizeof(double)));
     // pair form of the centrally symmetric rectangle rules
     std::vector<double> qp(kNumPairs * kQ, 0.);
     double qc[2] = {0., 0.};
@@ -1369,27 +1373,28 @@ int kemcu_create(kemcu_ctx** out, const kemcu_config* cfg)
         if (np != pair_n[r] || nc != (center[r] >= 0 ? 1 : 0))
             return fail(ctx, KEMCU_ECUDA, "rectangle rule %d: unexpected node pairing", rule_n[r]);
     }
-    KC(cudaMemcpyToSymbol(c_qp, qp.data(), qp.size() * sizeof(double)));
-    KC(cudaMemcpyToSymbol(c_qc, qc, sizeof qc));
+    KC(constant(c_qp, qp.data(), qp.size() * sizeof(double)));
+    KC(constant(c_qc, qc, sizeof qc));
     {
         std::vector<float> q32(q.begin(), q.end()), qp32(qp.begin(), qp.end());
         const float qc32[2] = {(float) qc[0], (float) qc[1]};
-        KC(cudaMemcpyToSymbol(c_q32, q32.data(), q32.size() * sizeof(float)));
-        KC(cudaMemcpyToSymbol(c_qp32, qp32.data(), qp32.size() * sizeof(float)));
-        KC(cudaMemcpyToSymbol(c_qc32, qc32, sizeof qc32));
+        KC(constant(c_q32, q32.data(), q32.size() * sizeof(float)));
+        KC(constant(c_qp32, qp32.data(), qp32.size() * sizeof(float)));
+        KC(constant(c_qc32, qc32, sizeof qc32));
     }
-    KC(cudaMemcpyToSymbol(c_gl, gl.data(), gl.size() * sizeof(double)));
-    KC(cudaMemcpyToSymbol(c_k, &ctx->k, sizeof(Constants)));
+    KC(constant(c_gl, gl.data(), gl.size() * sizeof(double)));
+    KC(constant(c_k, &ctx->k, sizeof(Constants)));
     double rt[kNumRoots], irt[kNumRoots];
     for (int i = 0; i < kNumRoots; i++) {
         rt[i] = std::sqrt((double) i);
         irt[i] = i ? 1. / std::sqrt((double) i) : 0.;
     }
-    KC(cudaMemcpyToSymbol(c_rt, rt, sizeof rt));
-    KC(cudaMemcpyToSymbol(c_irt, irt, sizeof irt));
+    KC(constant(c_rt, rt, sizeof rt));
+    KC(constant(c_irt, irt, sizeof irt));
     double rk[kStages][kStages];
     rk8_table(rk);
-    KC(cudaMemcpyToSymbol(c_rk8, rk, sizeof rk));
+    KC(constant(c_rk8, rk, sizeof rk));
+    KC(cudaStreamSynchronize(ctx->stream));
     return KEMCU_OK;
 }
 
@@ -1553,7 +1558,9 @@ int kemcu_set_sigma(kemcu_ctx* ctx, const double* sigma)
         return rc;
     if (!sigma)
         return fail(ctx, KEMCU_EINVAL, "null sigma");
-    KC(cudaMemcpy(ctx->d_sigma, sigma, ctx->n * sizeof(double), cudaMemcpyHostToDevice));
+    KC(cudaSetDevice(ctx->device));
+    KC(cudaMemcpyAsync(ctx->d_sigma, sigma, ctx->n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    KC(cudaStreamSynchronize(ctx->stream));
     ctx->have_sigma = true;
     return KEMCU_OK;
 }
@@ -1563,7 +1570,9 @@ int kemcu_get_sigma(kemcu_ctx* ctx, double* sigma)
     int rc = check_ready(ctx, true);
     if (rc)
         return rc;
-    KC(cudaMemcpy(sigma, ctx->d_sigma, ctx->n * sizeof(double), cudaMemcpyDeviceToHost));
+    KC(cudaSetDevice(ctx->device));
+    KC(cudaMemcpyAsync(sigma, ctx->d_sigma, ctx->n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    KC(cudaStreamSynchronize(ctx->stream));
     return KEMCU_OK;
 }
 
