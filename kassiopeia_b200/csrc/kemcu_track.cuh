@@ -8,9 +8,10 @@
 //   d/dt (t, s, x, p) = (1, |v|, v, q E(x)),  v = p / (m gamma),  gamma = sqrt(1 + p^2 / (m c)^2)
 // with E(x) the Kahan-summed direct sum of KIntegratingFieldSolver::ElectricField.
 //
-// Layout: a CTA owns 32 slots, one per lane, and W warps that share the elements: warp w sums
-// elements w, w + W, ... for all 32 slots, and warp 0 adds the warps' sums in order and advances the
-// slots. The element records come a warp at a time through its own piece of shared memory, the next
+// Layout: a CTA owns 32 slots, one per lane, and W warps that share the elements: part c of kTrackParts
+// is elements c, c + kTrackParts, ..., warp w sums parts w, w + W, ... one after another for all 32
+// slots, and warp 0 adds the parts' sums in order and advances the slots. The parts do not depend on W,
+// which follows the number of tracks. The element records come a warp at a time through its own piece of shared memory, the next
 // one's loads in flight during the pairs of this one, so a stage has no CTA barrier but the two around
 // it. (One thread per track left 4 warps on an SM at 16,384 tracks, waiting for FP64 latencies.) Slots
 // take tracks in Morton order of their positions, so that a warp's lanes agree on an element's form;
@@ -28,6 +29,7 @@ namespace kemcu
 {
 
 constexpr int kTrackSlots = 32;  // per CTA: a lane each
+constexpr int kTrackParts = 16;  // sums over the elements, the most warps of a CTA
 constexpr int kStages = 13;
 constexpr int kTrackK = 6;     // stored per stage and slot: v (3), q E (3)
 
@@ -135,6 +137,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems 
     __shared__ double s_k[kStages][kTrackK][kTrackSlots];
     __shared__ double s_x[3][kTrackSlots];
     __shared__ __align__(16) double s_far[W][kFarGenStride], s_rec[W][rRecSize];
+    // the parts' sums (a warp with one part leaves them where its records were)
+    static_assert(W <= kTrackParts && kTrackParts % W == 0 && kFarGenStride >= 3 * kTrackSlots, "parts of the sum");
+    __shared__ double s_part[W < kTrackParts ? kTrackParts : 1][3 * kTrackSlots];
+    auto part = [&](int c) { return W < kTrackParts ? s_part[c] : s_far[c]; };
     __shared__ int s_any;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int track = -1, tsteps = 0;
@@ -156,7 +162,6 @@ __global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems 
     // this warp's share of the field at the 32 slot positions
     auto field = [&]() {
         const V3 X = v3(s_x[0][lane], s_x[1][lane], s_x[2][lane]);
-        Kahan ex, ey, ez;
         constexpr int NV = (kFarGenStride + 31) / 32;
         double v[NV], r = 0., pre_next = 0., sg_next = 0.;
         int2 at = make_int2(0, 0);
@@ -174,28 +179,32 @@ __global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems 
         };
         if (warp < el.n)
             fetch(warp);
-        for (int j = warp; j < el.n; j += W) {
-            __syncwarp();
-            const bool general = at.y != 0;
-            const int len = general ? kFarGenStride : kFarSymStride;
+        for (int c = warp; c < kTrackParts; c += W) {
+            Kahan ex, ey, ez;
+            for (int j = c; j < el.n; j += kTrackParts) {
+                __syncwarp();
+                const bool general = at.y != 0;
+                const int len = general ? kFarGenStride : kFarSymStride;
 #pragma unroll
-            for (int k = 0; k < NV; k++)
-                if (lane + 32 * k < len)
-                    s_far[warp][lane + 32 * k] = v[k];
-            s_rec[warp][lane] = r;
+                for (int k = 0; k < NV; k++)
+                    if (lane + 32 * k < len)
+                        s_far[warp][lane + 32 * k] = v[k];
+                s_rec[warp][lane] = r;
+                __syncwarp();
+                const double pre = pre_next, sg = sg_next;
+                const int next = j + kTrackParts < el.n ? j + kTrackParts : c + W < kTrackParts ? c + W : el.n;
+                if (next < el.n)
+                    fetch(next);
+                const V3 E = track_pair<MIXED>(s_far[warp], general, s_rec[warp], el.V.rwg + (size_t) j * wRecSize, pre, X);
+                ex.add(E.x * sg);
+                ey.add(E.y * sg);
+                ez.add(E.z * sg);
+            }
             __syncwarp();
-            const double pre = pre_next, sg = sg_next;
-            if (j + W < el.n)
-                fetch(j + W);
-            const V3 E = track_pair<MIXED>(s_far[warp], general, s_rec[warp], el.V.rwg + (size_t) j * wRecSize, pre, X);
-            ex.add(E.x * sg);
-            ey.add(E.y * sg);
-            ez.add(E.z * sg);
+            part(c)[lane] = ex.s;
+            part(c)[kTrackSlots + lane] = ey.s;
+            part(c)[2 * kTrackSlots + lane] = ez.s;
         }
-        __syncwarp();  // the record's piece now takes the warp's sums
-        s_far[warp][lane] = ex.s;
-        s_far[warp][32 + lane] = ey.s;
-        s_far[warp][64 + lane] = ez.s;
     };
     if (warp == 0)
         pull();
@@ -254,10 +263,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems 
             __syncthreads();
             if (warp == 0) {
                 Kahan ex, ey, ez;
-                for (int w = 0; w < W; w++) {
-                    ex.add(s_far[w][lane]);
-                    ey.add(s_far[w][32 + lane]);
-                    ez.add(s_far[w][64 + lane]);
+                for (int c = 0; c < kTrackParts; c++) {
+                    ex.add(part(c)[lane]);
+                    ey.add(part(c)[kTrackSlots + lane]);
+                    ez.add(part(c)[2 * kTrackSlots + lane]);
                 }
                 const double p2 = dot(Pm, Pm);
                 const double gam = sqrt(1. + p2 / (prm.mass * prm.mass * prm.c2));
