@@ -7,6 +7,7 @@ import pytest
 
 import kassiopeia_b200 as K
 from kassiopeia_b200 import geometry as G
+from oracle import golden
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +38,49 @@ def test_budget_too_small_for_the_operator_keeps_columns_on_the_fly():
         ctx.SetGeometry(m)
         x, _ = ctx.SolveRobinHood(b, tol=1e-7)
         assert np.max(np.abs(b - ctx.Multiply(x))) <= 2e-7
+
+
+@pytest.mark.parametrize("name", ["icosphere_L2", "mixed_small", "c1_sphere"])
+def test_columns_on_the_fly_match_the_reference(name):
+    # no room for kept columns: one CTA, or (1,280 rows) a cluster, computes every column (near list and cubature
+    # bands; mixed_small has Neumann rows and wires); the reference's number of checks, and its solution
+    tol = 1e-8
+    fx = golden.load(name)
+    if name == "c1_sphere":
+        m, checks, sigma, direct = G.icosphere(3), fx["robinhood_iterations"], fx["robinhood_sigma"], fx["sigma_direct"]
+    else:
+        rh = golden.load("robinhood")
+        m, checks, sigma = golden.mesh_from(fx), rh[f"{name}_{tol:.0e}_iterations"], rh[f"{name}_{tol:.0e}_sigma"]
+        direct = fx["sigma_direct" if name == "icosphere_L2" else "x_direct"]
+
+    def rel(a, b):
+        return np.max(np.abs(a - b)) / np.max(np.abs(b))
+    bound = max(5 * rel(sigma, direct), 100 * tol)
+    with K.CUDAElectrostaticContext(0, assembled_budget_bytes=1000) as ctx:
+        ctx.SetGeometry(m)
+        x, st = ctx.SolveRobinHood(tol=tol)
+        assert st["rel_residual"] <= tol and abs(st["iterations"] - int(checks)) <= 1
+        assert rel(x, direct) <= bound and rel(x, sigma) <= bound
+        with pytest.raises(K.KemcuError):  # the budget is the caller's
+            ctx.SolveRobinHood(tol=tol, assembled=True)
+    with K.CUDAElectrostaticContext(0) as ctx:  # kept columns: entries of another quadrature, 1e-14 apart
+        ctx.SetGeometry(m)
+        y, st2 = ctx.SolveRobinHood(tol=tol)
+        assert abs(st2["iterations"] - st["iterations"]) <= 1 and rel(y, x) <= 2 * bound
+
+
+def test_kept_columns_end_with_the_solve():
+    torch = pytest.importorskip("torch")
+    full = G.icosphere(4)
+    n = 3000  # 72 MB of columns
+    m = G.Mesh(full.shape[:n], full.boundary[:n], full.geom[:n], full.value[:n])
+    with K.CUDAElectrostaticContext(0) as ctx:
+        ctx.SetGeometry(m)
+        ctx.SolveRobinHood(np.ones(n), tol=1e-3, max_subiterations=10, raise_on_failure=False, assembled=False)
+        free = torch.cuda.mem_get_info()[0]
+        ctx.SetGeometry(m)
+        ctx.Multiply(np.ones(n), assembled=True)
+        held = free - torch.cuda.mem_get_info()[0]
+        assert held > 60e6  # the operator that was asked for; the solve had kept none
+        ctx.SolveRobinHood(np.ones(n), tol=1e-3, max_subiterations=10, raise_on_failure=False)
+        assert free - torch.cuda.mem_get_info()[0] > 60e6  # and leaves it
