@@ -989,16 +989,16 @@ template<bool MIXED, bool POT, bool FIELD, bool F32 = false> __device__ __forcei
     return epi_far<MIXED, POT, FIELD, F32>(e, P, d, r2, band);
 }
 
-// epi with the analytic band from the element's near record w (rwg_build_kernel). Not inlined: the
-// kernels whose distant pairs take the series call it for the few that remain, and carry none of its
-// registers in their loops.
+// epi with the analytic band from the element's near record w (rwg_build_kernel): epi_here in place, for
+// the direct sum, which works its near list off at one site; epi through a call, for kernels that evaluate
+// single pairs or whose loops should not carry its registers.
 template<int NV, bool POT, bool FIELD>
 __device__ __noinline__ Out4 rwg_call(const double* __restrict__ e, const double* __restrict__ w, V3 P)
 {
     return rwg_pair<NV, POT, FIELD>(e, w, P);
 }
 template<bool MIXED, bool POT, bool FIELD, bool F32 = false>
-__device__ __noinline__ Out4 epi(const double* __restrict__ e, const double* __restrict__ w, V3 P)
+__device__ __forceinline__ Out4 epi_here(const double* __restrict__ e, const double* __restrict__ w, V3 P)
 {
     V3 d;
     double r2;
@@ -1010,6 +1010,11 @@ __device__ __noinline__ Out4 epi(const double* __restrict__ e, const double* __r
         return type == kTriangle ? rwg_call<3, POT, FIELD>(e, w, P) : rwg_call<4, POT, FIELD>(e, w, P);
     }
     return epi_far<MIXED, POT, FIELD, F32>(e, P, d, r2, band);
+}
+template<bool MIXED, bool POT, bool FIELD, bool F32 = false>
+__device__ __noinline__ Out4 epi(const double* __restrict__ e, const double* __restrict__ w, V3 P)
+{
+    return epi_here<MIXED, POT, FIELD, F32>(e, w, P);
 }
 // the same with the rectangles' largest rule from a table in shared memory
 template<bool MIXED, bool POT, bool FIELD, bool F32 = false>

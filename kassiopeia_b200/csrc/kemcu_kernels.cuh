@@ -273,7 +273,11 @@ struct FarView
 // series loops then contain no call and none of that code's registers. The list is worked off
 // between tiles whenever another tile might not fit, the element records kNearStage at a time through
 // shared memory: their loads run ahead of the pairs, which would otherwise wait for L2 once per element.
-constexpr int kNearList = 64, kNearStage = 2;
+// A short list: while one warp works its list off, the others run out of tiles (the ring holds kPipe of them) and
+// wait. 32 entries against 64, ms: 20,000 points and 28,800 slivers 20.0 and 22.0 (MIXED), 22.0 and 24.5 (FP64);
+// their product 20.1 and 22.3; 400,000 points of a coaxial pair 136 and 140. It also bounds the plain sums
+// of the direct sum's list at 32 terms.
+constexpr int kNearList = 32, kNearStage = 2;
 struct NearStore
 {
     double rec[kNearStage][rRecSize];
@@ -484,7 +488,7 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
         L.drain(rec, [&](int e, const double* r) {
             const double sg = sigma[e];
             for (int p = 0; p < kPair; p++) {
-                const Out4 v = epi<MIXED, POT, FIELD, F32>(r, V.rwg + (size_t) e * wRecSize, p == 0 ? P[0] : P[kPair - 1]);
+                const Out4 v = epi_here<MIXED, POT, FIELD, F32>(r, V.rwg + (size_t) e * wRecSize, p == 0 ? P[0] : P[kPair - 1]);
                 const double w[4] = {v.ex * sg, v.ey * sg, v.ez * sg, v.phi * sg};
 #pragma unroll
                 for (int k = 0; k < NS; k++) {
@@ -523,14 +527,12 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
                     }
                 });
             keep();
-            if (L.full())
+            if (L.full() || (i == ntiles - 1 && L.n > 0))  // one site: its code is large
                 near();
         }
         R.release(i, side);
     }
     R.finish(ok, flag);
-    if (L.n > 0)
-        near();
 #pragma unroll
     for (int p = 0; p < kPair; p++) {
         const int q = base + 32 * p;
