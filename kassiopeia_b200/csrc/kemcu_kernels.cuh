@@ -338,13 +338,13 @@ template<int T> struct Tier
 // holds for all of them, so that the choice is uniform: far(f, j, p, F, d) receives element j's sums
 // for point p (f: its record, d: the point relative to its centroid); elements without one go to the list. A lane per element finds the tier for the warp's
 // bounding sphere; an element whose tier that leaves open is tested point by point.
-template<bool FIELD, bool FAST, int NP, class Far>
+template<bool FIELD, bool FAST, bool F32, int NP, class Far>
 __device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, const V3 (&P)[NP], V3 wc, double wr,
                                            NearList& L, Far far)
 {
     const int lane = threadIdx.x & 31;
     const int stride = T.general ? kFarGenStride : kFarSymStride;
-    const int tier = lane < T.count ? far_tier<FAST>(rec + lane * stride, wc, wr) : 0;
+    const int tier = lane < T.count ? far_tier<FAST, F32>(rec + lane * stride, wc, wr) : 0;
     const unsigned m3 = __ballot_sync(0xffffffffu, tier == 3), m2 = __ballot_sync(0xffffffffu, tier == 2);
     unsigned m1 = __ballot_sync(0xffffffffu, tier == 1);
     for (unsigned m = ~(m1 | m2 | m3) & ((1u << T.count) - 1u); m; m &= m - 1u) {
@@ -353,7 +353,7 @@ __device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, 
         bool low = true;
 #pragma unroll
         for (int p = 0; p < NP; p++)
-            low = low && far_point<FAST>(f, P[p]);
+            low = low && far_point<FAST, F32>(f, P[p]);
         if (__all_sync(0xffffffffu, low))
             m1 |= 1u << j;
         else {
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
             const FarTile T = S.tile[i % kPipe];
             const double* sp = S.side[i % kPipe][0];
             clear();
-            tile_pairs<FIELD, MIXED || F32>(
+            tile_pairs<FIELD, MIXED || F32, F32>(
                 S.rec[i % kPipe], T, P, wc, wr, L,
                 [&](const double* f, int j, int p, const FarSum& F, V3 d) {
                     const double q = sp[j] * F.ir;
@@ -674,18 +674,18 @@ constexpr int kMaxRhs = 8;
 
 // the entries of one tile's columns in kPair rows per lane: emit(p, j, A(row p, first + j)). A warp
 // without a Neumann row sums potentials only; Neumann rows take the field along their normal.
-template<bool FAST, class Emit>
+template<bool FAST, bool F32, class Emit>
 __device__ __forceinline__ void tile_entries(const double* far, const FarTile& T, const double* pre,
                                              const TargetRec* __restrict__ tgt, const int (&row)[kPair],
                                              const V3 (&C)[kPair], bool any_neumann, V3 wc, double wr, NearList& L,
                                              Emit emit)
 {
     if (!any_neumann)
-        tile_pairs<false, FAST>(far, T, C, wc, wr, L, [&](const double*, int j, int p, const FarSum& F, V3) {
+        tile_pairs<false, FAST, F32>(far, T, C, wc, wr, L, [&](const double*, int j, int p, const FarSum& F, V3) {
             emit(p, j, (pre[j] * F.ir) * F.S);
         });
     else
-        tile_pairs<true, FAST>(far, T, C, wc, wr, L, [&](const double* f, int j, int p, const FarSum& F, V3 d) {
+        tile_pairs<true, FAST, F32>(far, T, C, wc, wr, L, [&](const double* f, int j, int p, const FarSum& F, V3 d) {
             const TargetRec& t = tgt[row[p]];
             const V3 nn = v3(t.normal[0], t.normal[1], t.normal[2]);
             const double q = pre[j] * F.ir;
@@ -761,13 +761,13 @@ __global__ void __launch_bounds__(kThreads, NR == 1 ? kMinBlocks : 4)
         if (busy) {
             const FarTile T = S.tile[q % kPipe];
             const double(*sd)[kFarSym] = S.side[q % kPipe];
-            tile_entries<MIXED || F32>(S.rec[q % kPipe], T, sd[NR], tgt, row, C, any_neumann, wc, wr, L,
-                                       [&](int p, int j, double a) {
+            tile_entries<MIXED || F32, F32>(S.rec[q % kPipe], T, sd[NR], tgt, row, C, any_neumann, wc, wr, L,
+                                            [&](int p, int j, double a) {
 #pragma unroll
-                                           for (int r = 0; r < NR; r++)
-                                               if (NR == 1 || r < nrhs)
-                                                   acc[r][p].add(a * sd[r][j]);
-                                       });
+                                                for (int r = 0; r < NR; r++)
+                                                    if (NR == 1 || r < nrhs)
+                                                        acc[r][p].add(a * sd[r][j]);
+                                            });
             if (L.full() || (q == ntiles - 1 && L.n > 0))  // one place: its code is large
                 near();
         }
@@ -849,8 +849,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         }
         if (busy) {
             const FarTile T = S.tile[q % kPipe];
-            tile_entries<MIXED>(S.rec[q % kPipe], T, S.side[q % kPipe][0], tgt, row, C, any_neumann, wc, wr, L,
-                                [&](int p, int j, double a) { store(p, T.first + j, a); });
+            tile_entries<MIXED, false>(S.rec[q % kPipe], T, S.side[q % kPipe][0], tgt, row, C, any_neumann, wc, wr, L,
+                                       [&](int p, int j, double a) { store(p, T.first + j, a); });
             if (L.full() || (q == ntiles - 1 && L.n > 0))  // one place: its code is large
                 near();
         }
