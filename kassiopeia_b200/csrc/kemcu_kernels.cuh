@@ -1169,7 +1169,11 @@ __global__ void morton_kernel(const double* __restrict__ P, int n, const double*
 }
 
 // the same for the matrix rows' collocation points
-__global__ void morton_rows_kernel(const TargetRec* __restrict__ tgt, int n, const double* __restrict__ box,
+struct Box
+{
+    double v[6];
+};
+__global__ void morton_rows_kernel(const TargetRec* __restrict__ tgt, int n, const Box box,
                                    unsigned long long* __restrict__ key, int* __restrict__ idx)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1177,8 +1181,8 @@ __global__ void morton_rows_kernel(const TargetRec* __restrict__ tgt, int n, con
         return;
     unsigned q[3];
     for (int c = 0; c < 3; c++) {
-        const double ext = box[3 + c] - box[c];
-        const double t = ext > 0. ? (tgt[i].cen[c] - box[c]) / ext : 0.;
+        const double ext = box.v[3 + c] - box.v[c];
+        const double t = ext > 0. ? (tgt[i].cen[c] - box.v[c]) / ext : 0.;
         q[c] = (unsigned) fmin(fmax(t * 2097151.0, 0.), 2097151.0);
     }
     key[i] = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);

@@ -60,6 +60,7 @@ struct kemcu_ctx
     std::vector<TargetRec> h_tgt;      // n matrix-row targets
     std::vector<double> h_rhs;         // boundary values
     std::vector<int32_t> h_shape;
+    DevBuf geo;  // what the geometry fixes, from d_rec to d_rows: one allocation
     double* d_rec = nullptr;
     TargetRec* d_tgt = nullptr;
     double* d_sigma = nullptr;
@@ -67,7 +68,7 @@ struct kemcu_ctx
     double* d_far = nullptr;
     FarTile* d_tiles = nullptr;
     double* d_pre = nullptr;
-    int2* d_where = nullptr;  // per element: its far record (16-byte units) and whether it is general
+    int2* d_where = nullptr;  // per element: its far record (far_where)
     double* d_rwg = nullptr;  // near records (rwg_build_kernel)
     int ntiles = 0;
     int* d_rows = nullptr;  // matrix rows in Morton order of their collocation points
@@ -343,52 +344,50 @@ FarView far_view(const kemcu_ctx* ctx)
     return FarView{ctx->d_far, ctx->d_tiles, ctx->ntiles, ctx->d_pre, ctx->d_rwg};
 }
 
-// The far records of the context's planar elements. Tiles in element order: a run of up to kFarSym
+// The far records' tiles of the context's planar elements, in element order: a run of up to kFarSym
 // elements with two mirror axes (rectangles with orthogonal sides, wires), else up to kFarGen
-// elements of any kind in the general form.
-int build_far(kemcu_ctx* ctx)
+// elements of any kind in the general form. Returns the doubles that the records take.
+size_t far_tiling(const kemcu_ctx* ctx, std::vector<FarTile>& tiles)
 {
     const size_t n = ctx->n;
-    std::vector<char> sym(n);
-    for (size_t e = 0; e < n; e++) {
+    auto sym = [&](size_t e) {
         const double* r = &ctx->h_rec[e * rRecSize];
         // below 1e-14 the cosine of the sides' angle changes no moment's last digit
-        sym[e] = ctx->h_shape[e] == kLineSegment ||
-                 (ctx->h_shape[e] == kRectangle && std::fabs(r[rAB2]) <= 2e-14 * std::sqrt(r[rAA] * r[rBB]));
-    }
-    std::vector<FarTile> tiles;
+        return ctx->h_shape[e] == kLineSegment ||
+               (ctx->h_shape[e] == kRectangle && r[rAB2] * r[rAB2] <= 4e-28 * (r[rAA] * r[rBB]));
+    };
     size_t off = 0;
     for (size_t e = 0; e < n;) {
         size_t k = 0;
-        while (k < (size_t) kFarSym && e + k < n && sym[e + k])
+        while (k < (size_t) kFarSym && e + k < n && sym(e + k))
             k++;
         const bool general = k < std::min((size_t) kFarGen, n - e);
         if (general)
             k = std::min((size_t) kFarGen, n - e);
-        tiles.push_back(FarTile{(int) e, (int) k, general ? 1 : 0, (int) (off / 2)});
+        tiles.push_back(FarTile{(int) e, (int) k, general ? 1 : 0, (long long) (off / 2)});
         off += k * (general ? kFarGenStride : kFarSymStride);
         e += k;
     }
-    if (off / 2 > (size_t) 0x7fffffff)
-        return fail(ctx, KEMCU_EINVAL, "%zu elements exceed the far-record table", n);
-    const FmGl g = fm_gauss_legendre(kFarQ);
-    FarTables gl;
-    far_tables(gl);
-    for (int i = 0; i < kFarQ; i++) {
-        gl.x[i] = g.x[i];
-        gl.w[i] = g.w[i];
-    }
-    ctx->ntiles = (int) tiles.size();
-    KC(cudaMalloc(&ctx->d_far, off * sizeof(double)));
-    KC(cudaMalloc(&ctx->d_tiles, tiles.size() * sizeof(FarTile)));
-    KC(cudaMalloc(&ctx->d_pre, n * sizeof(double)));
-    KC(cudaMalloc(&ctx->d_where, n * sizeof(int2)));
-    KC(cudaMemcpyAsync(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(FarTile),
-                       cudaMemcpyHostToDevice, ctx->stream));
-    far_build_kernel<<<(unsigned) ((tiles.size() * kFarSym + 127) / 128), 128, 0, ctx->stream>>>(
-        ctx->d_rec, ctx->d_tiles, ctx->ntiles, gl, ctx->d_far, ctx->d_pre, ctx->d_where);
+    return off;
+}
+
+// the far and near records, from the element records on the device
+int build_far(kemcu_ctx* ctx)
+{
+    static const FarTables tables = [] {
+        FarTables t;
+        far_tables(t);
+        const FmGl g = fm_gauss_legendre(kFarQ);
+        for (int i = 0; i < kFarQ; i++) {
+            t.x[i] = g.x[i];
+            t.w[i] = g.w[i];
+        }
+        return t;
+    }();
+    const size_t threads = (size_t) ctx->ntiles * kFarSym * kFarLanes, n = ctx->n;
+    far_build_kernel<<<(unsigned) ((threads + kFarBuild - 1) / kFarBuild), kFarBuild, 0, ctx->stream>>>(
+        ctx->d_rec, ctx->d_tiles, ctx->ntiles, tables, ctx->d_far, ctx->d_pre, ctx->d_where);
     KCHECK_LAUNCH();
-    KC(cudaMalloc(&ctx->d_rwg, n * wRecSize * sizeof(double)));
     rwg_build_kernel<<<(unsigned) ((n + 127) / 128), 128, 0, ctx->stream>>>(ctx->d_rec, (int) n, ctx->d_rwg);
     KCHECK_LAUNCH();
     return KEMCU_OK;
@@ -406,30 +405,26 @@ size_t cub_sort_bytes(size_t n)
 int build_rows(kemcu_ctx* ctx)
 {
     const size_t n = ctx->n;
-    double box[6] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
+    Box box = {{1e300, 1e300, 1e300, -1e300, -1e300, -1e300}};
     for (size_t i = 0; i < n; i++)
         for (int c = 0; c < 3; c++) {
-            box[c] = std::min(box[c], ctx->h_tgt[i].cen[c]);
-            box[3 + c] = std::max(box[3 + c], ctx->h_tgt[i].cen[c]);
+            box.v[c] = std::min(box.v[c], ctx->h_tgt[i].cen[c]);
+            box.v[3 + c] = std::max(box.v[3 + c], ctx->h_tgt[i].cen[c]);
         }
-    KC(cudaMalloc(&ctx->d_rows, n * sizeof(int)));
     const size_t cub_bytes = cub_sort_bytes(n);
     auto up = [](size_t b) { return (b + 255) & ~(size_t) 255; };
     void* base;
-    if (int rc = ensure(ctx, sSort, 2 * up(n * 8) + up(n * 4) + 256 + up(cub_bytes), &base))
+    if (int rc = ensure(ctx, sSort, 2 * up(n * 8) + up(n * 4) + up(cub_bytes), &base))
         return rc;
     char* q = (char*) base;
     auto* k0 = (unsigned long long*) q;
     auto* k1 = (unsigned long long*) (q + up(n * 8));
     int* i0 = (int*) (q + 2 * up(n * 8));
-    double* dbox = (double*) (q + 2 * up(n * 8) + up(n * 4));
-    void* tmp = (char*) dbox + 256;
-    KC(cudaMemcpyAsync(dbox, box, sizeof box, cudaMemcpyHostToDevice, ctx->stream));
-    morton_rows_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->d_tgt, (int) n, dbox, k0, i0);
+    void* tmp = q + 2 * up(n * 8) + up(n * 4);
+    morton_rows_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->d_tgt, (int) n, box, k0, i0);
     KCHECK_LAUNCH();
     size_t tb = cub_bytes;
     KC(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, i0, ctx->d_rows, (int) n, 0, 63, ctx->stream));
-    KC(cudaStreamSynchronize(ctx->stream));  // box is on this stack frame
     return KEMCU_OK;
 }
 
@@ -1408,20 +1403,12 @@ int kemcu_destroy(kemcu_ctx* ctx)
         for (auto& b : ctx->scratch)
             if (b.p)
                 cudaFree(b.p);
-        cudaFree(ctx->d_rec);
-        cudaFree(ctx->d_tgt);
-        cudaFree(ctx->d_sigma);
+        cudaFree(ctx->geo.p);
         cudaFree(ctx->d_a64);
         cudaFree(ctx->d_a32);
         cudaFree(ctx->d_near_ptr);
         cudaFree(ctx->d_near_row);
         cudaFree(ctx->d_near_val);
-        cudaFree(ctx->d_far);
-        cudaFree(ctx->d_tiles);
-        cudaFree(ctx->d_pre);
-        cudaFree(ctx->d_where);
-        cudaFree(ctx->d_rwg);
-        cudaFree(ctx->d_rows);
         cudaFreeHost(ctx->h_stage);
         cudaFree(ctx->d_counter);
         cudaFree(ctx->d_flag);
@@ -1484,20 +1471,11 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
                                        "triangles, rectangles or line segments");
     // release everything that depends on the old geometry
     fm_release(ctx);
-    cudaFree(ctx->d_rec);
-    cudaFree(ctx->d_tgt);
-    cudaFree(ctx->d_sigma);
     cudaFree(ctx->d_a64);
     cudaFree(ctx->d_a32);
     cudaFree(ctx->d_near_ptr);
     cudaFree(ctx->d_near_row);
     cudaFree(ctx->d_near_val);
-    cudaFree(ctx->d_far);
-    cudaFree(ctx->d_tiles);
-    cudaFree(ctx->d_pre);
-    cudaFree(ctx->d_where);
-    cudaFree(ctx->d_rwg);
-    cudaFree(ctx->d_rows);
     ctx->d_rec = nullptr;
     ctx->d_tgt = nullptr;
     ctx->d_sigma = nullptr;
@@ -1512,7 +1490,6 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     ctx->d_where = nullptr;
     ctx->d_rwg = nullptr;
     ctx->d_rows = nullptr;
-    ctx->ntiles = 0;
     ctx->have_sigma = false;
     ctx->n = 0;
     ctx->h_rec.assign(n * rRecSize, 0.);
@@ -1528,22 +1505,62 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
             build_record(geom11 + 11 * i, shape[i], boundary[i], value[i], ctx->k, ctx->h_rec.data() + i * rRecSize,
                          ctx->h_tgt[i], ctx->h_rhs[i]);
     }
-    KC(cudaMalloc(&ctx->d_rec, n * rRecSize * sizeof(double)));
-    KC(cudaMalloc(&ctx->d_tgt, n * sizeof(TargetRec)));
-    KC(cudaMalloc(&ctx->d_sigma, n * sizeof(double)));
-    KC(cudaMemcpyAsync(ctx->d_rec, ctx->h_rec.data(), n * rRecSize * sizeof(double),
-                       cudaMemcpyHostToDevice, ctx->stream));
-    KC(cudaMemcpyAsync(ctx->d_tgt, ctx->h_tgt.data(), n * sizeof(TargetRec), cudaMemcpyHostToDevice, ctx->stream));
-    KC(cudaMemsetAsync(ctx->d_sigma, 0, n * sizeof(double), ctx->stream));
     ctx->n = n;
+    std::vector<FarTile> tiles;
+    const size_t far = ctx->axisym ? 0 : far_tiling(ctx, tiles);
+    const size_t planar = ctx->axisym ? 0 : n;
+    ctx->ntiles = (int) tiles.size();
+    // One allocation, kept for the next geometry while it fits and is not more than twice what that needs:
+    // allocating and freeing the parts took longer than building the records of a small mesh.
+    size_t bytes = 0;
+    auto part = [&](auto*& p, size_t count) {  // first pass: sizes; second pass: places
+        p = ctx->geo.p ? reinterpret_cast<std::remove_reference_t<decltype(p)>>((char*) ctx->geo.p + bytes) : nullptr;
+        bytes += (count * sizeof(*p) + 255) & ~(size_t) 255;
+    };
+    auto parts = [&]() {
+        bytes = 0;
+        part(ctx->d_rec, n * rRecSize);
+        part(ctx->d_tgt, n);
+        part(ctx->d_sigma, n);
+        part(ctx->d_far, far);
+        part(ctx->d_tiles, tiles.size());
+        part(ctx->d_pre, planar);
+        part(ctx->d_where, planar);
+        part(ctx->d_rwg, planar * wRecSize);
+        part(ctx->d_rows, planar);
+    };
+    parts();
+    int rc = KEMCU_OK;
+    if (ctx->geo.bytes < bytes || ctx->geo.bytes > 2 * bytes + ((size_t) 1 << 20)) {
+        cudaFree(ctx->geo.p);
+        ctx->geo = DevBuf();
+        if (cudaMalloc(&ctx->geo.p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->geo.p = nullptr;
+            rc = fail(ctx, KEMCU_ENOMEM, "device allocation of %zu bytes for %zu elements failed", bytes, n);
+        }
+        else
+            ctx->geo.bytes = bytes;
+        parts();
+    }
+    auto upload = [&](void* dst, const void* src, size_t size) {
+        if (!rc && cudaMemcpyAsync(dst, src, size, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+            rc = fail(ctx, KEMCU_ECUDA, "element records: %s", cudaGetErrorString(cudaGetLastError()));
+    };
+    upload(ctx->d_rec, ctx->h_rec.data(), n * rRecSize * sizeof(double));
+    upload(ctx->d_tgt, ctx->h_tgt.data(), n * sizeof(TargetRec));
+    if (!rc && cudaMemsetAsync(ctx->d_sigma, 0, n * sizeof(double), ctx->stream) != cudaSuccess)
+        rc = fail(ctx, KEMCU_ECUDA, "charge densities: %s", cudaGetErrorString(cudaGetLastError()));
     if (!ctx->axisym) {
-        int rc = build_far(ctx);
+        upload(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(FarTile));
+        if (!rc)
+            rc = build_far(ctx);
         if (!rc)
             rc = build_rows(ctx);
-        if (rc) {
-            ctx->n = 0;
-            return rc;
-        }
+    }
+    if (rc) {
+        ctx->n = 0;
+        return rc;
     }
     // the records are in place for whichever stream the next call runs on; the copies above are ordered on
     // this stream because a copy from pageable memory may return before it has arrived

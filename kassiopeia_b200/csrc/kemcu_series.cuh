@@ -80,8 +80,18 @@ static_assert(2 * fSymF + kSEnd <= 2 * kFarSymStride && 2 * fGenF + kGEnd <= 2 *
 // one tile: elements [first, first + count), doubles offset of its records, general or symmetric
 struct FarTile
 {
-    int first, count, general, off16;  // off16: offset in 16-byte units
+    int first, count, general;
+    long long off16;  // offset in 16-byte units
 };
+// where an element's far record is: the low 32 bits of its offset, the high bits and whether it is general
+__host__ __device__ inline int2 far_where(long long off16, bool general)
+{
+    return make_int2((int) (unsigned) off16, (int) (off16 >> 32) * 2 + (general ? 1 : 0));
+}
+__host__ __device__ inline size_t far_offset(int2 at)
+{
+    return 2 * (((size_t) (at.y >> 1) << 32) | (unsigned) at.x);
+}
 
 // ------------------------------------------------------------------------- building
 constexpr int kFarOrder = 12;  // moments: up to the first order that any tier leaves out
@@ -116,75 +126,98 @@ inline void far_tables(FarTables& t)  // all but the quadrature rule
     }
 }
 
-struct FarMoments
+// One warp builds a record; as plain C++ one lane does.
+#ifdef __CUDACC__
+constexpr int kFarLanes = 32;
+__device__ __forceinline__ double far_max(double v)
 {
-    double m[kFarOrder + 1][kFarOrder + 1];  // < x^a y^b > / s^(a + b), a + b <= kFarOrder
+    for (int o = 16; o > 0; o >>= 1)
+        v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+#else
+#define __shared__ static
+constexpr int kFarLanes = 1;
+inline double far_max(double v)
+{
+    return v;
+}
+inline void __syncwarp() {}
+inline void __syncthreads() {}
+#endif
+constexpr int kFarBuild = 4 * kFarLanes;  // threads of a CTA
+constexpr int kFarDirs = 25;              // directions that |G_n| is looked at in
+
+// coefficients of G_n, n <= kFarOrder: those of X^i Y^j with i + j = n, n - 2, ...
+__host__ __device__ constexpr int far_count(int n)
+{
+    return (n + 2) * (n + 2) / 4;
+}
+__host__ __device__ constexpr int far_base(int n)  // orders 2, 3, ..., n - 1 come first
+{
+    int s = 0;
+    for (int q = 2; q < n; q++)
+        s += far_count(q);
+    return s;
+}
+constexpr int kFarCoefs = far_base(kFarOrder + 1);
+__device__ __forceinline__ int far_index(int n, int i, int j)  // within order n
+{
+    const int m = (n - i - j) / 2;
+    return m * (n + 1) - m * (m - 1) + i;
+}
+
+// a warp's workspace
+struct FarWork
+{
+    double M[kFarOrder + 1][kFarOrder + 1];  // < x^a y^b > / s^(a + b), a + b <= kFarOrder
+    double c[kFarCoefs];
+    double g[kFarOrder + 1];  // largest |G_n|
+    double r[16];
+    alignas(16) double f[kFarGenStride];
 };
-
-// coefficient of X^i Y^j in G_n (i + j = n - 2m)
-__device__ __noinline__ double far_coef(const FarTables& t, const FarMoments& M, int n, int i, int j)
+struct FarBinLeg
 {
-    const int k = i + j, m = (n - k) / 2;
-    double s = 0.;
-    for (int a = 0; a <= m; a++)
-        s += t.bin[m][a] * M.m[i + 2 * a][j + 2 * (m - a)];
-    return t.leg[n][m] * t.bin[k][i] * s;
-}
-
-// largest |G_n| over directions (in the plane, at 60 degrees from its normal and along it)
-__device__ __noinline__ double far_largest(const FarTables& t, const FarMoments& M, int n)
-{
-    double v0[12], v1[12], vz = 0.;
-    for (int q = 0; q < 12; q++)
-        v0[q] = v1[q] = 0.;
-    for (int k = n; k >= 0; k -= 2)
-        for (int i = 0; i <= k; i++) {
-            const double c = far_coef(t, M, n, i, k - i);
-            if (k == 0)
-                vz = c;
-            for (int q = 0; q < 12; q++) {
-                double v = c;
-                for (int a = 0; a < i; a++)
-                    v *= t.ca[q];
-                for (int a = i; a < k; a++)
-                    v *= t.sa[q];
-                v0[q] += v;
-                for (int a = 0; a < k; a++)
-                    v *= 0.8660254037844386;
-                v1[q] += v;
-            }
-        }
-    double big = fabs(vz);
-    for (int q = 0; q < 12; q++)
-        big = fmax(big, fmax(fabs(v0[q]), fabs(v1[q])));
-    return big;
-}
+    double bin[kFarOrder + 1][kFarOrder + 1], leg[kFarOrder + 1][kFarOrder / 2 + 1];
+};
 
 // the coefficients of the class (px, py) of G_n, X^px Y^py poly(X^2, Y^2) of degree `deg`, in
 // the order far_poly reads them (powers of X^2 descending; within one, powers of Y^2 descending)
-template<class T> __device__ __noinline__ int far_class(const FarTables& t, const FarMoments& M, int n, int px, int py, int deg, T* out)
+template<int N, int PX, int PY, int DEG, class T> __device__ __forceinline__ void far_class(const FarWork& W, int lane, T* out)
 {
-    int k = 0;
-    for (int i = deg; i >= 0; i--)
-        for (int j = deg - i; j >= 0; j--)
-            out[k++] = (T) far_coef(t, M, n, 2 * i + px, 2 * j + py);
-    return k;
+    for (int k = lane; k < far_terms(DEG); k += kFarLanes) {
+        int row = 0, first = 0;  // row: DEG - i, of row + 1 terms
+        while (first + row + 1 <= k)
+            first += ++row;
+        const int i = DEG - row, j = row - (k - first);
+        out[k] = (T) W.c[far_base(N) + far_index(N, 2 * i + PX, 2 * j + PY)];
+    }
 }
 
-// Far record of every element from its element record, one thread per element; the moments of
-// rectangles and wires are closed forms, a triangle's an exact cubature.
+// Far record of every element from its element record, one warp per slot of the tiles; the moments of
+// rectangles and wires in symmetric tiles are closed forms, the others' an exact cubature. (One
+// thread per element was a chain of 0.96 ms whatever their number.)
 __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* __restrict__ tiles, int ntiles,
                                  const __grid_constant__ FarTables gl, double* __restrict__ far, double* __restrict__ pre, int2* __restrict__ where)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ti = q / kFarSym, k = q % kFarSym;
+    __shared__ FarBinLeg s_t;
+    __shared__ FarWork s_w[kFarBuild / kFarLanes];
+    for (int i = threadIdx.x; i < (kFarOrder + 1) * (kFarOrder + 1); i += blockDim.x)
+        s_t.bin[i / (kFarOrder + 1)][i % (kFarOrder + 1)] = gl.bin[i / (kFarOrder + 1)][i % (kFarOrder + 1)];
+    for (int i = threadIdx.x; i < (kFarOrder + 1) * (kFarOrder / 2 + 1); i += blockDim.x)
+        s_t.leg[i / (kFarOrder / 2 + 1)][i % (kFarOrder / 2 + 1)] = gl.leg[i / (kFarOrder / 2 + 1)][i % (kFarOrder / 2 + 1)];
+    __syncthreads();
+    const int lane = threadIdx.x % kFarLanes;
+    const size_t q = (blockIdx.x * (size_t) blockDim.x + threadIdx.x) / kFarLanes;
+    const int ti = (int) (q / kFarSym), k = (int) (q % kFarSym);
     if (ti >= ntiles || k >= tiles[ti].count)
         return;
+    FarWork& W = s_w[threadIdx.x / kFarLanes];
     const FarTile T = tiles[ti];
     const double* e = rec + (size_t) (T.first + k) * rRecSize;
     const int stride = T.general ? kFarGenStride : kFarSymStride;
-    double* f = far + 2 * (size_t) T.off16 + (size_t) k * stride;
-    for (int i = 0; i < stride; i++)
+    double* f = W.f;
+    for (int i = lane; i < stride; i += kFarLanes)
         f[i] = 0.;
     const int type = (int) e[rType];
     const V3 a = ld3(e + rEa), b = ld3(e + rEb), c = ld3(e + rCen);
@@ -198,135 +231,193 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
     e2 = (1. / norm(e2)) * e2;
     const double bx = dot(b, e1), by = dot(b, e2);
     // s and the moments over s
-    FarMoments M;
-    for (int i = 0; i <= kFarOrder; i++)
-        for (int j = 0; j <= kFarOrder; j++)
-            M.m[i][j] = 0.;
     double s;
-    if (type == kTriangle) {
-        const double x0 = -(la + bx) / 3., y0 = -by / 3.;
+    // the corner (x0, y0) and the sides that its nodes (u, v) in [0, 1]^2 run along
+    const bool triangle = type == kTriangle;
+    const double wx = type == kLineSegment ? 0. : bx, wy = type == kLineSegment ? 0. : by;
+    double x0, y0;
+    if (triangle) {
+        x0 = -(la + bx) / 3., y0 = -by / 3.;
         const double x1 = la + x0, y1 = y0, x2 = bx + x0, y2 = by + y0;
         s = sqrt(fmax(x0 * x0 + y0 * y0, fmax(x1 * x1 + y1 * y1, x2 * x2 + y2 * y2)));
-        for (int i = 0; i < kFarQ; i++)
-            for (int j = 0; j < kFarQ; j++) {
-                const double u = gl.x[i], v = gl.x[j] * (1. - u), w = 2. * gl.w[i] * gl.w[j] * (1. - u);
-                const double x = (x0 + u * la + v * bx) / s, y = (y0 + v * by) / s;
-                double xp = w;
-                for (int ax = 0; ax <= kFarOrder; ax++) {
-                    double v2 = xp;
-                    for (int ay = 0; ax + ay <= kFarOrder; ay++) {
-                        M.m[ax][ay] += v2;
-                        v2 *= y;
-                    }
-                    xp *= x;
-                }
-            }
     }
-    else {
-        // the parallelogram u a + v b, u, v in [-1/2, 1/2] (wires: b = 0)
-        const double wx = type == kLineSegment ? 0. : bx, wy = type == kLineSegment ? 0. : by;
+    else {  // the parallelogram u a + v b, u, v in [-1/2, 1/2] (wires: b = 0)
         const double cx1 = 0.5 * (la + wx), cx2 = 0.5 * (la - wx), cy = 0.5 * wy;
         s = sqrt(fmax(cx1 * cx1 + cy * cy, cx2 * cx2 + cy * cy));
-        if (!T.general) {
-            const double hx = 0.5 * la / s, hy = cy / s;
-            double xp = 1.;
-            for (int ax = 0; ax <= kFarOrder; ax += 2) {
-                double v2 = xp / (ax + 1.);
-                for (int ay = 0; ax + ay <= kFarOrder; ay += 2) {
-                    M.m[ax][ay] = v2 / (ay + 1.);
-                    v2 *= hy * hy;
-                }
-                xp *= hx * hx;
-            }
+        x0 = -cx1, y0 = -cy;
+    }
+    const double is = 1. / s;
+    if (!T.general) {
+        const double hx = 0.5 * la * is, hy = 0.5 * wy * is;
+        for (int m = lane; m < (kFarOrder / 2 + 1) * (kFarOrder / 2 + 1); m += kFarLanes) {
+            const int i = m / (kFarOrder / 2 + 1), j = m % (kFarOrder / 2 + 1);
+            double v = 1. / ((2. * i + 1.) * (2. * j + 1.));
+            for (int p = 0; p < i; p++)
+                v *= hx * hx;
+            for (int p = 0; p < j; p++)
+                v *= hy * hy;
+            if (i + j <= kFarOrder / 2)
+                W.M[2 * i][2 * j] = v;
         }
-        else
+    }
+    else
+        for (int ax = lane; ax <= kFarOrder; ax += kFarLanes) {  // a lane per power of x
+            double m[kFarOrder + 1];
+#pragma unroll
+            for (int ay = 0; ay <= kFarOrder; ay++)
+                m[ay] = 0.;
+#pragma unroll 1
             for (int i = 0; i < kFarQ; i++)
+#pragma unroll 1
                 for (int j = 0; j < kFarQ; j++) {
-                    const double u = gl.x[i] - 0.5, v = gl.x[j] - 0.5, w = gl.w[i] * gl.w[j];
-                    const double x = (u * la + v * wx) / s, y = v * wy / s;
-                    double xp = w;
-                    for (int ax = 0; ax <= kFarOrder; ax++) {
-                        double v2 = xp;
-                        for (int ay = 0; ax + ay <= kFarOrder; ay++) {
-                            M.m[ax][ay] += v2;
-                            v2 *= y;
-                        }
-                        xp *= x;
+                    const double u = gl.x[i], h = triangle ? 1. - u : 1., v = gl.x[j] * h;
+                    const double x = (x0 + u * la + v * wx) * is, y = (y0 + v * wy) * is;
+                    double p = (triangle ? 2. : 1.) * gl.w[i] * gl.w[j] * h, x2 = x;
+#pragma unroll
+                    for (int bit = 1; bit <= kFarOrder; bit <<= 1) {
+                        if (ax & bit)
+                            p *= x2;
+                        x2 *= x2;
+                    }
+#pragma unroll
+                    for (int ay = 0; ay <= kFarOrder; ay++) {
+                        m[ay] += p;
+                        p *= y;
                     }
                 }
+#pragma unroll
+            for (int ay = 0; ay <= kFarOrder; ay++)
+                if (ax + ay <= kFarOrder)
+                    W.M[ax][ay] = m[ay];
+        }
+    __syncwarp();
+    // coefficient of X^i Y^j in G_n (i + j = p = n - 2m); two mirror axes leave even n, i and j
+    for (int w = lane; w < kFarCoefs; w += kFarLanes) {
+        int n = 2, t = w;
+        while (t >= far_count(n))
+            t -= far_count(n++);
+        int p = n;
+        while (t > p) {
+            t -= p + 1;
+            p -= 2;
+        }
+        const int i = t, j = p - t, m = (n - p) / 2;
+        double v = 0.;
+        if (T.general || !(i & 1 || j & 1)) {
+            for (int z = 0; z <= m; z++)
+                v += s_t.bin[m][z] * W.M[i + 2 * z][j + 2 * (m - z)];
+            v *= s_t.leg[n][m] * s_t.bin[p][i];
+        }
+        W.c[w] = v;
     }
-    f[fCen] = c.x, f[fCen + 1] = c.y, f[fCen + 2] = c.z;
-    f[fSize] = s;
-    f[fE1] = e1.x, f[fE1 + 1] = e1.y, f[fE1 + 2] = e1.z;
-    f[fE1 + 3] = e2.x, f[fE1 + 4] = e2.y, f[fE1 + 5] = e2.z;
-    far_class(gl, M, 2, 0, 0, 1, f + fD2);
-    far_class(gl, M, 4, 0, 0, 2, f + fD4);
+    __syncwarp();
+    // largest |G_n| over directions in the plane (every 15 degrees), at 60 degrees from its normal and along it
+    for (int n = 4; n <= kFarOrder; n++) {
+        if (n == 5 || (!T.general && n & 1)) {
+            if (lane == 0)
+                W.g[n] = 0.;
+            continue;
+        }
+        double big = 0.;
+        for (int z = lane; z < kFarDirs; z += kFarLanes) {
+            const double x = z < 24 ? gl.ca[z % 12] * (z < 12 ? 1. : 0.8660254037844386) : 0.;
+            const double y = z < 24 ? gl.sa[z % 12] * (z < 12 ? 1. : 0.8660254037844386) : 0.;
+            const double* cn = W.c + far_base(n);
+            double v = 0.;
+            for (int p = n; p >= 0; p -= 2) {
+                double yp = 1., h = 0.;
+                for (int i = p; i >= 0; i--) {  // sum over i of c x^i y^(p - i)
+                    h = fma(h, x, cn[i] * yp);
+                    yp *= y;
+                }
+                v += h;
+                cn += p + 1;
+            }
+            big = fmax(big, fabs(v));
+        }
+        big = far_max(big);
+        if (lane == 0)
+            W.g[n] = big;
+    }
+    __syncwarp();
+    if (lane == 0) {
+        f[fCen] = c.x, f[fCen + 1] = c.y, f[fCen + 2] = c.z;
+        f[fSize] = s;
+        f[fE1] = e1.x, f[fE1 + 1] = e1.y, f[fE1 + 2] = e1.z;
+        f[fE1 + 3] = e2.x, f[fE1 + 4] = e2.y, f[fE1 + 5] = e2.z;
+    }
+    far_class<2, 0, 0, 1>(W, lane, f + fD2);
+    far_class<4, 0, 0, 2>(W, lane, f + fD4);
     if (T.general) {
-        far_class(gl, M, 2, 1, 1, 0, f + fD2 + 3);
-        far_class(gl, M, 3, 1, 0, 1, f + fGenD3);
-        far_class(gl, M, 3, 0, 1, 1, f + fGenD3 + 3);
-        far_class(gl, M, 4, 1, 1, 1, f + fGenQ4);
-        far_class(gl, M, 5, 1, 0, 2, f + fGenD5);
-        far_class(gl, M, 5, 0, 1, 2, f + fGenD5 + 6);
+        far_class<2, 1, 1, 0>(W, lane, f + fD2 + 3);
+        far_class<3, 1, 0, 1>(W, lane, f + fGenD3);
+        far_class<3, 0, 1, 1>(W, lane, f + fGenD3 + 3);
+        far_class<4, 1, 1, 1>(W, lane, f + fGenQ4);
+        far_class<5, 1, 0, 2>(W, lane, f + fGenD5);
+        far_class<5, 0, 1, 2>(W, lane, f + fGenD5 + 6);
         float* g = reinterpret_cast<float*>(f + fGenF);
-        far_class(gl, M, 5, 1, 0, 2, g + kG5p);
-        far_class(gl, M, 5, 0, 1, 2, g + kG5q);
-        far_class(gl, M, 6, 0, 0, 3, g + kG6p);
-        far_class(gl, M, 6, 1, 1, 2, g + kG6q);
-        far_class(gl, M, 7, 1, 0, 3, g + kG7p);
-        far_class(gl, M, 7, 0, 1, 3, g + kG7q);
-        far_class(gl, M, 8, 0, 0, 4, g + kG8p);
-        far_class(gl, M, 8, 1, 1, 3, g + kG8q);
-        far_class(gl, M, 9, 1, 0, 4, g + kG9p);
-        far_class(gl, M, 9, 0, 1, 4, g + kG9q);
-        far_class(gl, M, 10, 0, 0, 5, g + kG10p);
-        far_class(gl, M, 10, 1, 1, 4, g + kG10q);
+        far_class<5, 1, 0, 2>(W, lane, g + kG5p);
+        far_class<5, 0, 1, 2>(W, lane, g + kG5q);
+        far_class<6, 0, 0, 3>(W, lane, g + kG6p);
+        far_class<6, 1, 1, 2>(W, lane, g + kG6q);
+        far_class<7, 1, 0, 3>(W, lane, g + kG7p);
+        far_class<7, 0, 1, 3>(W, lane, g + kG7q);
+        far_class<8, 0, 0, 4>(W, lane, g + kG8p);
+        far_class<8, 1, 1, 3>(W, lane, g + kG8q);
+        far_class<9, 1, 0, 4>(W, lane, g + kG9p);
+        far_class<9, 0, 1, 4>(W, lane, g + kG9q);
+        far_class<10, 0, 0, 5>(W, lane, g + kG10p);
+        far_class<10, 1, 1, 4>(W, lane, g + kG10q);
     }
     else {
         float* g = reinterpret_cast<float*>(f + fSymF);
-        far_class(gl, M, 4, 0, 0, 2, g + kS4);
-        far_class(gl, M, 6, 0, 0, 3, f + fSymD6);
-        far_class(gl, M, 6, 0, 0, 3, g + kS6);
-        far_class(gl, M, 8, 0, 0, 4, g + kS8);
-        far_class(gl, M, 10, 0, 0, 5, g + kS10);
+        far_class<4, 0, 0, 2>(W, lane, g + kS4);
+        far_class<6, 0, 0, 3>(W, lane, f + fSymD6);
+        far_class<6, 0, 0, 3>(W, lane, g + kS6);
+        far_class<8, 0, 0, 4>(W, lane, g + kS8);
+        far_class<10, 0, 0, 5>(W, lane, g + kS10);
     }
     // Cuts: the first order left out, n, contributes t^n G_n to the value and (n + 1) times that to
     // the field, held to `eps` of the term at the cut; sampled directions and the later orders
     // (R >= 5 s) are covered by the factor 1.5. Odd and even orders are looked at (parallelograms have
     // no odd ones). An order n evaluated in FP32 rounds by at most ~4e-7 (n + 1) t^n G_n. Never near
     // the analytic band.
-    const double g7 = T.general ? far_largest(gl, M, 7) : 0., g8 = far_largest(gl, M, 8),
-                 g9 = T.general ? far_largest(gl, M, 9) : 0., g10 = far_largest(gl, M, 10),
-                 g11 = T.general ? far_largest(gl, M, 11) : 0., g12 = far_largest(gl, M, 12),
-                 g4 = far_largest(gl, M, 4), g6 = far_largest(gl, M, 6);
-    auto reach = [&](double g, int n, double eps) { return pow(1.5 * (n + 1) * g / eps, 1. / n); };
-    auto rounds = [&](double g, int n, double eps) { return pow(4e-7 * (n + 1) * g / eps, 1. / n); };
-    auto distance = [&](double r) { return fmax(s * fmax(5., r), sqrt(2. * e[rCut])); };
-    for (int form = 0; form < 2; form++) {
-        const double eps = form ? 1e-14 : 5e-16;
-        double* c = f + (form ? fCutM : fCut);
-        // symmetric: n <= 6, 8, 10; general: n <= 6, 8, 10
-        double r1 = fmax(reach(g11, 11, eps), reach(g12, 12, eps));
-        double r2 = fmax(reach(g9, 9, eps), reach(g10, 10, eps));
-        double r3 = fmax(reach(g7, 7, eps), reach(g8, 8, eps));
-        if (form && !T.general)  // n = 4 in FP32 beyond the first cut
-            r3 = fmax(r3, rounds(g4, 4, 3e-13));
-        else {
-            if (T.general)
-                r1 = fmax(r1, rounds(g6, 6, 1e-15));
-            r2 = fmax(r2, rounds(g6, 6, 1e-15));
-        }
-        r2 = fmax(r2, r1);
-        r3 = fmax(r3, r2);
-        c[0] = distance(r3), c[1] = distance(r2), c[2] = distance(r1);
+    for (int z = lane; z < 14; z += kFarLanes) {
+        const double eps = z < 6 ? 5e-16 : z < 12 ? 1e-14 : z == 12 ? 3e-13 : 1e-15;  // FP64, MIXED; FP32 orders
+        const int n = z < 12 ? 7 + z % 6 : z == 12 ? 4 : 6;
+        W.r[z] = pow((z < 12 ? 1.5 : 4e-7) * (n + 1) * W.g[n] / eps, 1. / n);
     }
-    // a degenerate element (no plane, no extent) keeps the cubature everywhere
-    const double chk = e1.x + e1.y + e1.z + e2.x + e2.y + e2.z + f[fCut] + f[fCut + 2] + f[fCutM] + f[fCutM + 2];
-    if (!(s > 0.) || !isfinite(chk))
-        for (int i = 0; i < 6; i++)
-            f[fCut + i] = CUDART_INF;
-    where[T.first + k] = make_int2(T.off16 + k * stride / 2, T.general);
-    pre[T.first + k] = type == kLineSegment ? e[rPrefac] * e[rA] : e[rPrefac];
+    __syncwarp();
+    if (lane == 0) {
+        auto distance = [&](double r) { return fmax(s * fmax(5., r), sqrt(2. * e[rCut])); };
+        for (int form = 0; form < 2; form++) {
+            const double* r = W.r + 6 * form;
+            double* cut = f + (form ? fCutM : fCut);
+            // symmetric: n <= 6, 8, 10; general: n <= 6, 8, 10
+            double r1 = fmax(r[4], r[5]), r2 = fmax(r[2], r[3]), r3 = fmax(r[0], r[1]);
+            if (form && !T.general)  // n = 4 in FP32 beyond the first cut
+                r3 = fmax(r3, W.r[12]);
+            else {
+                if (T.general)
+                    r1 = fmax(r1, W.r[13]);
+                r2 = fmax(r2, W.r[13]);
+            }
+            r2 = fmax(r2, r1);
+            r3 = fmax(r3, r2);
+            cut[0] = distance(r3), cut[1] = distance(r2), cut[2] = distance(r1);
+        }
+        // a degenerate element (no plane, no extent) keeps the cubature everywhere
+        const double chk = e1.x + e1.y + e1.z + e2.x + e2.y + e2.z + f[fCut] + f[fCut + 2] + f[fCutM] + f[fCutM + 2];
+        if (!(s > 0.) || !isfinite(chk))
+            for (int i = 0; i < 6; i++)
+                f[fCut + i] = CUDART_INF;
+        where[T.first + k] = far_where(T.off16 + k * stride / 2, T.general);
+        pre[T.first + k] = type == kLineSegment ? e[rPrefac] * e[rA] : e[rPrefac];
+    }
+    __syncwarp();
+    double* out = far + 2 * (size_t) T.off16 + (size_t) k * stride;
+    for (int i = lane; i < stride; i += kFarLanes)
+        out[i] = f[i];
 }
 
 // ------------------------------------------------------------------------- evaluation

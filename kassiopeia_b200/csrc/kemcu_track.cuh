@@ -113,12 +113,12 @@ template<bool MIXED> __device__ __forceinline__ V3 track_pair(const double* f, b
     return v3(r.ex, r.ey, r.ez);
 }
 
-// far record of element j: its tile holds kFarSym symmetric or kFarGen general elements in order
+// the elements as the tracker takes them
 struct TrackElems
 {
     FarView V;
     const double* rec;
-    const int2* where;  // per element: offset of its far record in 16-byte units, general
+    const int2* where;  // per element: its far record (far_where)
     const double* sigma;
     int n;
 };
@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems 
         int2 at = make_int2(0, 0);
         auto fetch = [&](int j) {
             at = el.where[j];
-            const double* f = el.V.far + 2 * (size_t) at.x;
-            const int len = at.y ? kFarGenStride : kFarSymStride;
+            const double* f = el.V.far + far_offset(at);
+            const int len = at.y & 1 ? kFarGenStride : kFarSymStride;
 #pragma unroll
             for (int k = 0; k < NV; k++)
                 if (lane + 32 * k < len)
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems 
             Kahan ex, ey, ez;
             for (int j = c; j < el.n; j += kTrackParts) {
                 __syncwarp();
-                const bool general = at.y != 0;
+                const bool general = at.y & 1;
                 const int len = general ? kFarGenStride : kFarSymStride;
 #pragma unroll
                 for (int k = 0; k < NV; k++)
