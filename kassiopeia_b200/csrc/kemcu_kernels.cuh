@@ -550,15 +550,20 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
 // other lanes would repeat it. Each CTA sums kFewElems elements for one point; the sums of the CTAs
 // are added in order by reduce_splits.
 constexpr int kFewPoints = 8, kFewElems = 128;
+struct FewPoints
+{
+    double v[3 * kFewPoints];
+};
 template<bool MIXED, bool POT, bool FIELD, bool F32>
 __global__ void __launch_bounds__(kFewElems) field_few_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
                                                               const double* __restrict__ sigma, int n_elem,
-                                                              const double* __restrict__ pts, int n_pts,
-                                                              double* __restrict__ partial)
+                                                              const double* __restrict__ pts, const FewPoints host,
+                                                              int n_pts, double* __restrict__ partial)
 {
     __shared__ double s_w[4][kFewElems / 32];
     const int e = blockIdx.y * kFewElems + threadIdx.x, q = blockIdx.x;
-    const V3 P = v3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]);
+    // points in device memory, or (null) the caller's as an argument
+    const V3 P = pts ? v3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]) : v3(host.v[3 * q], host.v[3 * q + 1], host.v[3 * q + 2]);
     double v[4] = {0., 0., 0., 0.};
     if (e < n_elem) {
         const Out4 r = epi<MIXED, POT, FIELD, F32>(rec + (size_t) e * rRecSize, rwg + (size_t) e * wRecSize, P);

@@ -84,7 +84,6 @@ struct kemcu_ctx
     double* d_near_val = nullptr;
     // grow-only scratch
     DevBuf scratch[16];
-    void* h_stage = nullptr;  // pinned host memory for the copies of small calls (kStageBytes)
     unsigned* d_counter = nullptr;
     int* d_flag = nullptr;
     double* noalloc_scratch = nullptr;  // device address of g_noalloc_scratch on this context's device
@@ -428,6 +427,8 @@ int build_rows(kemcu_ctx* ctx)
     return KEMCU_OK;
 }
 
+constexpr size_t kSortMin = 4096;  // below this the point set is evaluated in caller order
+
 // axisymmetric elements: FP64 element integrals whatever the precision argument. The element
 // range is split over gridDim.y (axisym_split), partial sums in `scratch` (n x 4 x split
 // doubles, capped at `scratch_cap` doubles; null: grow-only scratch of the context)
@@ -545,15 +546,16 @@ void finish_variant(kemcu_ctx* ctx)
 }
 
 template<bool MIXED, bool F32>
-void few_form(dim3 grid, cudaStream_t st, int what, const kemcu_ctx* ctx, const double* pts, int np, double* part)
+void few_form(dim3 grid, cudaStream_t st, int what, const kemcu_ctx* ctx, const double* pts, const FewPoints& host, int np,
+              double* part)
 {
     const int ne = (int) ctx->n;
     if (what == KEMCU_POTENTIAL)
-        field_few_kernel<MIXED, true, false, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, np, part);
+        field_few_kernel<MIXED, true, false, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, host, np, part);
     else if (what == KEMCU_FIELD)
-        field_few_kernel<MIXED, false, true, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, np, part);
+        field_few_kernel<MIXED, false, true, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, host, np, part);
     else
-        field_few_kernel<MIXED, true, true, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, np, part);
+        field_few_kernel<MIXED, true, true, F32><<<grid, kFewElems, 0, st>>>(ctx->d_rec, ctx->d_rwg, ctx->d_sigma, ne, pts, host, np, part);
 }
 
 // the planar direct sum at device points (d_out n x 4): K1, split `split` ways over the element
@@ -630,10 +632,6 @@ int launch_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d_out, i
     return launch_planar_field(ctx, d_pts, n, d_out, precision, what, split, partial);
 }
 
-// bytes of the context's pinned staging memory: the points, results and flags of a few points
-constexpr size_t kStageBytes = 4096;
-constexpr size_t kSortMin = 4096;  // below this the point set is evaluated in caller order
-
 int check_finite(kemcu_ctx* ctx, const double* d, size_t m, const char* what)
 {
     KC(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
@@ -650,9 +648,9 @@ int check_finite(kemcu_ctx* ctx, const double* d, size_t m, const char* what)
 }
 
 // A handful of points (field_few_kernel), planar elements. The points come from device memory dP or
-// host memory P, the results go to dout or, from host memory, to out. One wait for the GPU, on copies
-// through pinned memory: a probe's time is launches, copies and waits (99.6 us for one point of a
-// 1,280-triangle sphere with K1, two memsets, four kernels and three waits).
+// host memory P (as an argument of the kernel), the results go to dout or, from host memory, to out. One copy
+// and one wait: a probe's time is launches, copies and waits (99.6 us for one point of a 1,280-triangle
+// sphere with K1, two memsets, four kernels and three waits).
 bool few_points(const kemcu_ctx* ctx, size_t n)
 {
     // (the tuner's forced shapes are K1's)
@@ -664,49 +662,44 @@ int field_few(kemcu_ctx* ctx, const double* P, const double* dP, size_t n, doubl
               int what)
 {
     const int split = (int) ((ctx->n + kFewElems - 1) / kFewElems), m = 4 * (int) n;
+    struct Result
+    {
+        double v[4 * kFewPoints];
+        int flag[2];
+    } h;
     void* base;
-    const size_t bytes = (4 + 3) * kFewPoints * sizeof(double) + 2 * sizeof(int);
-    static_assert((4 + 3) * kFewPoints * sizeof(double) + 2 * sizeof(int) <= kStageBytes, "staging of a few points");
-    if (int rc = ensure(ctx, sPartial, bytes + 64 + (size_t) split * m * sizeof(double), &base))
+    if (int rc = ensure(ctx, sPartial, ((sizeof h + 63) & ~(size_t) 63) + (size_t) split * m * sizeof(double), &base))
         return rc;
-    // results | flags | points | partial sums
-    double* d_res = (double*) base;
-    int* d_fl = (int*) (d_res + 4 * kFewPoints);
-    double* d_pts = d_res + 4 * kFewPoints + 1;
-    double* d_part = (double*) ((char*) base + ((bytes + 63) & ~(size_t) 63));
-    double* h = (double*) ctx->h_stage;
+    Result* d = (Result*) base;
+    double* d_part = (double*) ((char*) base + ((sizeof h + 63) & ~(size_t) 63));
     cudaStream_t st = ctx->stream;
-    if (P) {
-        std::memcpy(h, P, n * 3 * sizeof(double));
-        KC(cudaMemcpyAsync(d_pts, h, n * 3 * sizeof(double), cudaMemcpyHostToDevice, st));
-    }
+    FewPoints host{};
+    if (P)
+        std::memcpy(host.v, P, n * 3 * sizeof(double));
     KC(cudaEventRecord(ctx->ev0, st));
     const dim3 grid((unsigned) n, (unsigned) split);
-    const double* pts = P ? d_pts : dP;
     if (precision == KEMCU_FP32)
-        few_form<false, true>(grid, st, what, ctx, pts, (int) n, d_part);
+        few_form<false, true>(grid, st, what, ctx, dP, host, (int) n, d_part);
     else if (precision == KEMCU_MIXED)
-        few_form<true, false>(grid, st, what, ctx, pts, (int) n, d_part);
+        few_form<true, false>(grid, st, what, ctx, dP, host, (int) n, d_part);
     else
-        few_form<false, false>(grid, st, what, ctx, pts, (int) n, d_part);
+        few_form<false, false>(grid, st, what, ctx, dP, host, (int) n, d_part);
     KCHECK_LAUNCH();
-    field_few_sum_kernel<<<1, 32, 0, st>>>(d_part, split, m, out ? d_res : dout, d_fl);
+    field_few_sum_kernel<<<1, 32, 0, st>>>(d_part, split, m, out ? d->v : dout, d->flag);
     KCHECK_LAUNCH();
     KC(cudaEventRecord(ctx->ev1, st));
-    // results and flags lie together
-    const int* hf = (const int*) (h + 4 * kFewPoints);
     if (out)
-        KC(cudaMemcpyAsync(h, d_res, 4 * kFewPoints * sizeof(double) + 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        KC(cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, st));
     else
-        KC(cudaMemcpyAsync((void*) hf, d_fl, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        KC(cudaMemcpyAsync(h.flag, d->flag, sizeof h.flag, cudaMemcpyDeviceToHost, st));
     KC(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     ctx->last_ms = ms;
-    if (hf[0])
+    if (h.flag[0])
         return fail(ctx, KEMCU_ENONFINITE, "field result contains NaN or Inf");
     if (out)
-        std::memcpy(out, h, m * sizeof(double));
+        std::memcpy(out, h.v, m * sizeof(double));
     return KEMCU_OK;
 }
 
@@ -1300,7 +1293,6 @@ int kemcu_create(kemcu_ctx** out, const kemcu_config* cfg)
     KC(cudaEventCreate(&ctx->tv0));
     KC(cudaEventCreate(&ctx->tv1));
     ctx->autotune = cfg->autotune != 0;
-    KC(cudaMallocHost(&ctx->h_stage, kStageBytes));
     KC(cudaMalloc(&ctx->d_counter, 64 * sizeof(unsigned)));
     KC(cudaMemsetAsync(ctx->d_counter, 0, 64 * sizeof(unsigned), ctx->stream));
     // [0]: non-finite values seen; [1]: a direct-sum pipeline wait timed out
@@ -1409,7 +1401,6 @@ int kemcu_destroy(kemcu_ctx* ctx)
         cudaFree(ctx->d_near_ptr);
         cudaFree(ctx->d_near_row);
         cudaFree(ctx->d_near_val);
-        cudaFreeHost(ctx->h_stage);
         cudaFree(ctx->d_counter);
         cudaFree(ctx->d_flag);
         fm_release(ctx);
