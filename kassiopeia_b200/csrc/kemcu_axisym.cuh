@@ -428,15 +428,16 @@ __device__ __forceinline__ AxPar ax_par(const double* e, double x, double y, dou
     return q;
 }
 
-// potential per unit charge density of element e at (x, y, z)
+// potential per unit charge density of element e at (x, y, z); FAST: with the shorter form of the ring
+template<bool FAST = true>
 __device__ __forceinline__ double ax_potential(const double* e, double x, double y, double z)
 {
     const AxPar q = ax_par(e, x, y, z);
     double v[1];
     if (e[aType] == kAxRing)
-        RingPotential<true>()(x, q, v);  // the ring integrand does not depend on its position argument
+        RingPotential<FAST>()(x, q, v);  // the ring integrand does not depend on its position argument
     else
-        conic_integral(RingPotential<true>(), q, v);
+        conic_integral(RingPotential<FAST>(), q, v);
     return e[aPre] * v[0];
 }
 
@@ -488,7 +489,7 @@ constexpr int kAxFieldMinBlocks = 5;
 // direct sum over the elements [e0, e1) of split blockIdx.y at each point, compensated (Kahan)
 // over the elements as KIntegratingFieldSolver does (KElectrostaticIntegratingFieldSolver.hh:
 // 261-339); out n x 4, or partial[split][n][4] summed by reduce_splits in split order
-template<bool POT, bool FIELD>
+template<bool POT, bool FIELD, bool FAST = true>
 __global__ void __launch_bounds__(kAxThreads, kAxFieldMinBlocks)
     axisym_field_kernel(const double* __restrict__ rec, int rec_stride, const double* __restrict__ sigma, int ne,
                         const double* __restrict__ P, int np, double* __restrict__ out, double* __restrict__ partial)
@@ -509,7 +510,7 @@ __global__ void __launch_bounds__(kAxThreads, kAxFieldMinBlocks)
         else if (FIELD)
             ax_field(e, x, y, z, v);
         else
-            v[3] = ax_potential(e, x, y, z);
+            v[3] = ax_potential<FAST>(e, x, y, z);
 #pragma unroll
         for (int m = 0; m < 4; m++) {
             const double yk = v[m] * sg - c[m];

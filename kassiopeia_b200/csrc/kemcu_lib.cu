@@ -451,7 +451,14 @@ int launch_axisym_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d
         }
     }
     const dim3 grid((unsigned) ((n + kAxThreads - 1) / kAxThreads), (unsigned) split);
-    if (what == KEMCU_POTENTIAL)
+    // The potential of points in caller order (fewer than kSortMin) takes the series alone: K by the mean is a
+    // longer chain than Cody's series, and where a warp's points lie on both sides of the shorter form's
+    // border it runs both. 896 elements: 8 points 211 us with the shorter form, 161 without; 1,000 points
+    // 386 and 317; 20,000 (sorted) 2.83 and 4.28 ms.
+    if (what == KEMCU_POTENTIAL && n < kSortMin)
+        axisym_field_kernel<true, false, false><<<grid, kAxThreads, 0, ctx->stream>>>(ctx->d_rec, rRecSize, ctx->d_sigma, ne,
+                                                                                      d_pts, np, d_out, partial);
+    else if (what == KEMCU_POTENTIAL)
         axisym_field_kernel<true, false><<<grid, kAxThreads, 0, ctx->stream>>>(ctx->d_rec, rRecSize, ctx->d_sigma, ne,
                                                                                d_pts, np, d_out, partial);
     else if (what == KEMCU_FIELD)
