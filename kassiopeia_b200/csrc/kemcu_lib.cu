@@ -61,6 +61,8 @@ struct kemcu_ctx
     std::vector<double> h_rhs;         // boundary values
     std::vector<int32_t> h_shape;
     DevBuf geo;  // what the geometry fixes, from d_rec to d_rows: one allocation
+    // which of its parts are computed: by the first call that reads them (ready_far and so on)
+    bool has_far = false, has_near = false, has_rows = false;
     double* d_rec = nullptr;
     TargetRec* d_tgt = nullptr;
     double* d_sigma = nullptr;
@@ -338,11 +340,6 @@ int grid_split(const kemcu_ctx* ctx, size_t n_pts)
     return (int) std::max((size_t) 1, split);
 }
 
-FarView far_view(const kemcu_ctx* ctx)
-{
-    return FarView{ctx->d_far, ctx->d_tiles, ctx->ntiles, ctx->d_pre, ctx->d_rwg};
-}
-
 // The far records' tiles of the context's planar elements, in element order: a run of up to kFarSym
 // elements with two mirror axes (rectangles with orthogonal sides, wires), else up to kFarGen
 // elements of any kind in the general form. Returns the doubles that the records take.
@@ -370,8 +367,22 @@ size_t far_tiling(const kemcu_ctx* ctx, std::vector<FarTile>& tiles)
     return off;
 }
 
-// the far and near records, from the element records on the device
-int build_far(kemcu_ctx* ctx)
+// The records that a geometry's kernels read are computed by the first call that reads them, into memory
+// that SetGeometry set aside (nothing is allocated, so every call may): a probe, the adjoint or a fast
+// multipole tree read no far records, a field no row order.
+int ready_near(kemcu_ctx* ctx)
+{
+    if (ctx->has_near || ctx->axisym)
+        return KEMCU_OK;
+    const size_t n = ctx->n;
+    rwg_build_kernel<<<(unsigned) ((n + 127) / 128), 128, 0, ctx->stream>>>(ctx->d_rec, (int) n, ctx->d_rwg);
+    KCHECK_LAUNCH();
+    ctx->has_near = true;
+    return KEMCU_OK;
+}
+
+// near and far records, as the pair kernels take them
+int ready_far(kemcu_ctx* ctx, FarView* view)
 {
     static const FarTables tables = [] {
         FarTables t;
@@ -383,12 +394,16 @@ int build_far(kemcu_ctx* ctx)
         }
         return t;
     }();
-    const size_t threads = (size_t) ctx->ntiles * kFarSym * kFarLanes, n = ctx->n;
-    far_build_kernel<<<(unsigned) ((threads + kFarBuild - 1) / kFarBuild), kFarBuild, 0, ctx->stream>>>(
-        ctx->d_rec, ctx->d_tiles, ctx->ntiles, tables, ctx->d_far, ctx->d_pre, ctx->d_where);
-    KCHECK_LAUNCH();
-    rwg_build_kernel<<<(unsigned) ((n + 127) / 128), 128, 0, ctx->stream>>>(ctx->d_rec, (int) n, ctx->d_rwg);
-    KCHECK_LAUNCH();
+    if (int rc = ready_near(ctx))
+        return rc;
+    if (!ctx->has_far) {
+        const size_t threads = (size_t) ctx->ntiles * kFarSym * kFarLanes;
+        far_build_kernel<<<(unsigned) ((threads + kFarBuild - 1) / kFarBuild), kFarBuild, 0, ctx->stream>>>(
+            ctx->d_rec, ctx->d_tiles, ctx->ntiles, tables, ctx->d_far, ctx->d_pre, ctx->d_where);
+        KCHECK_LAUNCH();
+        ctx->has_far = true;
+    }
+    *view = FarView{ctx->d_far, ctx->d_tiles, ctx->ntiles, ctx->d_pre, ctx->d_rwg};
     return KEMCU_OK;
 }
 
@@ -401,8 +416,10 @@ size_t cub_sort_bytes(size_t n)
 }
 
 // the matrix rows in Morton order of their collocation points
-int build_rows(kemcu_ctx* ctx)
+int ready_rows(kemcu_ctx* ctx)
 {
+    if (ctx->has_rows)
+        return KEMCU_OK;
     const size_t n = ctx->n;
     Box box = {{1e300, 1e300, 1e300, -1e300, -1e300, -1e300}};
     for (size_t i = 0; i < n; i++)
@@ -422,8 +439,11 @@ int build_rows(kemcu_ctx* ctx)
     void* tmp = q + 2 * up(n * 8) + up(n * 4);
     morton_rows_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->d_tgt, (int) n, box, k0, i0);
     KCHECK_LAUNCH();
+    // cells of 1/2048 of the box (1/256 below 4,096 rows, where one CTA sorts, a pass per few bits)
     size_t tb = cub_bytes;
-    KC(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, i0, ctx->d_rows, (int) n, 0, 63, ctx->stream));
+    const int bits = n < 4096 ? 24 : 33;
+    KC(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, i0, ctx->d_rows, (int) n, 63 - bits, 63, ctx->stream));
+    ctx->has_rows = true;
     return KEMCU_OK;
 }
 
@@ -575,7 +595,9 @@ int launch_planar_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d
         return rc;
     const bool mixed = precision == KEMCU_MIXED;
     const double* sg = ctx->d_sigma;
-    const FarView fv = far_view(ctx);
+    FarView fv;
+    if (int rc = ready_far(ctx, &fv))
+        return rc;
     const int np = (int) n;
     double* part = split > 1 ? partial : nullptr;
     int* fl = ctx->d_flag + 1;
@@ -679,6 +701,8 @@ int field_few(kemcu_ctx* ctx, const double* P, const double* dP, size_t n, doubl
         return rc;
     Result* d = (Result*) base;
     double* d_part = (double*) ((char*) base + ((sizeof h + 63) & ~(size_t) 63));
+    if (int rc = ready_near(ctx))
+        return rc;
     cudaStream_t st = ctx->stream;
     FewPoints host{};
     if (P)
@@ -799,7 +823,10 @@ int apply_op(kemcu_ctx* ctx, int op, const double* d_x, double* d_y, int nrhs)
         }
         dim3 grid((n + kPair * kThreads - 1) / (kPair * kThreads), split);
         int* fl = ctx->d_flag + 1;
-        const FarView fv = far_view(ctx);
+        FarView fv;
+        int rc;
+        if ((rc = ready_far(ctx, &fv)) || (rc = ready_rows(ctx)))
+            return rc;
         if (op == kFree32) {
             if (nrhs == 1)
                 matvec_kernel<false, 1, true><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, n, d_x, nrhs, d_y, partial, fl);
@@ -877,6 +904,10 @@ int assemble(kemcu_ctx* ctx, bool want32)
     const size_t n = ctx->n;
     if (ctx->d_a64 && (!want32 || ctx->d_a32))
         return KEMCU_OK;
+    FarView fv{};
+    int rc;
+    if (!ctx->axisym && ((rc = ready_far(ctx, &fv)) || (rc = ready_rows(ctx))))
+        return rc;
     const size_t ld = op_ld(n);
     const size_t bytes64 = ld * n * sizeof(double), bytes32 = want32 ? ld * n * sizeof(float) : 0;
     size_t budget = ctx->assembled_budget;
@@ -907,7 +938,7 @@ int assemble(kemcu_ctx* ctx, bool want32)
     }
     const int split = grid_split(ctx, n);
     dim3 grid((unsigned) ((n + kPair * kThreads - 1) / (kPair * kThreads)), (unsigned) split);
-    assemble_kernel<false><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, far_view(ctx), ctx->d_tgt, ctx->d_rows, (int) n,
+    assemble_kernel<false><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, (int) n,
                                                               ctx->d_a64, fill32 ? ctx->d_a32 : nullptr, ctx->d_flag + 1);
     KCHECK_LAUNCH();
     return KEMCU_OK;
@@ -1549,13 +1580,9 @@ int kemcu_set_geometry(kemcu_ctx* ctx, size_t n, const int32_t* shape, const int
     upload(ctx->d_tgt, ctx->h_tgt.data(), n * sizeof(TargetRec));
     if (!rc && cudaMemsetAsync(ctx->d_sigma, 0, n * sizeof(double), ctx->stream) != cudaSuccess)
         rc = fail(ctx, KEMCU_ECUDA, "charge densities: %s", cudaGetErrorString(cudaGetLastError()));
-    if (!ctx->axisym) {
+    if (!ctx->axisym)
         upload(ctx->d_tiles, tiles.data(), tiles.size() * sizeof(FarTile));
-        if (!rc)
-            rc = build_far(ctx);
-        if (!rc)
-            rc = build_rows(ctx);
-    }
+    ctx->has_far = ctx->has_near = ctx->has_rows = false;
     if (rc) {
         ctx->n = 0;
         return rc;
@@ -1801,7 +1828,7 @@ int kemcu_matrix_element(kemcu_ctx* ctx, size_t i, size_t j, double* a)
     KC(cudaSetDevice(ctx->device));
     // one thread computes the entry, in the FP64 form of the matvec
     void* d;
-    if ((rc = ensure(ctx, sVec1, sizeof(double), &d)))
+    if ((rc = ensure(ctx, sVec1, sizeof(double), &d)) || (rc = ready_near(ctx)))
         return rc;
     if (ctx->axisym)
         axisym_entry_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_rec, rRecSize, (int) i, (int) j, (double*) d);
