@@ -1173,7 +1173,8 @@ __global__ void morton_kernel(const double* __restrict__ P, int n, const double*
     idx[i] = i;
 }
 
-// the same for the matrix rows' collocation points
+// the same for the matrix rows' collocation points, the Neumann rows after the others: a warp with one of them
+// sums fields for all its rows
 struct Box
 {
     double v[6];
@@ -1190,7 +1191,8 @@ __global__ void morton_rows_kernel(const TargetRec* __restrict__ tgt, int n, con
         const double t = ext > 0. ? (tgt[i].cen[c] - box.v[c]) / ext : 0.;
         q[c] = (unsigned) fmin(fmax(t * 2097151.0, 0.), 2097151.0);
     }
-    key[i] = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
+    key[i] = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2) |
+             (tgt[i].neumann != 0. ? 1ull << 63 : 0ull);
     idx[i] = i;
 }
 

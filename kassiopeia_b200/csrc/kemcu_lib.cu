@@ -415,7 +415,7 @@ size_t cub_sort_bytes(size_t n)
     return b;
 }
 
-// the matrix rows in Morton order of their collocation points
+// the matrix rows in Morton order of their collocation points, Neumann rows last
 int ready_rows(kemcu_ctx* ctx)
 {
     if (ctx->has_rows)
@@ -442,7 +442,7 @@ int ready_rows(kemcu_ctx* ctx)
     // cells of 1/2048 of the box (1/256 below 4,096 rows, where one CTA sorts, a pass per few bits)
     size_t tb = cub_bytes;
     const int bits = n < 4096 ? 24 : 33;
-    KC(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, i0, ctx->d_rows, (int) n, 63 - bits, 63, ctx->stream));
+    KC(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, i0, ctx->d_rows, (int) n, 63 - bits, 64, ctx->stream));
     ctx->has_rows = true;
     return KEMCU_OK;
 }
