@@ -140,11 +140,11 @@ __device__ __forceinline__ void node_moments(const double* e, V3 d, double R2, V
 }
 
 // Bound by the FP64 pipe: ~28 operations a node (43 when the field and the moments were two passes).
-// Four resident CTAs: the analytic integrals of the near pairs would take 255 registers, which left 8
-// warps per SM.
+// Four resident CTAs (MINB): the analytic integrals of the near pairs would take 255 registers, which left 8
+// warps per SM. A grid of at most two CTAs per SM gains nothing from that and keeps the registers.
 constexpr int kAdjMinBlocks = 4;
-template<bool MIXED>
-__global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks) vjp_kernel(const double* __restrict__ rec, int n_elem,
+template<bool MIXED, int MINB>
+__global__ void __launch_bounds__(kAdjThreads, MINB) vjp_kernel(const double* __restrict__ rec, int n_elem,
                                                           const double* __restrict__ pts, const double* __restrict__ wts,
                                                           int n_pts, double* __restrict__ part_s,
                                                           double* __restrict__ part_g)
