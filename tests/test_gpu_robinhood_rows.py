@@ -56,7 +56,7 @@ def test_columns_on_the_fly_match_the_reference(name):
     def rel(a, b):
         return np.max(np.abs(a - b)) / np.max(np.abs(b))
     bound = max(5 * rel(sigma, direct), 100 * tol)
-    with K.CUDAElectrostaticContext(0, assembled_budget_bytes=1000) as ctx:
+    with K.CUDAElectrostaticContext(0, assembled_budget_bytes=8) as ctx:
         ctx.SetGeometry(m)
         x, st = ctx.SolveRobinHood(tol=tol)
         assert st["rel_residual"] <= tol and abs(st["iterations"] - int(checks)) <= 1
