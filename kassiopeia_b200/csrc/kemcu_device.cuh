@@ -19,9 +19,9 @@
 // + t'^2 |B N2|^2 with per-pair C1 = -2 d.(A N1), C2 = -2 d.(B N2): five FMAs per node instead of
 // forming the node and the difference vector, and the field sum collapses to
 // d S0 - (A N1) Ss - (B N2) St with three scalar node sums. Two reciprocal square roots, both
-// from the FP32-class hardware estimate (rsqrt.approx.f64, ~2^-23 relative):
+// from the FP32-class hardware estimate (rsqrt.approx.f64; measured on B200: within 9.1e-7, 2^-20, relative):
 //   * FP64  -- refined by one FP64 step of third order (within one unit in the last place);
-//   * MIXED -- refined by one FP64 Newton step (~1e-13 relative).
+//   * MIXED -- refined by one FP64 Newton step (within 1.3e-12 relative, typically 1e-13).
 // RWG near-field integrals and the analytic line segment are FP64 in both forms.
 #pragma once
 
@@ -212,7 +212,8 @@ __device__ __forceinline__ double rsqrt2_fast(double x)
 }
 // Twice the FP64 reciprocal square root to within about one unit in the last place: the
 // MIXED estimate refined by a second Newton step on z = 2y, 2 y2 = z + (z/8) (4 - x z^2)
-// (the correction is ~1e-13 of z, so its own rounding stays below half an ulp). FP64 form.
+// (the correction is at most ~1e-12 of z, so its own rounding stays below half an ulp). The analytic integrals'
+// form; the nodes take rsqrt_cubic.
 __device__ __forceinline__ double rsqrt2_acc(double x)
 {
     const double z = rsqrt2_fast(x);
@@ -220,8 +221,8 @@ __device__ __forceinline__ double rsqrt2_acc(double x)
     return fma(0.125 * z, e4, z);
 }
 // The FP64 reciprocal square root to within about one unit in the last place in one step of third
-// order from the hardware estimate y0 (relative error below 2^-22): with e = 1 - x y0^2,
-// 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3 e^2/8 + O(e^3)), and 5 e^3/16 < 1e-19. Five FP64
+// order (Householder's) from the hardware estimate y0 (relative error below 2^-20): with e = 1 - x y0^2,
+// 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3 e^2/8 + O(e^3)), and 5 e^3/16 < 3e-18. Five FP64
 // operations after the estimate (the two Newton steps of rsqrt2_acc take seven).
 __device__ __forceinline__ double rsqrt_cubic(double x)
 {
