@@ -331,11 +331,13 @@ int pipe_status(kemcu_ctx* ctx, const char* what)
 
 int grid_split(const kemcu_ctx* ctx, size_t n_pts)
 {
-    // enough CTAs for four waves of the resident CTAs per SM, each split keeping >= 2 tiles
+    // enough CTAs for four waves of the resident CTAs per SM, each split keeping >= 2 tiles, or one where
+    // the grid would leave SMs without a CTA
     const size_t blocks = (n_pts + kPair * kThreads - 1) / (kPair * kThreads);
     const size_t want = (size_t) ctx->num_sms * kMinBlocks * 4;
     size_t split = blocks >= want ? 1 : (want + blocks - 1) / blocks;
-    split = std::min(split, std::max((size_t) 1, (size_t) ctx->ntiles / 2));
+    const size_t tiles = std::max(ctx->ntiles, 1), most = std::max((size_t) 1, tiles / 2);
+    split = blocks * std::min(split, most) < (size_t) ctx->num_sms ? std::min(split, tiles) : std::min(split, most);
     split = std::min(split, (size_t) 65535);
     return (int) std::max((size_t) 1, split);
 }
