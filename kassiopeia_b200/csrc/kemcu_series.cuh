@@ -233,7 +233,7 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
     // s and the moments over s
     double s;
     // the corner (x0, y0) and the sides that its nodes (u, v) in [0, 1]^2 run along
-    const bool triangle = type == kTriangle;
+    const bool triangle = type == kTriangle, wire = type == kLineSegment;
     const double wx = type == kLineSegment ? 0. : bx, wy = type == kLineSegment ? 0. : by;
     double x0, y0;
     if (triangle) {
@@ -382,8 +382,11 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
     // (R >= 5 s) are covered by the factor 1.5. Odd and even orders are looked at (parallelograms have
     // no odd ones). An order n evaluated in FP32 rounds by at most ~4e-7 (n + 1) t^n G_n. Never near
     // the analytic band.
-    for (int z = lane; z < 14; z += kFarLanes) {
-        const double eps = z < 6 ? 5e-16 : z < 12 ? 1e-14 : z == 12 ? 3e-13 : 1e-15;  // FP64, MIXED; FP32 orders
+    for (int z = lane; z < 15; z += kFarLanes) {
+        // FP64, MIXED; FP32 orders (the last: of general elements' nearest tier, whose orders 7 to 10 are FP32 too).
+        // Wires are FP64 in every form
+        const double eps = z < 6 || (wire && z < 12) ? 5e-16 : z < 12 ? 1e-14
+                           : z == 12 && !wire        ? 3e-13 : z < 14 ? 1e-15 : 1e-15;
         const int n = z < 12 ? 7 + z % 6 : z == 12 ? 4 : 6;
         W.r[z] = pow((z < 12 ? 1.5 : 4e-7) * (n + 1) * W.g[n] / eps, 1. / n);
     }
@@ -397,14 +400,15 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
             double r1 = fmax(r[4], r[5]), r2 = fmax(r[2], r[3]), r3 = fmax(r[0], r[1]);
             if (form && !T.general)  // n = 4 in FP32 beyond the first cut
                 r3 = fmax(r3, W.r[12]);
-            else {
-                if (T.general)
-                    r1 = fmax(r1, W.r[13]);
+            if (!form || T.general || wire) {
+                if (form || T.general)
+                    r1 = fmax(r1, W.r[form ? 13 : 14]);
                 r2 = fmax(r2, W.r[13]);
             }
             r2 = fmax(r2, r1);
             r3 = fmax(r3, r2);
-            cut[0] = distance(r3), cut[1] = distance(r2), cut[2] = distance(r1);
+            const double twice = form && wire ? 2. : 1.;  // the FP32 form takes half of these cuts
+            cut[0] = twice * distance(r3), cut[1] = twice * distance(r2), cut[2] = twice * distance(r1);
         }
         // a degenerate element (no plane, no extent) keeps the cubature everywhere
         const double chk = e1.x + e1.y + e1.z + e2.x + e2.y + e2.z + f[fCut] + f[fCut + 2] + f[fCutM] + f[fCutM + 2];
@@ -691,8 +695,9 @@ __device__ __forceinline__ void far_gen(const double* f, const double (&X)[NP], 
     }
 }
 
-// the pairs of far record f with NP points; FAST: the MIXED reciprocal square root. f is 16-byte
-// aligned.
+// the pairs of far record f with NP points; FAST: the MIXED form's orders. f is 16-byte aligned. The reciprocal
+// distance is FP64's in both forms: one Newton step's error, which 7 to 33 nodes average, would go into every
+// pair whole (single pairs' field 5.2e-13 instead of 3.2e-13 in the mean, 3.1e-12 instead of 1.4e-12 at most).
 template<bool GENERAL, int TIER, bool FIELD, bool FAST, int NP>
 __device__ __forceinline__ void far_pairs(const double* f, const V3 (&P)[NP], V3 (&d)[NP], FarSum (&F)[NP])
 {
@@ -703,7 +708,7 @@ __device__ __forceinline__ void far_pairs(const double* f, const V3 (&P)[NP], V3
 #pragma unroll
     for (int p = 0; p < NP; p++) {
         d[p] = v3(P[p].x - hd[fCen], P[p].y - hd[fCen + 1], P[p].z - hd[fCen + 2]);
-        F[p].ir = kPotScale<FAST> * irsq<FAST>(dot(d[p], d[p]));
+        F[p].ir = kPotScale<false> * irsq<false>(dot(d[p], d[p]));
         X[p] = F[p].ir * dot(d[p], e1);
         Y[p] = F[p].ir * dot(d[p], e2);
     }
