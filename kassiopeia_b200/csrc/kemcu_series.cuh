@@ -386,7 +386,7 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
         // FP64, MIXED; FP32 orders (the last: of general elements' nearest tier, whose orders 7 to 10 are FP32 too).
         // Wires are FP64 in every form
         const double eps = z < 6 || (wire && z < 12) ? 5e-16 : z < 12 ? 1e-14
-                           : z == 12 && !wire        ? 3e-13 : z < 14 ? 1e-15 : 1e-15;
+                           : z == 12 && !wire        ? 3e-13 : z < 14 ? 1e-15 : 3e-16;
         const int n = z < 12 ? 7 + z % 6 : z == 12 ? 4 : 6;
         W.r[z] = pow((z < 12 ? 1.5 : 4e-7) * (n + 1) * W.g[n] / eps, 1. / n);
     }
