@@ -237,18 +237,10 @@ template<int SIDE, int NP> struct FarRing
     }
 };
 
-// A warp's points (NP per lane) in a bounding sphere. Called by all 32 lanes.
-template<int NP> __device__ __forceinline__ void warp_sphere(const V3 (&P)[NP], V3& wc, double& wr)
+// A warp's points in a bounding sphere. Called by all 32 lanes.
+__device__ __forceinline__ void warp_sphere(V3 P, V3& wc, double& wr)
 {
-    double lo[3] = {P[0].x, P[0].y, P[0].z}, hi[3] = {P[0].x, P[0].y, P[0].z};
-#pragma unroll
-    for (int p = 1; p < NP; p++) {
-        const double v[3] = {P[p].x, P[p].y, P[p].z};
-        for (int c = 0; c < 3; c++) {
-            lo[c] = fmin(lo[c], v[c]);
-            hi[c] = fmax(hi[c], v[c]);
-        }
-    }
+    double lo[3] = {P.x, P.y, P.z}, hi[3] = {P.x, P.y, P.z};
     for (int o = 16; o > 0; o >>= 1)
         for (int c = 0; c < 3; c++) {
             lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
@@ -321,26 +313,17 @@ struct NearList
     }
 };
 
-// Points per lane of the pair kernels. Two share every coefficient read from shared memory, but the field
-// kernels then spill (193 against 147 ms for 400,000 points of a coaxial pair), and so does the product (26.4
-// against 21.7 ms over 28,800 triangles).
-#ifndef KEMCU_PAIR
-#define KEMCU_PAIR 1
-#endif
-constexpr int kPair = KEMCU_PAIR;
-
 template<int T> struct Tier
 {
     static constexpr int value = T;
 };
 
-// The elements of one tile against a warp's points (NP per lane), each by the cheapest series that
-// holds for all of them, so that the choice is uniform: far(f, j, p, F, d) receives element j's sums
-// for point p (f: its record, d: the point relative to its centroid); elements without one go to the list. A lane per element finds the tier for the warp's
-// bounding sphere; an element whose tier that leaves open is tested point by point.
-template<bool FIELD, bool FAST, bool F32, int NP, class Far>
-__device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, const V3 (&P)[NP], V3 wc, double wr,
-                                           NearList& L, Far far)
+// The elements of one tile against a warp's points, each by the cheapest series that holds for all of them, so
+// that the choice is uniform: far(f, j, F, d) receives element j's sums (f: its record, d: the point relative to its
+// centroid); elements without one go to the list. A lane per element finds the tier for the warp's bounding
+// sphere; an element whose tier that leaves open is tested point by point.
+template<bool FIELD, bool FAST, bool F32, class Far>
+__device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, V3 P, V3 wc, double wr, NearList& L, Far far)
 {
     const int lane = threadIdx.x & 31;
     const int stride = T.general ? kFarGenStride : kFarSymStride;
@@ -349,12 +332,7 @@ __device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, 
     unsigned m1 = __ballot_sync(0xffffffffu, tier == 1);
     for (unsigned m = ~(m1 | m2 | m3) & ((1u << T.count) - 1u); m; m &= m - 1u) {
         const int j = __ffs(m) - 1;
-        const double* f = rec + j * stride;
-        bool low = true;
-#pragma unroll
-        for (int p = 0; p < NP; p++)
-            low = low && far_point<FAST, F32>(f, P[p]);
-        if (__all_sync(0xffffffffu, low))
+        if (__all_sync(0xffffffffu, far_point<FAST, F32>(rec + j * stride, P)))
             m1 |= 1u << j;
         else {
             if (lane == 0)
@@ -362,57 +340,36 @@ __device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, 
             L.n++;
         }
     }
-    // the field of general elements, whose sums take the most registers, point by point
-    constexpr int NG = FIELD ? 1 : NP;
-    auto general = [&](auto tier, unsigned m) {
+    auto series = [&](auto general, auto tier, unsigned m) {
         for (; m; m &= m - 1u) {
             const int j = __ffs(m) - 1;
-            const double* f = rec + j * kFarGenStride;
-#pragma unroll
-            for (int p0 = 0; p0 < NP; p0 += NG) {
-                V3 Q[NG], d[NG];
-                FarSum F[NG];
-#pragma unroll
-                for (int p = 0; p < NG; p++)
-                    Q[p] = P[p0 + p];
-                far_pairs<true, decltype(tier)::value, FIELD, FAST>(f, Q, d, F);
-#pragma unroll
-                for (int p = 0; p < NG; p++)
-                    far(f, j, p0 + p, F[p], d[p]);
-            }
-        }
-    };
-    auto symmetric = [&](auto tier, unsigned m) {
-        for (; m; m &= m - 1u) {
-            const int j = __ffs(m) - 1;
-            const double* f = rec + j * kFarSymStride;
-            V3 d[NP];
-            FarSum F[NP];
-            far_pairs<false, decltype(tier)::value, FIELD, FAST>(f, P, d, F);
-#pragma unroll
-            for (int p = 0; p < NP; p++)
-                far(f, j, p, F[p], d[p]);
+            const double* f = rec + j * (decltype(general)::value ? kFarGenStride : kFarSymStride);
+            const V3 Q[1] = {P};
+            V3 d[1];
+            FarSum F[1];
+            far_pairs<decltype(general)::value, decltype(tier)::value, FIELD, FAST>(f, Q, d, F);
+            far(f, j, F[0], d[0]);
         }
     };
     if (T.general) {
-        general(Tier<3>(), m3);
-        general(Tier<2>(), m2);
-        general(Tier<1>(), m1);
+        series(std::true_type(), Tier<3>(), m3);
+        series(std::true_type(), Tier<2>(), m2);
+        series(std::true_type(), Tier<1>(), m1);
     }
     else {
-        symmetric(Tier<3>(), m3);
-        symmetric(Tier<2>(), m2);
-        symmetric(Tier<1>(), m1);
+        series(std::false_type(), Tier<3>(), m3);
+        series(std::false_type(), Tier<2>(), m2);
+        series(std::false_type(), Tier<1>(), m1);
     }
 }
 
-// compensated sums of a CTA's threads in shared memory (touched once per tile): NS sums of kPair points
+// compensated sums of a CTA's threads in shared memory (touched once per tile)
 template<int NS> struct KahanStore
 {
-    double s[NS * kPair][kThreads], c[NS * kPair][kThreads];
+    double s[NS][kThreads], c[NS][kThreads];
     __device__ __forceinline__ void clear()
     {
-        for (int k = 0; k < NS * kPair; k++)
+        for (int k = 0; k < NS; k++)
             s[k][threadIdx.x] = c[k][threadIdx.x] = 0.;
     }
     __device__ __forceinline__ void add(int k, double v)
@@ -429,7 +386,7 @@ template<int NS> struct KahanStore
 
 // K1: field and/or potential at points. out layout per point: (Ex, Ey, Ez, phi).
 // Distant pairs by the far-field series, the others by the cubature bands or the analytic integrals,
-// from the element records in global memory (L1 / L2: few pairs). A warp takes kPair x 32
+// from the element records in global memory (L1 / L2: few pairs). A warp takes 32
 // consecutive points. Sums are plain within a tile (and within a near list), compensated across.
 // nsplit == gridDim.y; partial != nullptr when nsplit > 1 (then out is untouched).
 // flag |= 2 if a pipeline wait timed out (the outputs are then incomplete).
@@ -448,14 +405,10 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
     __shared__ __align__(128) FarRingStorage<1, kPipe> S;
     __shared__ KahanStore<NS> K;
     __shared__ NearStore s_near[kThreads / 32];
-    const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
-    const bool busy = base - (int) (threadIdx.x & 31) < n_pts;  // the warp has points
-    V3 P[kPair];
-#pragma unroll
-    for (int p = 0; p < kPair; p++) {  // lanes past the last point repeat it
-        const size_t pi = 3 * (size_t) min(base + 32 * p, n_pts - 1);
-        P[p] = v3(pts[pi], pts[pi + 1], pts[pi + 2]);
-    }
+    const int warp = threadIdx.x >> 5, q0 = (blockIdx.x * (kThreads / 32) + warp) * 32, q = q0 + (int) (threadIdx.x & 31);
+    const bool busy = q0 < n_pts;  // the warp has points
+    const size_t pi = 3 * (size_t) min(q, n_pts - 1);  // lanes past the last point repeat it
+    const V3 P = v3(pts[pi], pts[pi + 1], pts[pi + 2]);
     FarRing<1, kPipe> R(S, V.far, V.tiles, V.ntiles);
     auto side = [&](double (*sd)[kFarSym], int first, int cnt, int lane) {
         if (lane < cnt)
@@ -468,37 +421,26 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
     warp_sphere(P, wc, wr);
     K.clear();
     NearList L{s_near[warp], 0};
-    double t[NS][kPair];
+    double t[NS];
     auto clear = [&]() {
 #pragma unroll
         for (int k = 0; k < NS; k++)
-#pragma unroll
-            for (int p = 0; p < kPair; p++)
-                t[k][p] = 0.;
+            t[k] = 0.;
     };
     auto keep = [&]() {
 #pragma unroll
         for (int k = 0; k < NS; k++)
-#pragma unroll
-            for (int p = 0; p < kPair; p++)
-                K.add(k * kPair + p, t[k][p]);
+            K.add(k, t[k]);
     };
     auto near = [&]() {
         clear();
         L.drain(rec, [&](int e, const double* r) {
             const double sg = sigma[e];
-            for (int p = 0; p < kPair; p++) {
-                const Out4 v = epi_here<MIXED, POT, FIELD, F32>(r, V.rwg + (size_t) e * wRecSize, p == 0 ? P[0] : P[kPair - 1]);
-                const double w[4] = {v.ex * sg, v.ey * sg, v.ez * sg, v.phi * sg};
+            const Out4 v = epi_here<MIXED, POT, FIELD, F32>(r, V.rwg + (size_t) e * wRecSize, P);
+            const double w[4] = {v.ex * sg, v.ey * sg, v.ez * sg, v.phi * sg};
 #pragma unroll
-                for (int k = 0; k < NS; k++) {
-                    const double wk = k == kPhi ? w[3] : w[k];
-                    if (p == 0)
-                        t[k][0] += wk;
-                    else
-                        t[k][kPair - 1] += wk;
-                }
-            }
+            for (int k = 0; k < NS; k++)
+                t[k] += k == kPhi ? w[3] : w[k];
         });
         keep();
     };
@@ -514,16 +456,16 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
             clear();
             tile_pairs<FIELD, MIXED || F32, F32>(
                 S.rec[i % kPipe], T, P, wc, wr, L,
-                [&](const double* f, int j, int p, const FarSum& F, V3 d) {
-                    const double q = sp[j] * F.ir;
+                [&](const double* f, int j, const FarSum& F, V3 d) {
+                    const double g = sp[j] * F.ir;
                     if (POT)
-                        t[kPhi][p] = fma(q, F.S, t[kPhi][p]);
+                        t[kPhi] = fma(g, F.S, t[kPhi]);
                     if (FIELD) {
-                        const double k = q * F.ir, a = (k * F.ir) * F.cd, b = -k * F.c1, c = -k * F.c2;
+                        const double k = g * F.ir, a = (k * F.ir) * F.cd, b = -k * F.c1, c = -k * F.c2;
                         const V3 e1 = ld3(f + fE1), e2 = ld3(f + fE1 + 3);
-                        t[0][p] = fma(a, d.x, fma(b, e1.x, fma(c, e2.x, t[0][p])));
-                        t[1][p] = fma(a, d.y, fma(b, e1.y, fma(c, e2.y, t[1][p])));
-                        t[2][p] = fma(a, d.z, fma(b, e1.z, fma(c, e2.z, t[2][p])));
+                        t[0] = fma(a, d.x, fma(b, e1.x, fma(c, e2.x, t[0])));
+                        t[1] = fma(a, d.y, fma(b, e1.y, fma(c, e2.y, t[1])));
+                        t[2] = fma(a, d.z, fma(b, e1.z, fma(c, e2.z, t[2])));
                     }
                 });
             keep();
@@ -533,22 +475,18 @@ __global__ void __launch_bounds__(kThreads, MINB) field_kernel(const double* __r
         R.release(i, side);
     }
     R.finish(ok, flag);
-#pragma unroll
-    for (int p = 0; p < kPair; p++) {
-        const int q = base + 32 * p;
-        if (q < n_pts) {
-            double* o = partial ? partial + ((size_t) blockIdx.y * n_pts + q) * 4 : out + (size_t) q * 4;
-            o[0] = FIELD ? K.get(p) : 0.;
-            o[1] = FIELD ? K.get(kPair + p) : 0.;
-            o[2] = FIELD ? K.get(2 * kPair + p) : 0.;
-            o[3] = POT ? K.get(kPhi * kPair + p) : 0.;
-        }
+    if (q < n_pts) {
+        double* o = partial ? partial + ((size_t) blockIdx.y * n_pts + q) * 4 : out + (size_t) q * 4;
+        o[0] = FIELD ? K.get(0) : 0.;
+        o[1] = FIELD ? K.get(1) : 0.;
+        o[2] = FIELD ? K.get(2) : 0.;
+        o[3] = POT ? K.get(kPhi) : 0.;
     }
 }
 
 // a few points (one probe): a thread per element and point instead of a lane per point, whose
 // other lanes would repeat it. Each CTA sums kFewElems elements for one point; the sums of the CTAs
-// are added in order by reduce_splits.
+// are added in order by field_few_sum_kernel.
 constexpr int kFewPoints = 8, kFewElems = 128;
 struct FewPoints
 {
@@ -667,7 +605,8 @@ __device__ __forceinline__ double entry_far(const double* e, const TargetRec& t,
     return r.ex * t.normal[0] + r.ey * t.normal[1] + r.ez * t.normal[2];
 }
 
-// one entry A(i, j) (kemcu_matrix_element), the FP64 form the matvec uses
+// one entry A(i, j) (kemcu_matrix_element) in FP64, by the rules and the analytic integrals at any distance (the
+// products and the assembly take distant pairs by the series, a few 1e-15 apart)
 __global__ void entry_kernel(const double* __restrict__ rec, const double* __restrict__ rwg,
                              const TargetRec* __restrict__ tgt, int i, int j, double* __restrict__ a)
 {
@@ -677,26 +616,24 @@ __global__ void entry_kernel(const double* __restrict__ rec, const double* __res
 
 constexpr int kMaxRhs = 8;
 
-// the entries of one tile's columns in kPair rows per lane: emit(p, j, A(row p, first + j)). A warp
+// the entries of one tile's columns in a lane's row: emit(j, A(row, first + j)). A warp
 // without a Neumann row sums potentials only; Neumann rows take the field along their normal.
 template<bool FAST, bool F32, class Emit>
 __device__ __forceinline__ void tile_entries(const double* far, const FarTile& T, const double* pre,
-                                             const TargetRec* __restrict__ tgt, const int (&row)[kPair],
-                                             const V3 (&C)[kPair], bool any_neumann, V3 wc, double wr, NearList& L,
+                                             const TargetRec& t, V3 C, bool any_neumann, V3 wc, double wr, NearList& L,
                                              Emit emit)
 {
     if (!any_neumann)
-        tile_pairs<false, FAST, F32>(far, T, C, wc, wr, L, [&](const double*, int j, int p, const FarSum& F, V3) {
-            emit(p, j, (pre[j] * F.ir) * F.S);
+        tile_pairs<false, FAST, F32>(far, T, C, wc, wr, L, [&](const double*, int j, const FarSum& F, V3) {
+            emit(j, (pre[j] * F.ir) * F.S);
         });
     else
-        tile_pairs<true, FAST, F32>(far, T, C, wc, wr, L, [&](const double* f, int j, int p, const FarSum& F, V3 d) {
-            const TargetRec& t = tgt[row[p]];
+        tile_pairs<true, FAST, F32>(far, T, C, wc, wr, L, [&](const double* f, int j, const FarSum& F, V3 d) {
             const V3 nn = v3(t.normal[0], t.normal[1], t.normal[2]);
             const double q = pre[j] * F.ir;
             const double en = q * F.ir * (F.ir * F.cd * dot(nn, d) - F.c1 * dot(nn, ld3(f + fE1)) -
                                           F.c2 * dot(nn, ld3(f + fE1 + 3)));
-            emit(p, j, t.neumann == 0. ? q * F.S : en);
+            emit(j, t.neumann == 0. ? q * F.S : en);
         });
 }
 
@@ -715,19 +652,12 @@ __global__ void __launch_bounds__(kThreads, NR == 1 ? kMinBlocks : 4)
     __shared__ NearStore s_near[kThreads / 32];
     __shared__ __align__(16) PairTable s_rules;
     load_rules(s_rules);  // the ring's constructor has the barrier
-    const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
-    const bool busy = base - (int) (threadIdx.x & 31) < n;
-    int row[kPair];
-    V3 C[kPair];
-    bool neumann = false;
-#pragma unroll
-    for (int p = 0; p < kPair; p++) {
-        row[p] = rows[min(base + 32 * p, n - 1)];
-        const TargetRec& t = tgt[row[p]];
-        C[p] = v3(t.cen[0], t.cen[1], t.cen[2]);
-        neumann = neumann || t.neumann != 0.;
-    }
-    const bool any_neumann = __any_sync(0xffffffffu, neumann);
+    const int warp = threadIdx.x >> 5, q0 = (blockIdx.x * (kThreads / 32) + warp) * 32, q = q0 + (int) (threadIdx.x & 31);
+    const bool busy = q0 < n;
+    const int row = rows[min(q, n - 1)];
+    const TargetRec& t = tgt[row];
+    const V3 C = v3(t.cen[0], t.cen[1], t.cen[2]);
+    const bool any_neumann = __any_sync(0xffffffffu, t.neumann != 0.);
     FarRing<NR + 1, kPipe> R(S, V.far, V.tiles, V.ntiles);
     auto side = [&](double (*sd)[kFarSym], int first, int cnt, int lane) {
         if (lane < cnt) {
@@ -742,55 +672,48 @@ __global__ void __launch_bounds__(kThreads, NR == 1 ? kMinBlocks : 4)
     double wr;
     warp_sphere(C, wc, wr);
     NearList L{s_near[warp], 0};
-    Kahan acc[NR][kPair];
+    Kahan acc[NR];
     auto near = [&]() {
         L.drain(rec, [&](int e, const double* er) {
+            const double* w = V.rwg + (size_t) e * wRecSize;
+            const double a = any_neumann ? entry<MIXED, F32>(s_rules, er, w, t, C) : epi<MIXED, true, false, F32>(s_rules, er, w, C).phi;
 #pragma unroll
-            for (int p = 0; p < kPair; p++) {
-                const double* w = V.rwg + (size_t) e * wRecSize;
-                const double a = any_neumann ? entry<MIXED, F32>(s_rules, er, w, tgt[row[p]], C[p])
-                                             : epi<MIXED, true, false, F32>(s_rules, er, w, C[p]).phi;
-#pragma unroll
-                for (int r = 0; r < NR; r++)
-                    if (NR == 1 || r < nrhs)
-                        acc[r][p].add(a * x[(size_t) r * n + e]);
-            }
+            for (int r = 0; r < NR; r++)
+                if (NR == 1 || r < nrhs)
+                    acc[r].add(a * x[(size_t) r * n + e]);
         });
     };
     bool ok = true;
-    for (int q = 0; q < ntiles; q++) {
-        if (!__all_sync(0xffffffffu, R.wait(q))) {
+    for (int i = 0; i < ntiles; i++) {
+        if (!__all_sync(0xffffffffu, R.wait(i))) {
             ok = false;
             break;
         }
         if (busy) {
-            const FarTile T = S.tile[q % kPipe];
-            const double(*sd)[kFarSym] = S.side[q % kPipe];
-            tile_entries<MIXED || F32, F32>(S.rec[q % kPipe], T, sd[NR], tgt, row, C, any_neumann, wc, wr, L,
-                                            [&](int p, int j, double a) {
+            const FarTile T = S.tile[i % kPipe];
+            const double(*sd)[kFarSym] = S.side[i % kPipe];
+            tile_entries<MIXED || F32, F32>(S.rec[i % kPipe], T, sd[NR], t, C, any_neumann, wc, wr, L, [&](int j, double a) {
 #pragma unroll
-                                                for (int r = 0; r < NR; r++)
-                                                    if (NR == 1 || r < nrhs)
-                                                        acc[r][p].add(a * sd[r][j]);
-                                            });
-            if (L.full() || (q == ntiles - 1 && L.n > 0))  // one place: its code is large
+                for (int r = 0; r < NR; r++)
+                    if (NR == 1 || r < nrhs)
+                        acc[r].add(a * sd[r][j]);
+            });
+            if (L.full() || (i == ntiles - 1 && L.n > 0))  // one place: its code is large
                 near();
         }
-        R.release(q, side);
+        R.release(i, side);
     }
     R.finish(ok, flag);
+    if (q < n)
 #pragma unroll
-    for (int p = 0; p < kPair; p++)
-        if (base + 32 * p < n)
-#pragma unroll
-            for (int r = 0; r < NR; r++) {
-                if (NR > 1 && r >= nrhs)
-                    break;
-                if (partial)
-                    partial[((size_t) blockIdx.y * nrhs + r) * n + row[p]] = acc[r][p].s;
-                else
-                    y[(size_t) r * n + row[p]] = acc[r][p].s;
-            }
+        for (int r = 0; r < NR; r++) {
+            if (NR > 1 && r >= nrhs)
+                break;
+            if (partial)
+                partial[((size_t) blockIdx.y * nrhs + r) * n + row] = acc[r].s;
+            else
+                y[(size_t) r * n + row] = acc[r].s;
+        }
 }
 
 // operator assembly: column-major dense A (A[j * op_ld(n) + i] = A(i, j)), written in FP64 and, when
@@ -805,19 +728,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     __shared__ NearStore s_near[kThreads / 32];
     __shared__ __align__(16) PairTable s_rules;
     load_rules(s_rules);  // the ring's constructor has the barrier
-    const int warp = threadIdx.x >> 5, base = (blockIdx.x * (kThreads / 32) + warp) * 32 * kPair + (threadIdx.x & 31);
-    const bool busy = base - (int) (threadIdx.x & 31) < n;
-    int row[kPair];
-    V3 C[kPair];
-    bool neumann = false;
-#pragma unroll
-    for (int p = 0; p < kPair; p++) {
-        row[p] = rows[min(base + 32 * p, n - 1)];
-        const TargetRec& t = tgt[row[p]];
-        C[p] = v3(t.cen[0], t.cen[1], t.cen[2]);
-        neumann = neumann || t.neumann != 0.;
-    }
-    const bool any_neumann = __any_sync(0xffffffffu, neumann);
+    const int warp = threadIdx.x >> 5, q0 = (blockIdx.x * (kThreads / 32) + warp) * 32, q = q0 + (int) (threadIdx.x & 31);
+    const bool busy = q0 < n;
+    const int row = rows[min(q, n - 1)];
+    const TargetRec& t = tgt[row];
+    const V3 C = v3(t.cen[0], t.cen[1], t.cen[2]);
+    const bool any_neumann = __any_sync(0xffffffffu, t.neumann != 0.);
     FarRing<1, kPipe> R(S, V.far, V.tiles, V.ntiles);
     auto side = [&](double (*sd)[kFarSym], int first, int cnt, int lane) {
         if (lane < cnt)
@@ -829,9 +745,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     double wr;
     warp_sphere(C, wc, wr);
     NearList L{s_near[warp], 0};
-    auto store = [&](int p, int e, double a) {
-        if (base + 32 * p < n) {
-            const size_t idx = (size_t) e * op_ld(n) + row[p];
+    auto store = [&](int e, double a) {
+        if (q < n) {
+            const size_t idx = (size_t) e * op_ld(n) + row;
             if (a64)
                 a64[idx] = a;
             if (a32)
@@ -840,26 +756,24 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     };
     auto near = [&]() {
         L.drain(rec, [&](int e, const double* er) {
-#pragma unroll
-            for (int p = 0; p < kPair; p++)
-                store(p, e, any_neumann ? entry<MIXED>(s_rules, er, V.rwg + (size_t) e * wRecSize, tgt[row[p]], C[p])
-                                        : epi<MIXED, true, false>(s_rules, er, V.rwg + (size_t) e * wRecSize, C[p]).phi);
+            const double* w = V.rwg + (size_t) e * wRecSize;
+            store(e, any_neumann ? entry<MIXED>(s_rules, er, w, t, C) : epi<MIXED, true, false>(s_rules, er, w, C).phi);
         });
     };
     bool ok = true;
-    for (int q = 0; q < ntiles; q++) {
-        if (!__all_sync(0xffffffffu, R.wait(q))) {
+    for (int i = 0; i < ntiles; i++) {
+        if (!__all_sync(0xffffffffu, R.wait(i))) {
             ok = false;
             break;
         }
         if (busy) {
-            const FarTile T = S.tile[q % kPipe];
-            tile_entries<MIXED, false>(S.rec[q % kPipe], T, S.side[q % kPipe][0], tgt, row, C, any_neumann, wc, wr, L,
-                                       [&](int p, int j, double a) { store(p, T.first + j, a); });
-            if (L.full() || (q == ntiles - 1 && L.n > 0))  // one place: its code is large
+            const FarTile T = S.tile[i % kPipe];
+            tile_entries<MIXED, false>(S.rec[i % kPipe], T, S.side[i % kPipe][0], t, C, any_neumann, wc, wr, L,
+                                       [&](int j, double a) { store(T.first + j, a); });
+            if (L.full() || (i == ntiles - 1 && L.n > 0))  // one place: its code is large
                 near();
         }
-        R.release(q, side);
+        R.release(i, side);
     }
     R.finish(ok, flag);
 }

@@ -333,7 +333,7 @@ int grid_split(const kemcu_ctx* ctx, size_t n_pts)
 {
     // enough CTAs for four waves of the resident CTAs per SM, each split keeping >= 2 tiles, or one where
     // the grid would leave SMs without a CTA
-    const size_t blocks = (n_pts + kPair * kThreads - 1) / (kPair * kThreads);
+    const size_t blocks = (n_pts + kThreads - 1) / kThreads;
     const size_t want = (size_t) ctx->num_sms * kMinBlocks * 4;
     size_t split = blocks >= want ? 1 : (want + blocks - 1) / blocks;
     const size_t tiles = std::max(ctx->ntiles, 1), most = std::max((size_t) 1, tiles / 2);
@@ -592,7 +592,7 @@ void few_form(dim3 grid, cudaStream_t st, int what, const kemcu_ctx* ctx, const 
 int launch_planar_field(kemcu_ctx* ctx, const double* d_pts, size_t n, double* d_out, int precision, int what,
                         int split, double* partial)
 {
-    dim3 grid((unsigned) ((n + kPair * kThreads - 1) / (kPair * kThreads)), (unsigned) split);
+    dim3 grid((unsigned) ((n + kThreads - 1) / kThreads), (unsigned) split);
     if (int rc = clear_pipe_flag(ctx))
         return rc;
     const bool mixed = precision == KEMCU_MIXED;
@@ -823,7 +823,7 @@ int apply_op(kemcu_ctx* ctx, int op, const double* d_x, double* d_y, int nrhs)
                 return rc;
             partial = (double*) p;
         }
-        dim3 grid((n + kPair * kThreads - 1) / (kPair * kThreads), split);
+        dim3 grid((n + kThreads - 1) / kThreads, split);
         int* fl = ctx->d_flag + 1;
         FarView fv;
         int rc;
@@ -939,7 +939,7 @@ int assemble(kemcu_ctx* ctx, bool want32)
         return KEMCU_OK;
     }
     const int split = grid_split(ctx, n);
-    dim3 grid((unsigned) ((n + kPair * kThreads - 1) / (kPair * kThreads)), (unsigned) split);
+    dim3 grid((unsigned) ((n + kThreads - 1) / kThreads), (unsigned) split);
     assemble_kernel<false><<<grid, kThreads, 0, ctx->stream>>>(ctx->d_rec, fv, ctx->d_tgt, ctx->d_rows, (int) n,
                                                               ctx->d_a64, fill32 ? ctx->d_a32 : nullptr, ctx->d_flag + 1);
     KCHECK_LAUNCH();
