@@ -57,13 +57,17 @@ enum kemcu_boundary { KEMCU_DIRICHLET = 0, KEMCU_NEUMANN = 1 };
 /* arithmetic form of the element integrals */
 enum kemcu_precision {
     KEMCU_FP64 = 0,  /* every node in FP64: the plain form. Distant pairs are the rules' far-field
-                        series, whose FP32 tail and left-out orders are below 5e-16 of the pair */
+                        series, whose high orders, at most ~3e-9 of the pair, are FP32: a pair's
+                        field is within 2.1e-15 in the worst direction at a cut, 3e-16 in the mean,
+                        as the rules' own rounding */
     KEMCU_MIXED = 1, /* cubature nodes with the FP32-class hardware reciprocal square root
-                        refined by one FP64 Newton step (~1e-13 relative); RWG / analytic
-                        near field and the compensated accumulation as in FP64 */
+                        refined by one FP64 Newton step (within 1.3e-12 relative, ~1e-13 in the
+                        mean); distant pairs' series in FP64 but for orders from 4 on (a pair's
+                        field within 2.5e-13); RWG / analytic near field, wires and the
+                        compensated accumulation as in FP64 */
     KEMCU_FP32 = 2   /* far field in FP32: the cubature nodes of triangles and rectangles nearer
-                        than the far-field series (which is that of KEMCU_MIXED) on FP32 FMAs
-                        and the FP32 hardware reciprocal square root, relative to the
+                        than the far-field series (that of KEMCU_MIXED, from half its cuts on) on
+                        FP32 FMAs and the FP32 hardware reciprocal square root, relative to the
                         element's FP64 centre distance (~1e-7 relative per element); the RWG /
                         analytic near field, wires, the per-element set-up and the compensated
                         element sums in FP64. Field evaluation and matrix-free matvec only (the

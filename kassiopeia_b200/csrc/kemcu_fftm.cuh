@@ -753,7 +753,7 @@ __device__ __forceinline__ void fm_l2p(const double* Lh, int p, double ux, doubl
 // FFTM field solver does, KEBIFactory::MakeAnalytic()), else with the numeric policy.
 //
 // Resident CTAs the registers are bounded for: the chains of the analytic integrals leave the FP64 pipe
-// idle, and more warps fill it better than the spills cost. Coax, 80,000 elements, 10^6 points, degree 8,
+// idle, and more warps fill it better than the spills cost. Coax, 44,000 elements, 10^6 points, degree 8,
 // depth 6, ms per field and potential: 3 CTAs 9.28, 4 8.26, 5 7.80, 6 7.43, 7 7.29; the matrix product (kFmMatvecMinBlocks)
 // 5 CTAs 1.05, 6 1.06, 8 1.10 ms.
 constexpr int kFmEvalMinBlocks = 7, kFmMatvecMinBlocks = 5;

@@ -22,10 +22,12 @@
 // 193 instead of 147 ms for 400,000 points of a coaxial electrode pair.)
 //
 // Precision. FP64 form: n <= 4 in FP64, nearer elements also n = 5 (general) or 6 (symmetric); the
-// tail of higher orders is at most ~2e-9 of the term where it is used, so its FP32 rounding is 1e-16
-// of it, and the cuts bound the first orders left out by 5e-16 of the pair's field in the worst
-// direction at the cut. MIXED form (whose reciprocal square root is good to 8.5e-14): the far tier
-// keeps n = 4 in FP32 too, and the cuts bound the orders left out by 1e-14.
+// tail of higher orders is at most ~3e-9 of the term where it is used. The cuts bound the first orders
+// left out by 5e-16 of the pair's field in the worst direction at the cut, and the rounding of order 6 in FP32 by
+// 1e-15 (in the nearest tier of general elements, where orders 7 to 10 add theirs, 3e-16). Measured against
+// exact integrals, a pair's field at most 2.1e-15 and 2.5e-16 in the mean, a rule's 2.2e-15 and 2.4e-16. MIXED
+// form: n = 4 (symmetric elements' farthest tier) and 5 (general) in FP32 too, orders left out 1e-14, the FP32
+// orders 3e-13: at most 2.5e-13, where the rules' nodes give 1.4e-12. Wires keep FP64's precision in both.
 //
 // Included after kemcu_device.cuh (element records, V3, irsq); the functions here are plain C++
 // apart from their decorations, and tests/cxx/series_host.cc runs them on the CPU.

@@ -46,7 +46,8 @@ def test_robin_hood_assembled_columns_identical(ctx):
     ctx.SetGeometry(golden.mesh_from(fx))
     x1, s1 = ctx.SolveRobinHood(tol=1e-9)
     x2, s2 = ctx.SolveRobinHood(tol=1e-9, assembled=True)
-    # the assembled FP64 operator holds the same entries the matrix-free pass computes
+    # systems of this size keep their columns for the solve: the entries and the kernel of the assembled operator
+    # (columns computed on the fly are compared in test_gpu_robinhood_rows.py)
     assert s1["subiterations"] == s2["subiterations"]
     np.testing.assert_array_equal(x1, x2)
 
@@ -87,9 +88,9 @@ def test_robin_hood_callback_stops(ctx):
 
 
 def test_robin_hood_c1_at_size_on_many_ctas(ctx):
-    # configuration 1 (1,280 triangles): the rows are spread over several CTAs of one
-    # cooperative launch; the reference's KRobinHood needs the same number of checks, and the
-    # matrix-free and assembled columns give the same corrections bit for bit
+    # configuration 1 (1,280 triangles): the reference's KRobinHood needs the same number of checks, and the
+    # columns kept for a solve and the assembled operator's give the same corrections bit for bit (one CTA; columns
+    # on the fly, over several CTAs, are compared in test_gpu_robinhood_rows.py)
     from kassiopeia_b200 import geometry as G
 
     fx = golden.load("c1_sphere")
