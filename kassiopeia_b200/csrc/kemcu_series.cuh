@@ -394,8 +394,9 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
     }
     __syncwarp();
     if (lane == 0) {
-        auto distance = [&](double r) { return fmax(s * fmax(5., r), sqrt(2. * e[rCut])); };
         for (int form = 0; form < 2; form++) {
+            // half of MIXED's cuts, the FP32 form's, lie outside the analytic band too
+            auto distance = [&](double r) { return fmax(s * fmax(5., r), sqrt((form ? 4.0001 : 2.) * e[rCut])); };
             const double* r = W.r + 6 * form;
             double* cut = f + (form ? fCutM : fCut);
             // symmetric: n <= 6, 8, 10; general: n <= 6, 8, 10

@@ -84,3 +84,16 @@ def test_series_is_the_rules_sum_beyond_its_cuts(series, name, mixed):
             tol = 3e-14 if not mixed else 5e-13
             err = np.linalg.norm(out[:, :3] - want[:, :3], axis=1) / np.linalg.norm(want[:, :3], axis=1)
             assert err.max() <= tol and np.abs(out[:, 3] / want[:, 3] - 1).max() <= tol, (tier, far, err.max())
+
+
+@pytest.mark.parametrize("aspect", [1., .95, .84, .8, .5, .1])
+def test_half_of_the_mixed_cuts_is_outside_the_analytic_band(series, aspect):
+    # the FP32 form takes the series from there on, and its analytic pairs are FP64
+    for shape, b in ((G.RECTANGLE, [0., aspect]), (G.RECTANGLE, [.3 * aspect, .9 * aspect]), (G.TRIANGLE, [.5, aspect])):
+        A, B = 1., np.linalg.norm(b)
+        rec = np.zeros(32)
+        rec[0], rec[11], rec[14:16], rec[25] = A, 1., b, shape
+        size = (A + B + np.hypot(1. - b[0], b[1])) / 3 if shape == G.TRIANGLE else .5 * (A + B)
+        rec[29] = ({G.TRIANGLE: 3.42, G.RECTANGLE: 4.6}[shape] * size) ** 2
+        _, cuts = series(rec, int(shape == G.TRIANGLE or b[0] != 0.), 1, 3, np.zeros((2, 3)))
+        assert .5 * cuts.min() > np.sqrt(rec[29])
