@@ -24,7 +24,7 @@
 // Precision. FP64 form: n <= 4 in FP64, nearer elements also n = 5 (general) or 6 (symmetric); the
 // tail of higher orders is at most ~3e-9 of the term where it is used. The cuts bound the first orders
 // left out by 5e-16 of the pair's field in the worst direction at the cut, and the rounding of order 6 in FP32 by
-// 1e-15 (in the nearest tier of general elements, where orders 7 to 10 add theirs, 3e-16). Measured against
+// 1e-15 (in the nearest tier of general elements, where orders 7 to 10 add theirs, 2.5e-16). Measured against
 // exact integrals, a pair's field at most 2.1e-15 and 2.5e-16 in the mean, a rule's 2.2e-15 and 2.4e-16. MIXED
 // form: n = 4 (symmetric elements' farthest tier) and 5 (general) in FP32 too, orders left out 1e-14, the FP32
 // orders 3e-13: at most 2.5e-13, where the rules' nodes give 1.4e-12. Wires keep FP64's precision in both.
@@ -388,7 +388,7 @@ __global__ void far_build_kernel(const double* __restrict__ rec, const FarTile* 
         // FP64, MIXED; FP32 orders (the last: of general elements' nearest tier, whose orders 7 to 10 are FP32 too).
         // Wires are FP64 in every form
         const double eps = z < 6 || (wire && z < 12) ? 5e-16 : z < 12 ? 1e-14
-                           : z == 12 && !wire        ? 3e-13 : z < 14 ? 1e-15 : 3e-16;
+                           : z == 12 && !wire        ? 3e-13 : z < 14 ? 1e-15 : 2.5e-16;
         const int n = z < 12 ? 7 + z % 6 : z == 12 ? 4 : 6;
         W.r[z] = pow((z < 12 ? 1.5 : 4e-7) * (n + 1) * W.g[n] / eps, 1. / n);
     }
