@@ -179,8 +179,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) rk8_tracker_kernel(TrackElems 
         };
         if (warp < el.n)
             fetch(warp);
+#pragma unroll 1
         for (int c = warp; c < kTrackParts; c += W) {
             Kahan ex, ey, ez;
+#pragma unroll 1
             for (int j = c; j < el.n; j += kTrackParts) {
                 __syncwarp();
                 const bool general = at.y & 1;
