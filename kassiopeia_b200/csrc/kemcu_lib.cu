@@ -129,6 +129,7 @@ enum Scratch
     sZ,     // preconditioned Krylov basis (flexible GMRES) or the Jacobi-scaled vector
     sKry,   // BiCGStab vectors
     sInBasis, sInW, sInMisc, sInK,  // the inner GMRES of the implicit Krylov preconditioner
+    sCols,  // columns that a Robin Hood solve keeps (small ones)
     kNumScratch
 };
 static_assert(kNumScratch <= 16, "kemcu_ctx::scratch holds 16 slots");
@@ -901,7 +902,9 @@ int apply_op(kemcu_ctx* ctx, int op, const double* d_x, double* d_y, int nrhs)
                      : launch(dense_mma_kernel<float>, ctx->d_a32, kMmaRowsPerCta / 256);
 }
 
-int assemble(kemcu_ctx* ctx, bool want32)
+// slot: a scratch slot for the FP64 operator instead of an allocation of its own (the caller then takes it out
+// of the context)
+int assemble(kemcu_ctx* ctx, bool want32, int slot = -1)
 {
     const size_t n = ctx->n;
     if (ctx->d_a64 && (!want32 || ctx->d_a32))
@@ -913,6 +916,8 @@ int assemble(kemcu_ctx* ctx, bool want32)
     const size_t ld = op_ld(n);
     const size_t bytes64 = ld * n * sizeof(double), bytes32 = want32 ? ld * n * sizeof(float) : 0;
     size_t budget = ctx->assembled_budget;
+    if (budget == 0 && slot >= 0)
+        budget = bytes64 + bytes32;  // a workspace: as much as can be allocated
     if (budget == 0) {
         size_t fr = 0, tot = 0;
         KC(cudaMemGetInfo(&fr, &tot));
@@ -920,6 +925,8 @@ int assemble(kemcu_ctx* ctx, bool want32)
     }
     if (bytes64 + bytes32 > budget)
         return fail(ctx, KEMCU_ENOMEM, "assembled operator needs %zu bytes, budget %zu", bytes64 + bytes32, budget);
+    if (slot >= 0 && (rc = ensure(ctx, slot, bytes64, (void**) &ctx->d_a64)))
+        return rc;
     if (!ctx->d_a64 && cudaMalloc(&ctx->d_a64, bytes64) != cudaSuccess) {
         cudaGetLastError();
         ctx->d_a64 = nullptr;
