@@ -40,22 +40,12 @@ TOL = 1e-10
 # DRAM bytes (read + write) of one MIXED direct-sum launch over the default 1,000,000-point
 # workload, from a one-pass ncu capture of `python bench.py --profile --points 1000000`;
 # bench.py cannot run ncu itself, so the figure is reported only for that workload
-FIELD_TRAFFIC_BYTES_1M = 74.04e6 + 105.28e6
-# algorithmic flops per element-point interaction (field + potential) by band:
-# cubature / Gauss with n nodes: 20 n + 30 (node sums, ratio test); analytic near field:
-# fixed counts of one pass through the non-degenerate branch (frozen here)
-RWG_FLOPS = {0: 420, 1: 520, 2: 160}  # triangle, rectangle, analytic wire
-NODES = {0: {1: 33, 2: 12, 3: 7}, 1: {1: 33, 2: 12, 3: 7}, 2: {1: 16, 2: 4}}
-
-
-def flops_per_band(counts):
-    c = np.asarray(counts, dtype=np.float64).reshape(3, 4)
-    total = 0.0
-    for shape in range(3):
-        total += c[shape, 0] * RWG_FLOPS[shape]
-        for band, n in NODES[shape].items():
-            total += c[shape, band] * (20 * n + 30)
-    return total
+FIELD_TRAFFIC_BYTES_1M = 84.90e6 + 26.98e6
+# floating-point operations that an element-point pair of the field and potential cannot do without, at whatever
+# distance: the distance (8), its inverse square root (8), the two leading corrections of the element's extent
+# (14) and the sums into four outputs (10). The kernel does more (a distant pair's series 67 to 88 FP64
+# instructions, a near one a rule or the analytic integrals), so the roofline's fraction is a lower bound
+PAIR_FLOPS = 40
 
 
 # ----------------------------------------------------------------------------- CPU reference
@@ -310,12 +300,12 @@ def run_native(args, rank, world, dist):
     of32 = ctx.ElectricFieldAndPotential(sub, precision=K.FP32)
     err_fp32 = accuracy_vs(of32, o64)
 
-    # algorithmic work (band histogram on a 2% sample, scaled) and the FP64 roofline
+    # the reference's quadrature bands of a 2% sample (for the record), the least work and the FP64 roofline
     hs = P[::50]
     counts = np.zeros(12, dtype=np.int64)
     NN.lib().kemcu_band_histogram(ctx._h, np.ascontiguousarray(hs).ctypes.data_as(C.POINTER(C.c_double)), len(hs),
                                   counts.ctypes.data_as(C.POINTER(C.c_longlong)))
-    flops_per_step = flops_per_band(counts) * (N_POINTS / len(hs))
+    flops_per_step = float(PAIR_FLOPS) * N_POINTS * mesh.n
     f64 = C.c_double()
     f32 = C.c_double()
     NN.lib().kemcu_fma_peak(ctx._h, C.byref(f64), C.byref(f32))
@@ -816,7 +806,8 @@ def main():
                                "speedup_over_plain_fp64": r["ms_fp64"] / r["ms_fp32"],
                                "speedup_over_mixed": r["ms_mixed"] / r["ms_fp32"],
                                "accuracy_vs_fp64": r["err_fp32"],
-                               "notes": "cubature nodes of triangles and rectangles in FP32 relative to each "
+                               "notes": "far-field series of the MIXED form from half of its cuts on; nearer cubature "
+                                        "nodes of triangles and rectangles in FP32 relative to each "
                                         "element's FP64 centre distance; analytic near field, wires and the "
                                         "compensated element sums in FP64"},
             "accuracy_mixed_vs_fp64": {"max_rel_err_E_per_point": r["err_E"],
