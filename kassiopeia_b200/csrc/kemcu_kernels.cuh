@@ -328,12 +328,12 @@ __device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, 
     const int lane = threadIdx.x & 31;
     const int stride = T.general ? kFarGenStride : kFarSymStride;
     const int tier = lane < T.count ? far_tier<FAST, F32>(rec + lane * stride, wc, wr) : 0;
-    const unsigned m3 = __ballot_sync(0xffffffffu, tier == 3), m2 = __ballot_sync(0xffffffffu, tier == 2);
-    unsigned m1 = __ballot_sync(0xffffffffu, tier == 1);
+    const unsigned m3 = __ballot_sync(0xffffffffu, tier == 3);
+    unsigned m2 = __ballot_sync(0xffffffffu, tier == 2), m1 = F32 ? 0u : __ballot_sync(0xffffffffu, tier == 1);
     for (unsigned m = ~(m1 | m2 | m3) & ((1u << T.count) - 1u); m; m &= m - 1u) {
         const int j = __ffs(m) - 1;
         if (__all_sync(0xffffffffu, far_point<FAST, F32>(rec + j * stride, P)))
-            m1 |= 1u << j;
+            (F32 ? m2 : m1) |= 1u << j;
         else {
             if (lane == 0)
                 L.S.e[L.n] = T.first + j;
@@ -354,12 +354,14 @@ __device__ __forceinline__ void tile_pairs(const double* rec, const FarTile& T, 
     if (T.general) {
         series(std::true_type(), Tier<3>(), m3);
         series(std::true_type(), Tier<2>(), m2);
-        series(std::true_type(), Tier<1>(), m1);
+        if constexpr (!F32)
+            series(std::true_type(), Tier<1>(), m1);
     }
     else {
         series(std::false_type(), Tier<3>(), m3);
         series(std::false_type(), Tier<2>(), m2);
-        series(std::false_type(), Tier<1>(), m1);
+        if constexpr (!F32)
+            series(std::false_type(), Tier<1>(), m1);
     }
 }
 

@@ -725,10 +725,10 @@ __device__ __forceinline__ void far_pairs(const double* f, const V3 (&P)[NP], V3
 // The tier of one element (far record f) for all points within `wr` of `wc`: the largest of 3, 2, 1
 // whose cut every point's centre distance exceeds (with a 1e-9 margin for the rounding of either
 // side), or 0: some point may need the cubature or the analytic integrals.
-// F32, whose cubature nodes are good to 1e-7: the series holds from half of MIXED's cuts on, where the orders
-// left out grow by at most 2^12 from 1e-14 and the FP32 ones round to below 1e-10. With MIXED's cuts more pairs
-// than before took the rules' nodes or an FP64 series. 20,000 points and 28,800 slivers, ms: 14.8 without the
-// series, 20.7 with MIXED's cuts, 12.7 with half of them; their product 17.6, 16.4, 11.8.
+// F32, whose cubature nodes are good to 1e-7: the farther two tiers from half of MIXED's cuts on, where the orders
+// left out grow by at most 2^10 from 1e-14 and the FP32 ones round to below 1e-10 (the nearest tier costs more
+// than FP32 nodes: 4,000 scattered points and 28,800 slivers 6.3 ms with it, 5.6 without). 20,000 points and the
+// slivers, ms: 14.8 without the series, 20.7 with MIXED's cuts, 12.7 with half of them; their product 17.6, 16.4, 11.3.
 template<bool F32> constexpr double kFarCut = F32 ? 0.5 : 1.;
 template<bool FAST, bool F32> __device__ __forceinline__ int far_tier(const double* f, V3 wc, double wr)
 {
@@ -737,13 +737,13 @@ template<bool FAST, bool F32> __device__ __forceinline__ int far_tier(const doub
     const double* c = f + (FAST ? fCutM : fCut);
     constexpr double h = kFarCut<F32>;
     const double r3 = h * c[0] + wr, r2 = h * c[1] + wr, r1 = h * c[2] + wr;
-    return d2 > r3 * r3 ? 3 : d2 > r2 * r2 ? 2 : d2 > r1 * r1 ? 1 : 0;
+    return d2 > r3 * r3 ? 3 : d2 > r2 * r2 ? 2 : !F32 && d2 > r1 * r1 ? 1 : 0;
 }
-// one point: the series holds (tier 1)
+// one point: the series holds (tier 1; F32: tier 2)
 template<bool FAST, bool F32> __device__ __forceinline__ bool far_point(const double* f, V3 P)
 {
     const double dx = P.x - f[fCen], dy = P.y - f[fCen + 1], dz = P.z - f[fCen + 2];
-    const double r1 = kFarCut<F32> * f[(FAST ? fCutM : fCut) + 2];
+    const double r1 = kFarCut<F32> * f[(FAST ? fCutM : fCut) + (F32 ? 1 : 2)];
     return (dx * dx + dy * dy + dz * dz) * (1. - 1e-9) > r1 * r1;
 }
 
